@@ -151,6 +151,23 @@ int citlali_attention_prefill_tc_with(const void* q, int q_stride, int total_row
                                       int max_new, int nq, int nkv, int head_dim, int page_size, int window, float scale,
                                       int32_t* error_flag, float softcap, const float* gate, size_t gate_stride, const float* sink,
                                       const float* turns, int turn_pairs, float* out32, cudaStream_t stream);
+// The same over keys of 192 and values of 128 that lie as rows (runs of new tokens of latent attention): kv [key_total, nq * 256] is
+// the heads' keys of 128 and then their values of 128, shared_keys [key_total, 64] the rest of every head's key; the key of position
+// t of a sequence is row key_rows[seq] + t.  q is [total_rows, nq * 192]; gate is one number an element or a head.
+int citlali_attention_prefill_tc_latent(const void* q, int total_rows, const void* kv, const void* shared_keys, int key_total,
+                                        const int32_t* key_rows, const int32_t* seq_start, const int32_t* seq_past, void* out,
+                                        int sequences, int max_new, int nq, int window, float scale, int32_t* error_flag,
+                                        const float* gate, size_t gate_stride, int gate_per_head, const float* sink,
+                                        cudaStream_t stream);
+// Its operands.  The cached vectors [c | r] (R and P numbers) that the sequences' new rows see, as rows of c and of r (64 wide, zeros
+// behind P): a sequence's from a multiple of 128 positions to a multiple of 128, zeros where it sees nothing, key_rows as above.
+// max_tiles: the most tiles of 128 positions a sequence has; key_total: 128 times the tiles of all sequences.
+int citlali_latent_gather(const void* pool, const int32_t* page_table, int table_stride, int page_size, const int32_t* seq_start,
+                          const int32_t* seq_slot, const int32_t* seq_past, int sequences, int max_tiles, int R, int P, int window,
+                          void* latents, void* shared_keys, int32_t* key_rows, int key_total, cudaStream_t stream);
+// q [rows, H * (128 + P)] float32 -> out [rows, H * 192] bfloat16, the last P of a head turned by the row's position, zeros behind.
+int citlali_latent_queries(const float* q, int H, int P, const float* inv_freq, int rot_dims, int rot_halves, const int32_t* row_pos,
+                           void* out, int rows, cudaStream_t stream);
 
 // tokens[r] = argmax of logits[r, :] over finite values, lowest index on ties.
 int citlali_argmax_rows(const float* logits, int32_t* tokens, int rows, int vocab, cudaStream_t stream);

@@ -46,6 +46,13 @@
 // a pair of halves lies in the same lane of tensor memory) and a gate on the output.  Scores under a cap of up to 69 lie
 // within 2^100 of one: exponentials are then taken against zero, no maximum is looked for, and the two warps of a row's halves
 // do not meet before the end.
+//
+// A third instance (kLatentKeys) reads keys of 192 elements and values of 128 that lie as plain rows: what latent attention's cached
+// vectors become once a head's matrices are applied to them (latent_prefill.cu).  A key's last 64 elements, the rotated part, are
+// one matrix that all heads share.  Every head has keys of its own, so a block's two query tiles are row tiles of one head.  Shared
+// memory holds two query tiles of 48 KB, ONE key tile of 48 KB and two value tiles of 32 KB (a second key tile does not fit): the
+// next keys are fetched while P V of the tile before runs, on barriers of their own.  It is bound like the plain form by the
+// softmax warps and the issue of the MMAs (20 a tile instead of 16).
 #include "api.h"
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -194,6 +201,45 @@ __device__ __forceinline__ bool mma_values_and_look(uint32_t tmem_d, uint32_t tm
         : "=r"(seen) : "r"(tmem_d), "r"(tmem_p), "l"(desc_v), "r"(idesc), "r"(accumulate), "r"(bar), "r"(parity) : "memory");
     return seen != 0;
 }
+// The same scores over 192 elements: twelve K slices, the third 64 elements another `half_units` further.
+__device__ __forceinline__ bool mma_scores192_and_look(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                       uint32_t bar, uint32_t parity) {
+    uint32_t seen;
+    asm volatile(
+        "{\n"
+        ".reg .pred look, yes, no;\n"
+        ".reg .b64 a, b;\n"
+        "setp.eq.u32 yes, 0, 0;\n"
+        "setp.ne.u32 no, 0, 0;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 look, [%5], %6;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, no;\n"
+        "add.u64 a, %2, 2;\n add.u64 b, %3, 2;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 4;\n add.u64 b, %3, 4;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 6;\n add.u64 b, %3, 6;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 1024;\n add.u64 b, %3, 1024;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 1026;\n add.u64 b, %3, 1026;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 1028;\n add.u64 b, %3, 1028;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 1030;\n add.u64 b, %3, 1030;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 2048;\n add.u64 b, %3, 2048;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 2050;\n add.u64 b, %3, 2050;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 2052;\n add.u64 b, %3, 2052;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "add.u64 a, %2, 2054;\n add.u64 b, %3, 2054;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %4, yes;\n"
+        "selp.b32 %0, 1, 0, look;\n"
+        "}"
+        : "=r"(seen) : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(bar), "r"(parity) : "memory");
+    return seen != 0;
+}
 static_assert(kHalfTile >> 4 == 1024 && kHalfKeys == 64 && kD == 128 && kTileK == 128,
               "the offsets written into mma_scores_and_look and mma_values_and_look are those of 128 x 128 tiles");
 
@@ -232,7 +278,13 @@ struct Params {
     size_t gate_stride;
     int turn_pairs;
     float* out32;                        // the result in float32 instead of the rounded one (rows out_stride apart)
+    // kLatentKeys only: the key at position 0 of a sequence would be this row of the key and value matrices; the gate may be one
+    // number a head instead of one an element
+    const int32_t* key_rows;
+    int gate_per_head;
 };
+
+enum Form : int { kPlain = 0, kOptions = 1, kLatentKeys = 2 };
 
 // One of the block's two query tiles: its head, its first row within the sequence's new tokens, and the
 // key tiles it reads (none when it has no rows).
@@ -247,10 +299,12 @@ __device__ __forceinline__ float fast_rcp(float x) {
     return y;
 }
 
-template <bool kWith>
+template <int kForm>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, Params p) {
+    constexpr bool kWith = kForm != kPlain, kLatent = kForm == kLatentKeys;
+    constexpr uint32_t kQBytes = kLatent ? 3 * kHalfTile : kTileBytes;       // a tile of queries or keys
     extern __shared__ uint8_t smem_raw[];
     // kv_full[stage]: the keys and the values of a tile have landed (both producers arrive with their bytes);
     // kv_empty[stage]: the MMAs on them have finished
@@ -260,12 +314,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     __shared__ float pair_sum[2][2][kTileQ];                 // the same for the sums at the end (a thread that is done with its
                                                              // last tile must not write over a maximum its partner has yet to read)
     __shared__ int pair_vote[2][4][2];                       // [query tile][quarter][half]: this half wants the second pass
+    __shared__ __align__(8) uint64_t k_full, k_empty;        // kLatentKeys: its one key tile (kv_full and kv_empty are the values')
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     volatile int* abort_flag = &abort_word;
 
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t s_q = base, s_k = base + 2 * kTileBytes, s_v = base + 4 * kTileBytes;      // two tiles each
+    const uint32_t s_q = base, s_k = base + 2 * kQBytes, s_v = s_k + (kLatent ? kQBytes : 2 * kTileBytes);      // two tiles each (kLatentKeys: one of keys)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -275,13 +330,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         abort_word = 0;
         mbar_init(smem_u32(&q_bar), 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(smem_u32(&kv_full[i]), 2);
+            mbar_init(smem_u32(&kv_full[i]), kLatent ? 1 : 2);
             mbar_init(smem_u32(&kv_empty[i]), 1);
             mbar_init(smem_u32(&s_full[i]), 1);
             mbar_init(smem_u32(&p_full[i]), 8);
             mbar_init(smem_u32(&o_done[i]), 1);
             for (int qd = 0; qd < 4; ++qd) mbar_init(smem_u32(&pair_bar[i][qd]), 2);
         }
+        if constexpr (kLatent) { mbar_init(smem_u32(&k_full), 1); mbar_init(smem_u32(&k_empty), 1); }
         fence_barrier_init();
         fence_async_proxy();
     }
@@ -318,9 +374,40 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
     }
     const int g = qt[0].head / (p.nq / p.nkv);               // both query tiles read this key/value head
-    const int32_t* pages = p.page_table + (size_t)p.seq_slot[seq] * p.page_table_stride;
+    const int32_t* pages = kLatent ? nullptr : p.page_table + (size_t)p.seq_slot[seq] * p.page_table_stride;
 
-    if (warp == kWarpLoadK || warp == kWarpLoadV) {
+    if (kLatent && (warp == kWarpLoadK || warp == kWarpLoadV)) {
+        if (lane == 0 && t_hi >= t_lo) {
+            // map_k: [rows, nq * 128 of keys | nq * 128 of values]; map_v: [rows, 64], the part of the keys that all heads share
+            const int first_row = p.key_rows[seq], head = qt[0].head;
+            if (warp == kWarpLoadK) {
+                mbar_arrive_expect_tx(smem_u32(&q_bar), 2 * kQBytes);
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                        tma_load_2d(s_q + b * kQBytes + c * kHalfTile, &map_q, head * (kD + 64) + 64 * c, row0 + qt[b].q0, smem_u32(&q_bar));
+                for (int t = t_lo; t <= t_hi; ++t) {
+                    const int i = t - t_lo, row = first_row + t * kTileK;
+                    if (!mbar_wait(smem_u32(&k_empty), (i & 1u) ^ 1u, abort_flag, p.error_flag, 201)) break;
+                    mbar_arrive_expect_tx(smem_u32(&k_full), kQBytes);
+                    tma_load_2d(s_k, &map_k, head * kD, row, smem_u32(&k_full));
+                    tma_load_2d(s_k + kHalfTile, &map_k, head * kD + 64, row, smem_u32(&k_full));
+                    tma_load_2d(s_k + 2 * kHalfTile, &map_v, 0, row, smem_u32(&k_full));
+                }
+            } else {
+                for (int t = t_lo; t <= t_hi; ++t) {
+                    const int i = t - t_lo, st = i & 1, row = first_row + t * kTileK;
+                    const uint32_t full = smem_u32(&kv_full[st]), dst = s_v + st * kTileBytes;
+                    if (!mbar_wait(smem_u32(&kv_empty[st]), ((i >> 1) & 1u) ^ 1u, abort_flag, p.error_flag, 210)) break;
+                    mbar_arrive_expect_tx(full, kTileBytes);
+                    tma_load_2d(dst, &map_k, (p.nq + head) * kD, row, full);
+                    tma_load_2d(dst + kHalfTile, &map_k, (p.nq + head) * kD + 64, row, full);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kWarpLoadK || warp == kWarpLoadV) {
         if (lane == 0 && t_hi >= t_lo) {
             const bool is_k = warp == kWarpLoadK;
             if (is_k) {
@@ -383,8 +470,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // mma_scores_and_look); `look_bar` 0 means there is nothing to look at (the Q barrier, long passed, stands in).
             const uint32_t passed_bar = smem_u32(&q_bar);
             auto issue_qk = [&](int b, int t, uint32_t look_bar, uint32_t look_parity) -> bool {
-                const uint64_t a0 = dq0 + (b ? kTileUnits : 0), b0 = dk0 + (((t - t_lo) & 1) ? kTileUnits : 0);
-                const bool seen = mma_scores_and_look(tmem + b * kSubCols + kColS, a0, b0, idesc_qk,
+                const uint64_t a0 = dq0 + (b ? (kQBytes >> 4) : 0), b0 = dk0 + (!kLatent && ((t - t_lo) & 1) ? kTileUnits : 0);
+                const bool seen = (kLatent ? mma_scores192_and_look : mma_scores_and_look)(tmem + b * kSubCols + kColS, a0, b0, idesc_qk,
                                                       look_bar ? look_bar : passed_bar, look_bar ? look_parity : 0u);
                 mma_commit(smem_u32(&s_full[b]));
                 return seen && look_bar != 0;
@@ -400,6 +487,53 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             auto kv_bar = [&](int t) -> uint32_t { return smem_u32(&kv_full[(t - t_lo) & 1]); };
             auto kv_parity = [&](int t) -> uint32_t { return ((t - t_lo) >> 1) & 1u; };
             auto p_parity = [&](int b, int t) -> uint32_t { return (uint32_t)(t - qt[b].tile_lo) & 1u; };
+            if constexpr (kLatent) {
+                // As below, with the keys' one tile free as soon as both query tiles' scores are done and the values' after both
+                // products with P.  (The looks ahead: P V of query tile 0 looks at the next keys, its next scores at P of query
+                // tile 1, P V of query tile 1 at the next values, its next scores at the next P of query tile 0.)
+                const uint32_t kf = smem_u32(&k_full), ke = smem_u32(&k_empty);
+                auto need_k = [&](int t, bool seen) -> bool {
+                    return seen || mbar_wait(kf, (uint32_t)(t - t_lo) & 1u, abort_flag, p.error_flag, 204);
+                };
+                ok = mbar_wait(smem_u32(&q_bar), 0, abort_flag, p.error_flag, 202) && need_k(t_lo, false);
+                if (ok) {
+                    tc_fence_after();
+                    if (qt[0].reads(t_lo)) issue_qk(0, t_lo, 0, 0);
+                    if (qt[1].reads(t_lo)) issue_qk(1, t_lo, 0, 0);
+                    mma_commit(ke);
+                }
+                bool seen_p0 = false, seen_v = false;
+                for (int t = t_lo; t <= t_hi && ok; ++t) {
+                    const bool more = t + 1 <= t_hi;
+                    bool seen_k = false, seen_p1 = false;
+                    if (!need_kv(t, seen_v)) { ok = false; break; }
+                    seen_v = false;
+                    if (qt[0].reads(t)) {
+                        if (!need_p(0, t, seen_p0)) { ok = false; break; }
+                        seen_k = issue_pv(0, t, more ? kf : 0u, (uint32_t)(t + 1 - t_lo) & 1u);
+                    }
+                    if (more) {
+                        if (!need_k(t + 1, seen_k)) { ok = false; break; }
+                        if (qt[0].reads(t + 1)) {
+                            tc_fence_after();
+                            seen_p1 = issue_qk(0, t + 1, qt[1].reads(t) ? smem_u32(&p_full[1]) : 0u, qt[1].reads(t) ? p_parity(1, t) : 0u);
+                        }
+                    }
+                    if (qt[1].reads(t)) {
+                        if (!need_p(1, t, seen_p1)) { ok = false; break; }
+                        seen_v = issue_pv(1, t, more ? kv_bar(t + 1) : 0u, more ? kv_parity(t + 1) : 0u);
+                    }
+                    mma_commit(smem_u32(&kv_empty[(t - t_lo) & 1]));
+                    seen_p0 = false;
+                    if (more) {
+                        if (qt[1].reads(t + 1)) {
+                            const bool look = qt[0].reads(t + 1);
+                            seen_p0 = issue_qk(1, t + 1, look ? smem_u32(&p_full[0]) : 0u, look ? p_parity(0, t + 1) : 0u);
+                        }
+                        mma_commit(ke);
+                    }
+                }
+            } else {
             ok = mbar_wait(smem_u32(&q_bar), 0, abort_flag, p.error_flag, 202) && need_kv(t_lo, false);
             if (ok) {
                 tc_fence_after();
@@ -437,6 +571,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     const bool look = qt[0].reads(t + 1);
                     seen_p0 = issue_qk(1, t + 1, look ? smem_u32(&p_full[0]) : 0u, look ? p_parity(0, t + 1) : 0u);
                 }
+            }
             }
         }
         __syncwarp();
@@ -654,7 +789,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                                 }
                             }
                         }
-                        if (p.gate) {
+                        if (kLatent && p.gate && p.gate_per_head) {
+                            const float z = p.gate[row * p.gate_stride + me.head];
+                            const float f = 1.0f / (1.0f + expf(-z));
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * f);
+                        } else if (p.gate) {
                             const float* gt = p.gate + row * p.gate_stride + (size_t)me.head * kD + half * kHalfKeys + c0;
 #pragma unroll
                             for (int c = 0; c < 16; c += 4) {
@@ -759,8 +899,9 @@ static int launch_prefill_tc(const void* q, int q_stride, int total_rows, const 
     p.cap_out = softcap > 0.0f ? softcap * log2e : 0.0f;
     p.fixed_reference = p.cap_out > 0.0f && p.cap_out <= 100.0f ? 1 : 0;
     p.sink = sink; p.turns = (const float2*)turns; p.gate = gate; p.gate_stride = gate_stride; p.turn_pairs = turn_pairs; p.out32 = out32;
+    p.key_rows = nullptr; p.gate_per_head = 0;
     const size_t smem = (size_t)6 * fatc::kTileBytes + 1024;
-    auto kernel = with ? fatc::attention_prefill_tc_kernel<true> : fatc::attention_prefill_tc_kernel<false>;
+    auto kernel = with ? fatc::attention_prefill_tc_kernel<fatc::kOptions> : fatc::attention_prefill_tc_kernel<fatc::kPlain>;
     static bool configured[2] = {false, false};
     if (!configured[with]) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -797,4 +938,51 @@ extern "C" int citlali_attention_prefill_tc_with(const void* q, int q_stride, in
     return launch_prefill_tc(q, q_stride, total_rows, k_pool, v_pool, pool_pages, page_table, page_table_stride, seq_start, seq_slot,
                              seq_past, out, out_stride, sequences, max_new, nq, nkv, head_dim, page_size, window, scale, error_flag,
                              true, softcap, gate, gate_stride, sink, turns, turn_pairs, out32, stream);
+}
+
+// Causal attention of runs of new tokens over a latent cache, with the heads' matrices applied to the cached vectors beforehand
+// (see latent_prefill.cu, which makes the operands).  q [total_rows, nq * 192] (a head's 128 plain and 64 rotated elements); kv
+// [key_total, nq * 256]: the heads' keys of 128, then the heads' values of 128; shared_keys [key_total, 64]: the rotated part, one
+// for all heads.  The keys of a sequence lie in position order, position t at row key_rows[seq] + t; a key tile of 128 that holds a
+// visible key lies wholly in the sequence's own rows, and values of positions after the last are finite.  gate (or null): the
+// result is multiplied by sigmoid(gate), an element each or, with gate_per_head, a head.
+extern "C" int citlali_attention_prefill_tc_latent(const void* q, int total_rows, const void* kv, const void* shared_keys, int key_total,
+                                                   const int32_t* key_rows, const int32_t* seq_start, const int32_t* seq_past,
+                                                   void* out, int sequences, int max_new, int nq, int window, float scale,
+                                                   int32_t* error_flag, const float* gate, size_t gate_stride, int gate_per_head,
+                                                   const float* sink, cudaStream_t stream) {
+    if (sequences <= 0 || max_new <= 0) return 0;
+    if (nq <= 0 || nq > 65535 || max_new / fatc::kTileQ >= 65535 || sequences > 65535) {
+        set_last_error("attention_prefill_tc_latent: bad head count (%d) or too many sequences (%d)", nq, sequences);
+        return kBadShape;
+    }
+    if ((((uintptr_t)q | (uintptr_t)out | (uintptr_t)kv | (uintptr_t)shared_keys) & 15u) ||
+        (gate && !gate_per_head && (((uintptr_t)gate & 15u) || gate_stride % 4 != 0))) {
+        set_last_error("attention_prefill_tc_latent: operands must be 16-byte aligned");
+        return kBadAlignment;
+    }
+    CUtensorMap mq, mk, mr;
+    int rc;
+    if ((rc = fatc::make_map(&mq, q, (uint64_t)total_rows, (uint64_t)nq * 192, (uint64_t)nq * 192, fatc::kTileQ))) return rc;
+    if ((rc = fatc::make_map(&mk, kv, (uint64_t)key_total, (uint64_t)nq * 256, (uint64_t)nq * 256, fatc::kTileK))) return rc;
+    if ((rc = fatc::make_map(&mr, shared_keys, (uint64_t)key_total, 64, 64, fatc::kTileK))) return rc;
+    fatc::Params p{};
+    p.seq_start = seq_start; p.seq_past = seq_past; p.key_rows = key_rows;
+    p.out = (__nv_bfloat16*)out; p.out_stride = nq * fatc::kD;
+    p.nq = nq; p.nkv = nq; p.window = window;
+    p.scale_log2 = scale * 1.4426950408889634f;
+    p.error_flag = error_flag;
+    p.gate = gate; p.gate_stride = gate_stride; p.gate_per_head = gate_per_head; p.sink = sink;
+    const size_t smem = (size_t)3 * 3 * fatc::kHalfTile + 2 * fatc::kTileBytes + 1024;
+    auto kernel = fatc::attention_prefill_tc_kernel<fatc::kLatentKeys>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int row_tiles = (max_new + fatc::kTileQ - 1) / fatc::kTileQ;
+    dim3 grid(nq, (row_tiles + 1) / 2, sequences);
+    launch_kernel(kernel, grid, fatc::kThreads, smem, stream, mq, mk, mr, p);
+    return CITLALI_LAUNCH_CHECK();
 }

@@ -1250,3 +1250,72 @@ def latent_attention(q, pool, page_table, row_slot, row_pos, sink, out, H, R, E,
                                           _i(page_table.shape[1]), _ptr(row_slot), _ptr(row_pos), _ptr(sink), _ptr(out),
                                           _i(rows), _i(H), _i(R), _i(E), _i(page_size), _i(int(window or 0)), _f(scale),
                                           _stream()), "latent_attention")
+
+
+_KEY_TILE = 128
+
+
+def _seen_tiles(past: int, n: int, window: int):
+    """The tiles of 128 positions that ``n`` new rows behind ``past`` tokens see: the first and the one behind the last."""
+    lo = max(0, past - window + 1) if window else 0
+    return lo // _KEY_TILE, (past + n - 1) // _KEY_TILE + 1
+
+
+def latent_runs_as_attention(batch, dtype, H, R, P, D, V, window, gate, gate_per_head) -> bool:
+    """Whether a step's latent attention runs with the heads' keys and values written out (:func:`latent_run_attention`) instead of as
+    a walk over the latents.  Writing a cached vector's keys and values out costs 2 H R (D + V) operations on the dense product and a
+    visible pair then 2 H (192 + 128) on the prompt kernel, in tiles of 256 rows; the walk costs 2 H (2 R + P) a pair at an eighth of
+    that rate.  So: sequences of at least 64 new rows on average, and at most four visible keys a new row (with more, the keys and
+    values would also take more memory than the walk's own buffers).  Windows below 64, and steps with a sequence of fewer than 32
+    tokens in all, keep the walk: the rounding of the values averages out over the keys a row sees, and over a single key the walk has
+    none (a lone row: 0.0031 against 0.0023 off float64)."""
+    if (dtype != torch.bfloat16 or (window is not None and 0 < int(window) < 64) or D != 128 or V != 128 or R % 8 != 0 or P % 8 != 0 or P > 64
+            or batch.rows < 64 * batch.sequences or torch.cuda.is_current_stream_capturing()):
+        return False
+    if not gate_per_head and (gate.data_ptr() % 16 != 0 or gate.stride(0) % 4 != 0):
+        return False
+    tiles = 0
+    for p, n in zip(batch.past, batch.n_new):
+        if p + n < 32:
+            return False
+        first, behind = _seen_tiles(p, n, int(window or 0))
+        tiles += behind - first
+    return tiles * _KEY_TILE <= 4 * batch.rows + _KEY_TILE * batch.sequences
+
+
+def latent_run_attention(q, pool, page_table, page_size, batch, kv_up, sink, out, H, R, P, inv_freq, rot_dims, rot_halves, window, scale,
+                         gate, gate_per_head, error_flag):
+    """Latent attention of runs of new tokens with a key [W_uk c | r] and a value W_uv c a head: the cached vectors the step sees are
+    gathered into rows, one product with ``kv_up`` [H (128 + 128), R] (the heads' W_uk, then their W_uv) makes keys and values, and
+    the prompt kernel walks them.  ``q`` float32 [rows, H (128 + P)], unrotated; ``out`` bfloat16 [rows, H 128], gated."""
+    _need_cuda(q, pool, page_table, kv_up, sink, out, inv_freq)
+    rows, window = q.shape[0], int(window or 0)
+    require(q.dtype == torch.float32 and q.shape == (rows, H * (128 + P)) and pool.dtype == torch.bfloat16 and pool.shape[-1] == R + P
+            and kv_up.dtype == torch.bfloat16 and kv_up.shape == (H * 256, R) and out.dtype == torch.bfloat16
+            and out.shape == (rows, H * 128) and gate.dtype == torch.float32 and gate.shape[0] == rows
+            and (sink is None or (sink.dtype == torch.float32 and sink.numel() == H))
+            and (rot_dims == 0 or (inv_freq.dtype == torch.float32 and inv_freq.numel() == rot_dims // 2)),
+            "latent_run_attention: shapes or dtypes do not fit")
+    total = longest = 0
+    for p, n in zip(batch.past, batch.n_new):
+        first, behind = _seen_tiles(p, n, window)
+        total += behind - first
+        longest = max(longest, behind - first)
+    total *= _KEY_TILE
+    dev = q.device
+    latents = torch.empty((total, R), dtype=torch.bfloat16, device=dev)
+    shared_keys = torch.empty((total, 64), dtype=torch.bfloat16, device=dev)
+    key_rows = torch.empty((batch.sequences,), dtype=torch.int32, device=dev)
+    _check(lib().citlali_latent_gather(_ptr(pool), _ptr(page_table), _i(page_table.shape[1]), _i(page_size), _ptr(batch.seq_start),
+                                       _ptr(batch.seq_slot), _ptr(batch.seq_past), _i(batch.sequences), _i(longest), _i(R), _i(P),
+                                       _i(window), _ptr(latents), _ptr(shared_keys), _ptr(key_rows), _i(total), _stream()),
+           "latent_gather")
+    kv = torch.empty((total, H * 256), dtype=torch.bfloat16, device=dev)
+    gemm_tc(latents, kv_up, kv, error_flag=error_flag)
+    qb = torch.empty((rows, H * 192), dtype=torch.bfloat16, device=dev)
+    _check(lib().citlali_latent_queries(_ptr(q), _i(H), _i(P), _ptr(inv_freq), _i(rot_dims), _i(1 if rot_halves else 0),
+                                        _ptr(batch.row_pos), _ptr(qb), _i(rows), _stream()), "latent_queries")
+    _check(lib().citlali_attention_prefill_tc_latent(
+        _ptr(qb), _i(rows), _ptr(kv), _ptr(shared_keys), _i(total), _ptr(key_rows), _ptr(batch.seq_start), _ptr(batch.seq_past), _ptr(out),
+        _i(batch.sequences), _i(batch.max_new), _i(H), _i(window), _f(scale), _ptr(error_flag), _ptr(gate), _sz(gate.stride(0)),
+        _i(1 if gate_per_head else 0), _ptr(sink), _stream()), "attention_prefill_tc_latent")

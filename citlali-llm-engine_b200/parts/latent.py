@@ -5,7 +5,8 @@ part r (``rot_dim`` numbers, rotated by the position) that all heads share.  Hea
 W_uv,a c, its query [q_plain | q_rot] = W_uq RMSnorm(W_dq h) with q_rot rotated like r.  Since
 q_plain . (W_uk c) = (W_uk^T q_plain) . c, the heads' matrices are applied to the query before and to the weighted sum of
 latents after the walk over the cache (``ops.heads_product``), and the walk (``ops.latent_attention``) reads the cached
-vector once for every head.  Scores are scaled by ``scale``; position i sees j with 0 <= i - j < window (None: every
+vector once for every head.  Runs of new tokens in bfloat16 (head and value sizes of 128) write the heads' keys and values out
+instead and run as plain attention (``ops.latent_run_attention``).  Scores are scaled by ``scale``; position i sees j with 0 <= i - j < window (None: every
 j <= i); the softmax's denominator also counts exp(sink_a), a learned number per head without key or value (absent
 tensor name: none); the heads side by side are multiplied by sigmoid(W_g h), then pass the output matrix.  ``gate``
 "elements" (the default): W_g gives a number for every element of every head's output; "heads": one number a head.
@@ -40,7 +41,10 @@ from .linear import DenseLinear
 class LatentAttention:
     graph_safe = True
     can_overwrite = True
-    kernel_sources = ("latent_attention", "latent_attention_mma")
+
+    def kernel_sources(self, dtype):
+        walk = ("latent_attention", "latent_attention_mma")
+        return walk + ("latent_prefill", "attention_prefill_tc") if self._writes_keys_out(dtype) else walk
 
     def __init__(self, params, prefix: str):
         self.hidden = int(params["hidden_size"])
@@ -90,6 +94,10 @@ class LatentAttention:
             specs.append(TensorSpec(nm["sink"], (self.H,), "state"))
         return specs
 
+    def _writes_keys_out(self, dtype) -> bool:
+        """Whether runs of new tokens can run as plain attention at all (see ``ops.latent_runs_as_attention``)."""
+        return dtype == torch.bfloat16 and self.D == 128 and self.V == 128 and self.R % 8 == 0 and self.P % 8 == 0 and self.P <= 64
+
     def cache_requirement(self):
         if not self.kv_projection:
             return None
@@ -103,8 +111,10 @@ class LatentAttention:
         self.q_weight = bind_float32(weights, nm["dq_norm"], (self.RQ,), ctx)
         self.c_weight = bind_float32(weights, nm["dkv_norm"], (self.R,), ctx) if self.kv_projection else None
         self.sink = bind_float32(weights, nm["sink"], (self.H,), ctx) if nm["sink"] is not None else None
-        uk = torch.empty((self.H * self.D, self.R), dtype=ctx.dtype, device=ctx.device)
-        self.uv = torch.empty((self.H * self.V, self.R), dtype=ctx.dtype, device=ctx.device)
+        # one buffer [W_uk of every head; W_uv of every head]: as a whole it makes keys and values of cached vectors
+        both = torch.empty((self.H * (self.D + self.V), self.R), dtype=ctx.dtype, device=ctx.device)
+        uk, self.uv = both[:self.H * self.D], both[self.H * self.D:]
+        self.kv_up = both if self._writes_keys_out(ctx.dtype) else None
         for name, dst in ((nm["uk"], uk), (nm["uv"], self.uv)):
             require(tuple(weights[name].shape) == tuple(dst.shape),
                     f"unexpected tensor shape for {name}: got {list(weights[name].shape)}, expected {list(dst.shape)}")
@@ -116,6 +126,7 @@ class LatentAttention:
         self.inv_freq = (torch.pow(torch.tensor(self.rot_base, dtype=torch.float64), -2.0 * i / max(self.rot_dims, 1))
                          .to(torch.float32).to(ctx.device)) if self.rot_dims else None
         self.dtype = ctx.dtype
+        self.error_flag = ctx.error_flag
 
     def forward(self, h, batch, cache_view, residual, write_cache=True, overwrite=False):
         require(cache_view is not None and cache_view.requirement.head_dim == self.R + self.P
@@ -132,6 +143,12 @@ class LatentAttention:
                            self.rot_dims, batch.row_slot, batch.row_pos, table, pool, page, cq, self.eps,
                            rot_halves=self.rot_halves)
         q = self.uq.forward(cq, out_dtype=torch.float32)                      # [rows, H (D + P)]
+        gate = proj[:, self.gate_at:]
+        heads = torch.empty((rows, H * V), dtype=self.dtype, device=dev)
+        if self.kv_up is not None and ops.latent_runs_as_attention(batch, self.dtype, H, R, P, D, V, self.window, gate, self.gate_per_head):
+            ops.latent_run_attention(q, pool, table, page, batch, self.kv_up, self.sink, heads, H, R, P, self.inv_freq, self.rot_dims,
+                                     self.rot_halves, self.window, self.scale, gate, self.gate_per_head, self.error_flag)
+            return self._finish(heads, residual, overwrite)
         qa = torch.empty((rows, H * (R + P)), dtype=torch.float32, device=dev)
         ops.heads_product(q, H * (D + P), D + P, self.uk, D * R, 1, D, qa, H * (R + P), R + P, rows, H, D, R,
                           tail=P, inv_freq=self.inv_freq, rot_dims=self.rot_dims, row_pos=batch.row_pos,
@@ -139,9 +156,11 @@ class LatentAttention:
         mixed = torch.empty((rows, H * R), dtype=torch.float32, device=dev)
         ops.latent_attention(qa, pool, table, batch.row_slot, batch.row_pos, self.sink, mixed, H, R, R + P, page,
                              int(self.window or 0), self.scale)
-        heads = torch.empty((rows, H * V), dtype=self.dtype, device=dev)
         ops.heads_product(mixed, H * R, R, self.uv, V * R, 1, R, heads, H * V, V, rows, H, R, V,
-                          gate=proj[:, self.gate_at:], gate_stride=proj.shape[1], gate_per_head=self.gate_per_head)
+                          gate=gate, gate_stride=proj.shape[1], gate_per_head=self.gate_per_head)
+        return self._finish(heads, residual, overwrite)
+
+    def _finish(self, heads, residual, overwrite):
         if overwrite:
             self.o.forward(heads, out=residual)
         else:

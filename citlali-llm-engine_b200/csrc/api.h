@@ -258,6 +258,13 @@ int citlali_delta_prepare(const float* proj, int proj_stride, const float* taps_
 int citlali_delta_rule(const float* prep, int prep_stride, float* state, size_t state_stride, const int32_t* seq_start,
                        const int32_t* seq_slot, int sequences, int H, int KH, int D, int V, float* out, int pairs, int mode,
                        cudaStream_t stream);
+// The recurrence in mode 0 over runs of tokens, 32 at a time (the same numbers up to the order of the sums): two launches.  max_new:
+// the longest sequence's rows; D at most 128, and D, V and prep_stride multiples of four.  scratch: 16-byte aligned, as many floats
+// as citlali_delta_chunks_scratch_floats says for the step's rows.
+size_t citlali_delta_chunks_scratch_floats(int rows, int sequences, int H);
+int citlali_delta_chunks(const float* prep, int prep_stride, float* state, size_t state_stride, const int32_t* seq_start,
+                         const int32_t* seq_slot, int sequences, int max_new, int H, int KH, int D, int V, float* out, float* scratch,
+                         size_t scratch_floats, int rows, cudaStream_t stream);
 // y[r, h, :] = o[r, h, :] / sqrt(mean(o^2) + eps) * weight * act(gate[r * gate_stride + h V ...]); gate_act 0: SiLU, 1: sigmoid.
 int citlali_delta_output(const float* o, const float* gate, int gate_stride, const float* weight, void* y, int y_dtype,
                          int rows, int H, int V, float eps, int gate_act, cudaStream_t stream);

@@ -13,8 +13,8 @@
 //                    float32 (zeros behind P), rounded once.
 // Both are bound by the bytes they move (16 bytes a thread and access).
 //
-// A layer of 32 heads, R 512, P 64 over one prompt of 2,048 tokens: 1.48 ms (walk 1,145 us, heads' matrices 337 us) before; a step of
-// two such layers and two others went from 5.96 to 3.59 ms.
+// A layer of 32 heads, R 512, P 64 over one prompt of 2,048 tokens: 10 us gathering, 16 us for the queries, 40 us for the product, 68 us
+// of attention; before, 1,145 us for the walk and 337 us for the heads' matrices.
 #include "api.h"
 #include "common.cuh"
 

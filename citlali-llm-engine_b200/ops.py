@@ -687,6 +687,32 @@ def delta_rule(prep, state, seq_start, seq_slot, sequences, H, KH, D, V, out, pa
                                     _i(1 if pairs else 0), _i(mode), _stream()), "delta_rule")
 
 
+def delta_runs_in_chunks(batch, D, V, width) -> bool:
+    """Whether a step of the recurrence (one decay a head) runs 32 tokens at a time (:func:`delta_chunks`) or walks: from 48 rows a
+    sequence on, for sizes the chunks' 16-byte pieces take.  32 heads of 128 x 128, walk against chunks in us: one sequence of 24 / 48 /
+    256 / 2,048 rows 20 / 39 / 184 / 1,420 against 19 / 23 / 52 / 318; sixteen of 32 / 33 / 48 / 256 rows 136 / 140 / 196 / 967 against
+    108 / 172 / 172 / 588 (a chunk that begins is paid for whole)."""
+    return (batch.rows >= 48 * batch.sequences and D <= 128 and D % 4 == 0 and V % 4 == 0 and width % 4 == 0
+            and not torch.cuda.is_current_stream_capturing())
+
+
+def delta_chunks(prep, state, seq_start, seq_slot, sequences, max_new, H, KH, D, V, out):
+    """:func:`delta_rule` with one decay a head, 32 tokens at a time; ``max_new``: the longest sequence's rows."""
+    _need_cuda(prep, state, seq_start, seq_slot, out)
+    rows = prep.shape[0]
+    require(prep.dtype == torch.float32 and state.dtype == torch.float32 and out.dtype == torch.float32 and out.shape == (rows, H * V)
+            and state.shape[1] >= H * D * V and prep.shape[1] == 2 * KH * D + H * V + 2 * H, "delta_chunks: shapes or dtypes do not fit")
+    l = lib()
+    l.citlali_delta_chunks_scratch_floats.restype = ctypes.c_size_t
+    scratch = torch.empty(l.citlali_delta_chunks_scratch_floats(_i(rows), _i(sequences), _i(H)), dtype=torch.float32, device=prep.device)
+    _check(l.citlali_delta_chunks(_ptr(prep), _i(prep.shape[1]), _ptr(state), _sz(state.shape[1]), _ptr(seq_start), _ptr(seq_slot),
+                                  _i(sequences), _i(max_new), _i(H), _i(KH), _i(D), _i(V), _ptr(out), _ptr(scratch),
+                                  _sz(scratch.numel()), _i(rows), _stream()), "delta_chunks")
+
+
+_KERNELS_PER_CALL["delta_chunks"] = 2
+
+
 def delta_output(o, gate, gate_stride, weight, y, H, V, eps, gate_act="silu"):
     """``gate``: a view into rows that starts at the gate's first column; ``gate_act``: "silu" or "sigmoid"."""
     _need_cuda(o, weight, y)

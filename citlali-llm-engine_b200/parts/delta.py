@@ -50,7 +50,9 @@ def bind_float32(weights, name: str, shape, ctx) -> torch.Tensor:
 class GatedDeltaMixer:
     graph_safe = True        # slots and row ranges are read on the device; the launches depend on the counts alone
     can_overwrite = True
-    kernel_sources = ("delta_rule",)
+
+    def kernel_sources(self, dtype):
+        return ("delta_rule", "delta_chunks") if dtype == torch.bfloat16 and not self.channel_decay else ("delta_rule",)
 
     def __init__(self, params, prefix: str):
         self.hidden = int(params["hidden_size"])
@@ -147,10 +149,14 @@ class GatedDeltaMixer:
                               self.V, _UNIT_EPS, block_a_segment=few, beta_col=self.C,
                               decay_in=low[:, :self.H * self.GD], channel_decay=self.channel_decay)
         o = torch.empty((rows, hv), dtype=torch.float32, device=proj.device)
-        # bfloat16 steps take a sequence's rows two at a time; the 32-bit path keeps one order of operations for every cut
-        ops.delta_rule(prep, state, batch.seq_start, batch.seq_slot, batch.sequences, self.H, self.KH, self.D, self.V, o,
-                       pairs=self.dtype == torch.bfloat16,
-                       mode=ops.DELTA_CHANNEL_DECAY if self.channel_decay else ops.DELTA_HEAD_DECAY)
+        # bfloat16 steps take a sequence's rows 32 or two at a time; the 32-bit path keeps one order of operations for every cut
+        if self.dtype == torch.bfloat16 and not self.channel_decay and ops.delta_runs_in_chunks(batch, self.D, self.V, prep.shape[1]):
+            ops.delta_chunks(prep, state, batch.seq_start, batch.seq_slot, batch.sequences, batch.max_new, self.H, self.KH, self.D,
+                             self.V, o)
+        else:
+            ops.delta_rule(prep, state, batch.seq_start, batch.seq_slot, batch.sequences, self.H, self.KH, self.D, self.V, o,
+                           pairs=self.dtype == torch.bfloat16,
+                           mode=ops.DELTA_CHANNEL_DECAY if self.channel_decay else ops.DELTA_HEAD_DECAY)
         y = torch.empty((rows, hv), dtype=self.dtype, device=proj.device)
         ops.delta_output(o, gate, gate_stride, self.norm_w, y, self.H, self.V, self.eps, gate_act=self.gate_act)
         if overwrite:

@@ -1,0 +1,69 @@
+"""The gated delta rule 32 tokens at a time against the recurrence in float64, and no further off than the walk: lengths around a chunk,
+sequences side by side, states carried over, key and value sizes that do not fill the tiles, decays of nothing and of everything."""
+import pytest
+import torch
+
+from citlali_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def recurrence(prep, lengths, H, KH, D, V, S):
+    """Float64; ``S`` [sequences, H, D, V] is left as the state."""
+    C, out, at = 2 * KH * D + H * V, [], 0
+    p = prep.double()
+    for s, n in enumerate(lengths):
+        for t in range(at, at + n):
+            q = p[t, :KH * D].view(KH, D).repeat_interleave(H // KH, 0)
+            k = p[t, KH * D:2 * KH * D].view(KH, D).repeat_interleave(H // KH, 0)
+            v, beta, g = p[t, 2 * KH * D:C].view(H, V), p[t, C:C + H, None], p[t, C + H:, None]
+            S[s] *= g[..., None]
+            u = beta * (v - torch.einsum("hdv,hd->hv", S[s], k))
+            S[s] += k[..., None] * u[:, None]
+            out.append(torch.einsum("hdv,hd->hv", S[s], q).flatten())
+        at += n
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("D, V, H, KH, lengths, decays", [
+    (128, 128, 4, 2, [200, 1, 64], "mixed"), (128, 128, 2, 2, [31, 32, 33, 65], "slow"), (64, 40, 6, 2, [96, 7], "none"),
+    (20, 4, 2, 1, [70], "fast"), (128, 128, 32, 16, [100], "mixed"), (96, 36, 8, 8, [40, 129, 32, 5, 1], "mixed")])
+def test_chunks_against_float64_and_the_walk(D, V, H, KH, lengths, decays):
+    T, C = sum(lengths), 2 * KH * D + H * V
+    g = torch.Generator().manual_seed(D + T)
+    prep = torch.zeros(T, C + 2 * H)
+    unit = torch.nn.functional.normalize(torch.randn(T, 2 * KH, D, generator=g) + 0.3, dim=-1)      # keys that lean one way
+    prep[:, :2 * KH * D] = unit.view(T, -1)
+    prep[:, :KH * D] *= D ** -0.5
+    prep[:, 2 * KH * D:C] = torch.randn(T, H * V, generator=g)
+    prep[:, C:C + H] = torch.rand(T, H, generator=g)
+    r = torch.rand(T, H, generator=g)
+    prep[:, C + H:] = {"mixed": torch.where(r < 0.05, torch.zeros(()), r ** 0.1), "slow": 1 - 1e-3 * r, "none": torch.ones(T, H),
+                       "fast": 1e-6 * r}[decays]
+    bounds = [0]
+    for n in lengths:
+        bounds.append(bounds[-1] + n)
+    seq_start = torch.tensor(bounds, dtype=torch.int32, device=DEV)
+    slots = list(range(len(lengths)))[::-1]
+    seq_slot = torch.tensor(slots, dtype=torch.int32, device=DEV)
+    extra = 24                                                 # a state region holds more than S
+    start = torch.randn(len(lengths), H * D * V + extra, generator=g)
+    want_state = torch.stack([start[s, :H * D * V].view(H, D, V) for s in slots]).double()
+    want = [recurrence(prep, lengths, H, KH, D, V, want_state), recurrence(prep, lengths, H, KH, D, V, want_state)]
+    off = {}
+    for name in ("chunks", "walk"):
+        state, got = start.to(DEV), []
+        for _ in range(2):                                     # the same rows once more, from the states just left
+            out = torch.full((T, H * V), float("nan"), device=DEV)
+            if name == "chunks":
+                ops.delta_chunks(prep.to(DEV), state, seq_start, seq_slot, len(lengths), max(lengths), H, KH, D, V, out)
+            else:
+                ops.delta_rule(prep.to(DEV), state, seq_start, seq_slot, len(lengths), H, KH, D, V, out, pairs=True)
+            got.append(out.cpu())
+        assert torch.equal(state[:, H * D * V:].cpu(), start[:, H * D * V:])
+        left = torch.stack([state[s, :H * D * V].view(H, D, V) for s in slots]).cpu().double()
+        off[name] = [float((a.double() - b).norm() / b.norm()) for a, b in [(got[0], want[0]), (got[1], want[1]), (left, want_state)]]
+    # 32-bit sums: a few 2^-24 each, along chains of a chunk's 32 tokens instead of the walk's pairs
+    for a, b in zip(off["chunks"], off["walk"]):
+        assert a <= 2e-6 and a <= 2.0 * b + 1e-7, off

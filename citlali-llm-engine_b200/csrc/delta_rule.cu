@@ -111,6 +111,100 @@ delta_prepare_kernel(const float* __restrict__ proj, int proj_stride, const floa
     for (int i = lane + 256; i < n; i += 32) dst[c0 + i] *= f;
 }
 
+// The same for TAPS taps and segments of at most 32 CPL channels, RUN rows a warp: an input is read once, for the RUN rows whose
+// convolution it enters, instead of once a tap, and the taps once for all of them (the kernel above reads eight numbers for every one
+// it writes).  The same operations in the same order, so the same bits.  Bound by the bytes of proj and prep: 2,048 rows of 8,192
+// channels, four taps: 55 us, above 123 us.
+constexpr int kPrepareRun = 8;
+
+template <int TAPS, int CPL>
+__global__ void __launch_bounds__(128)
+delta_prepare_run_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ taps_w,
+                         const float* __restrict__ state, size_t state_stride, size_t conv_off, const int32_t* __restrict__ row_slot,
+                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ prep, int rows, int H,
+                         int KH, int D, int V, float unit_eps, int beta_col, int decay_col, const float* __restrict__ decay_in,
+                         int decay_stride, int channel_decay) {
+    dependents_may_launch();
+    wait_for_predecessor();
+    const int row0 = blockIdx.x * kPrepareRun, lane = threadIdx.x & 31;
+    const int seg = blockIdx.y * 4 + (threadIdx.x >> 5);
+    if (seg >= 2 * KH + H) return;
+    const int C = 2 * KH * D + H * V;
+    const int GD = channel_decay ? D : 1;                          // decays a head: one, or one a key channel
+    const int width = C + H + H * GD;
+    const int count = min(kPrepareRun, rows - row0);
+    if (seg >= 2 * KH) {
+        const int h = seg - 2 * KH;
+        auto row_of = [&](int r, int tid, int threads) {
+            write_strength_and_decay(proj + (size_t)r * proj_stride, beta_col, decay_col, decay_in ? decay_in + (size_t)r * decay_stride : nullptr,
+                                     a_log, dt_bias, prep + (size_t)r * width + C, H, GD, h, tid, threads);
+        };
+        if (GD == 1) {                                             // a lane a row
+            if (lane < count) row_of(row0 + lane, 0, 1);
+        } else {
+            for (int r = 0; r < count; ++r) row_of(row0 + r, lane, 32);
+        }
+    }
+    const bool unit = seg < 2 * KH;                           // q and k heads are made unit vectors
+    const int c0 = unit ? seg * D : 2 * KH * D + (seg - 2 * KH) * V, n = unit ? D : V;
+    float w[CPL][TAPS], past[CPL][TAPS - 1];                  // past[j][b]: channel j's input b + 1 tokens back
+#pragma unroll
+    for (int j = 0; j < CPL; ++j) {
+        const int i = lane + 32 * j;
+#pragma unroll
+        for (int t = 0; t < TAPS; ++t) w[j][t] = i < n ? taps_w[(size_t)(c0 + i) * TAPS + t] : 0.0f;
+    }
+    int slot_before = -1;
+#pragma unroll 4
+    for (int r = 0; r < count; ++r) {
+        const int row = row0 + r, slot = row_slot[row];
+        float x[CPL], v[CPL];
+#pragma unroll
+        for (int j = 0; j < CPL; ++j) {
+            const int i = lane + 32 * j;
+            x[j] = i < n ? proj[(size_t)row * proj_stride + c0 + i] : 0.0f;
+        }
+        if (r == 0 || slot != slot_before) {                  // the inputs behind the run's, or a sequence's, first row
+            int in_step = 0;                                  // how many of the tokens before this one are rows of this step
+            while (in_step < TAPS - 1 && row - in_step - 1 >= 0 && row_slot[row - in_step - 1] == slot) ++in_step;
+            const float* kept = state + (size_t)slot * state_stride + conv_off;
+#pragma unroll
+            for (int b = 1; b < TAPS; ++b)
+#pragma unroll
+                for (int j = 0; j < CPL; ++j) {
+                    const int i = lane + 32 * j, c = c0 + i;
+                    past[j][b - 1] = i >= n ? 0.0f
+                                     : b <= in_step ? proj[(size_t)(row - b) * proj_stride + c]
+                                                    : kept[(size_t)(TAPS - 1 - b + in_step) * C + c];
+                }
+            slot_before = slot;
+        }
+        float ss = 0.0f;
+#pragma unroll
+        for (int j = 0; j < CPL; ++j) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int b = TAPS - 1; b >= 1; --b) acc = fmaf(w[j][TAPS - 1 - b], past[j][b - 1], acc);      // oldest first
+            acc = fmaf(w[j][TAPS - 1], x[j], acc);
+            v[j] = lane + 32 * j < n ? siluf_(acc) : 0.0f;
+            ss = fmaf(v[j], v[j], ss);
+#pragma unroll
+            for (int b = TAPS - 1; b >= 2; --b) past[j][b - 1] = past[j][b - 2];
+            past[j][0] = x[j];
+        }
+        float f = 1.0f;
+        if (unit) {
+            ss = warp_sum(ss);
+            f = 1.0f / sqrtf(ss + unit_eps);
+            if (seg < KH) f /= sqrtf((float)D);
+        }
+        float* dst = prep + (size_t)row * width + c0;
+#pragma unroll
+        for (int j = 0; j < CPL; ++j)
+            if (lane + 32 * j < n) dst[lane + 32 * j] = v[j] * f;
+    }
+}
+
 // The same with a block of 128 threads a segment, a thread a channel: for steps of few rows, where a row's segments
 // are all the parallelism there is.  (It sums a head's squares in another order than the kernel above.)
 __global__ void __launch_bounds__(128)
@@ -435,6 +529,14 @@ extern "C" int citlali_delta_prepare(const float* proj, int proj_stride, const f
         launch_kernel(delta_prepare_block_kernel, prepare_grid, 128, smem, stream, proj, proj_stride, taps_w, taps,
                       (const float*)state, state_stride, conv_off, row_slot, a_log, dt_bias, prep, H, KH, D, V, unit_eps,
                       beta_col, decay_col, decay_in, decay_stride, channel_decay);
+    } else if (taps >= 2 && taps <= 4 && D <= 256 && V <= 256) {
+        dim3 prepare_grid((rows + kPrepareRun - 1) / kPrepareRun, (segments + 3) / 4);
+        const bool narrow = D <= 128 && V <= 128;
+        auto kernel = taps == 4 ? (narrow ? delta_prepare_run_kernel<4, 4> : delta_prepare_run_kernel<4, 8>)
+                      : taps == 3 ? (narrow ? delta_prepare_run_kernel<3, 4> : delta_prepare_run_kernel<3, 8>)
+                                  : (narrow ? delta_prepare_run_kernel<2, 4> : delta_prepare_run_kernel<2, 8>);
+        launch_kernel(kernel, prepare_grid, 128, 0, stream, proj, proj_stride, taps_w, (const float*)state, state_stride, conv_off, row_slot,
+                      a_log, dt_bias, prep, rows, H, KH, D, V, unit_eps, beta_col, decay_col, decay_in, decay_stride, channel_decay);
     } else {
         dim3 prepare_grid(rows, (segments + 7) / 8);
         launch_kernel(delta_prepare_kernel, prepare_grid, 256, 0, stream, proj, proj_stride, taps_w, taps, (const float*)state,

@@ -42,3 +42,39 @@ def test_attention_rows_of_a_group_have_the_bits_of_single_heads(nq, nkv, d, win
         want = (torch.softmax(s, -1) @ vv).transpose(0, 1).reshape(n, nq * d)
         assert float((outs[0][at:at + n].double() - want).abs().max()) <= (2e-5 if dtype == torch.float32 else 1e-2) * float(want.abs().max())
         at += n
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("D, V, channel", [(128, 128, False), (20, 40, False), (160, 72, False), (48, 256, True)])
+def test_delta_prepare_against_float64(taps, D, V, channel):
+    H, KH, lengths, past = 4, 2, [5, 1, 17, 2, 8, 30], 3        # runs of eight rows begin in, at and between sequences
+    T, C, GD = sum(lengths), 2 * KH * D + H * V, D if channel else 1
+    g = torch.Generator().manual_seed(taps * D)
+    proj = torch.randn(T, C + H * V + 2 * H, generator=g)
+    decay = torch.randn(T, H * GD, generator=g) if channel else None
+    w, a_log, bias = torch.randn(C, taps, generator=g), torch.randn(H, generator=g) * 0.3, torch.randn(H * GD, generator=g)
+    state = torch.randn(8, H * D * V + (taps - 1) * C, generator=g)
+    slots = [3, 0, 7, 5, 1, 2]
+    bounds = torch.tensor([0] + lengths).cumsum(0)
+    slot_of = torch.cat([torch.full((n,), s) for n, s in zip(lengths, slots)]).to(torch.int32)
+    got, kept = {}, state.to(DEV)
+    prep = torch.full((T, C + H + H * GD), float("nan"), device=DEV)
+    i32 = lambda t: torch.as_tensor(t, dtype=torch.int32, device=DEV)
+    ops.delta_prepare(proj.to(DEV), w.to(DEV), kept, H * D * V, i32(slot_of), i32(bounds), i32(slots), len(slots), a_log.to(DEV), bias.to(DEV),
+                      prep, H, KH, D, V, 1e-6, decay_in=None if decay is None else decay.to(DEV), channel_decay=channel)
+    prep = prep.cpu().double()
+    for b, (n, s) in enumerate(zip(lengths, slots)):
+        lo, hi = int(bounds[b]), int(bounds[b + 1])
+        before = state[s, H * D * V:].view(taps - 1, C)
+        x = torch.cat([before, proj[lo:hi, :C]]).double()
+        y = sum(x[t:t + n] * w[:, t].double() for t in range(taps))
+        y = y * torch.sigmoid(y)
+        q, k = (z.reshape(n, KH, D) / torch.sqrt((z.reshape(n, KH, D) ** 2).sum(-1, keepdim=True) + 1e-6) for z in (y[:, :KH * D], y[:, KH * D:2 * KH * D]))
+        want = torch.cat([q.flatten(1) * D ** -0.5, k.flatten(1), y[:, 2 * KH * D:]], 1)
+        assert float((prep[lo:hi, :C] - want).abs().max()) <= 3e-6 * float(want.abs().max())
+        beta = torch.sigmoid(proj[lo:hi, C + H * V:C + H * V + H].double())
+        pre = decay[lo:hi] if channel else proj[lo:hi, C + H * V + H:]
+        rate = torch.exp(a_log.double()).repeat_interleave(GD)
+        decays = torch.exp(-rate * torch.nn.functional.softplus(pre.double() + bias.double()))
+        assert float((prep[lo:hi, C:C + H] - beta).abs().max()) <= 1e-6 and float((prep[lo:hi, C + H:] - decays).abs().max()) <= 2e-6
+        assert torch.equal(kept[s, H * D * V:].cpu().view(taps - 1, C), torch.cat([before, proj[lo:hi, :C]])[n:])

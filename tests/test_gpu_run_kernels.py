@@ -78,3 +78,21 @@ def test_delta_prepare_against_float64(taps, D, V, channel):
         decays = torch.exp(-rate * torch.nn.functional.softplus(pre.double() + bias.double()))
         assert float((prep[lo:hi, C:C + H] - beta).abs().max()) <= 1e-6 and float((prep[lo:hi, C + H:] - decays).abs().max()) <= 2e-6
         assert torch.equal(kept[s, H * D * V:].cpu().view(taps - 1, C), torch.cat([before, proj[lo:hi, :C]])[n:])
+
+
+@pytest.mark.parametrize("S", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("rows, W", [(3, 64), (5, 30), (130, 2048)])
+def test_stream_writes_against_float64(S, rows, W):
+    g = torch.Generator().manual_seed(S * W)
+    X, y = torch.randn(S, rows, W, generator=g), torch.randn(rows, W, generator=g)
+    mix, w_out, w_in, gain = torch.randn(S, S, generator=g), torch.randn(S, generator=g), torch.randn(S, generator=g), torch.randn(W, generator=g)
+    want = torch.einsum("st,srw->trw", mix.double(), X.double()) + w_out.double()[:, None, None] * y.double()
+    wrote = X.to(DEV)
+    ops.hyper_write(wrote, y.to(DEV), mix.to(DEV), w_out.to(DEV))
+    assert float((wrote.cpu().double() - want).abs().max()) <= 3e-6 * float(want.abs().max())
+    both, h = X.to(DEV), torch.empty(rows, W, device=DEV)
+    ops.hyper_write_read_norm(both, y.to(DEV), mix.to(DEV), w_out.to(DEV), w_in.to(DEV), gain.to(DEV), 1e-5, h)
+    assert torch.equal(both.cpu(), wrote.cpu())
+    u = torch.einsum("s,srw->rw", w_in.double(), want)
+    ref = u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    assert float((h.cpu().double() - ref).abs().max()) <= 2e-5 * float(ref.abs().max())

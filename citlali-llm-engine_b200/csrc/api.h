@@ -197,6 +197,12 @@ int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int y_dtype, i
                            int mode, int force_splits, int32_t* error_flag, int sm_count,
                            void* emit_rows, float* emit_sumsq, const float* scale_sumsq, int scale_groups,
                            int scale_dim, float scale_eps, cudaStream_t stream);
+// The same with a bias (float32 [N] or null) and an activation on the float32 sums: mode bit 2 gates by gelu_tanh instead of SiLU, bit 3
+// stores bfloat16 max(v, 0)^2.
+int citlali_gemm_tc_act(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode, const float* bias,
+                        int32_t* error_flag, int sm_count, cudaStream_t stream);
+int citlali_gemm_tc_pair_act(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode, const float* bias,
+                             int32_t* error_flag, cudaStream_t stream);
 // The same product on pairs of SMs (tcgen05.mma with cta_group::2: a [256 x BN] tile per cluster of two
 // blocks, each fetching half of both operands).  With equal waves it takes 0.92-0.97 of the one-block
 // kernel's time at 512 to 4,096 rows and 0.82 at 8,192, and it loses where its 256-row tiles need a wave

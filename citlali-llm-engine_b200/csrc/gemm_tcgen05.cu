@@ -63,6 +63,7 @@ struct GemmParams {
     int scale_groups;
     int scale_dim;
     float scale_eps;
+    const float* bias;             // [N] or null (kAct only)
 };
 
 template <int BN>
@@ -88,7 +89,15 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
     return v;
 }
 
-template <int BN, bool kSwapped>
+// kAct: as in the pair kernel, the form whose epilogue adds a bias, squares or gates by GELU (tc_common.cuh).
+template <bool kFirst>
+__device__ __forceinline__ const float (&pick(const float (&)[kFirst ? 16 : 1], const float (&b)[16]))[16];
+template <>
+__device__ __forceinline__ const float (&pick<true>(const float (&a)[16], const float (&)[16]))[16] { return a; }
+template <>
+__device__ __forceinline__ const float (&pick<false>(const float (&)[1], const float (&b)[16]))[16] { return b; }
+
+template <int BN, bool kSwapped, bool kAct>
 __global__ void __launch_bounds__(threads_for(kSwapped, BN), (kSwapped && BN <= 128) ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmParams p) {
     constexpr int kStages = stages_for<BN>(kSwapped);
@@ -108,6 +117,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // memory at the very end of the kernel, which costs more than the norm kernel this saves)
     float x_old[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     bool have_old = false;
+    // kAct, few rows: the bias of the feature this lane will finish, fetched while the K loop runs for the same reason
+    float bias_ahead = 0.0f;
 
     dependents_may_launch();
     const uint32_t raw = smem_u32(smem_raw);
@@ -255,6 +266,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         __nv_bfloat16* outh = (__nv_bfloat16*)p.out;
         float gate_keep[16];
         const uint64_t out_policy = l2_evict_first_policy();
+        if (kAct && kSwapped && p.bias && p.splits > 1) {      // (a split tile's units differ by multiples of four: one feature a lane)
+            int ta, tb, sp;
+            decode(blockIdx.x, ta, tb, sp);
+            const int n = ta * kBM + (((warp - 2) * p.splits + sp) & 3) * 32 + lane;
+            if (n < p.N) bias_ahead = __ldg(p.bias + n);
+        }
         wait_for_predecessor();      // the epilogue reads and writes memory other kernels use
 
         // The factor of every row of x, if this product scales its rows: a warp adds a row's partial sums of squares in
@@ -289,11 +306,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
 
         // What becomes of 16 finished values: row i of the 128-row operand, rows j0 .. j0+15 of the other.
-        auto finish = [&](const float (&v)[16], int i, int j0, int c0) {
+        const bool gelu = kAct && p.out_kind == kGeluBF16;
+        const int out_kind = kAct && p.out_kind == kSquaredBF16 ? (int)kStoreBF16 : p.out_kind;
+        auto finish = [&](const float (&plain)[16], int i, int j0, int c0) {
+            float acted[kAct ? 16 : 1];
+            if constexpr (kAct) {
+                if constexpr (!kSwapped) {
+                    with_biases(plain, acted, p.bias, j0, p.N, p.out_kind);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) acted[c] = with_bias(plain[c], bias_ahead, p.out_kind);
+                }
+            }
+            const float(&v)[16] = pick<kAct>(acted, plain);
             if constexpr (!kSwapped) {
                 // i is a row m of x, j an output feature n
-                finish_rows(v, i, j0, c0, gate_keep, p.out, p.out_kind, p.M, p.N, epilogue_stage, lane, out_policy);
-            } else if (p.out_kind == kSwigluBF16) {
+                finish_rows<kAct>(v, i, j0, c0, gate_keep, p.out, out_kind, p.M, p.N, epilogue_stage, lane, out_policy);
+            } else if (p.out_kind == kSwigluBF16 || gelu) {
                 // i is an output feature n, j a row m of x.  Weight rows alternate in runs of 16 (gate rows, then the
                 // up rows of the same outputs): lanes 0-15 of a warp hold gate values, lanes 16-31 the matching up values
                 const int half_n = p.N >> 1;
@@ -304,7 +333,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const float mine = scaled && m < p.M ? v[c] * row_scale[m] : v[c];
                     const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
                     if ((lane & 16) == 0 && i < p.N && m < p.M)
-                        outh[(size_t)m * half_n + o_col] = __float2bfloat16_rn(silu_mul(mine, other));
+                        outh[(size_t)m * half_n + o_col] = __float2bfloat16_rn(gelu ? gelu_mul(mine, other) : silu_mul(mine, other));
                 }
             } else if (emits) {
                 // x[m, n] += v, and the updated row goes out as bfloat16 with the sum of its squares over this warp's
@@ -331,8 +360,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (m < p.M) {
                         const size_t o = (size_t)m * p.N + i;
                         const float val = scaled ? v[c] * row_scale[m] : v[c];
-                        if (p.out_kind == kStoreBF16) outh[o] = __float2bfloat16_rn(val);
-                        else if (p.out_kind == kAddF32) red_add_f32(outf + o, val);
+                        if (out_kind == kStoreBF16) outh[o] = __float2bfloat16_rn(val);
+                        else if (out_kind == kAddF32) red_add_f32(outf + o, val);
                         else outf[o] = val;
                     }
                 }
@@ -345,6 +374,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             decode(u, ta, tb, sp);
             const int kb0 = sp * kb_per_split, kb1 = min(kblocks, kb0 + kb_per_split);
             const int as = acc_it % kAccStages;
+            if (kAct && kSwapped && p.bias && p.splits == 1) {
+                const int n = ta * kBM + quarter * 32 + lane;
+                bias_ahead = n < p.N ? __ldg(p.bias + n) : 0.0f;
+            }
             const bool acc_ready = mbar_wait(smem_u32(&acc_full_bar[as]), (acc_it / kAccStages) & 1u, abort_flag, p.error_flag, 104);
             // (a split tile is its block's only unit: every thread of the cluster passes here exactly once)
             if (kSwapped && kRecvInRing && p.splits > 1) cluster_sync_all();
@@ -437,6 +470,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 float v[4] = {a.x, a.y, a.z, a.w};
                 const bool scaled = p.scale_sumsq != nullptr;
                 const bool emits = p.out_kind == kAddF32 && p.emit_rows != nullptr;
+                const bool gelu = kAct && p.out_kind == kGeluBF16;
+                if constexpr (kAct) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) v[e] = with_bias(v[e], bias_ahead, p.out_kind);
+                }
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     if (scaled && m0 + e < p.M) v[e] *= row_scale[m0 + e];
@@ -469,14 +507,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int m = m0 + e;
-                    if (p.out_kind == kSwigluBF16) {
+                    if (p.out_kind == kSwigluBF16 || gelu) {
                         // lanes 0-15 hold gate values, lanes 16-31 the up values of the same outputs
                         const float other = __shfl_xor_sync(0xffffffffu, v[e], 16);
                         if ((lane & 16) == 0 && n < p.N && m < p.M)
-                            outh[(size_t)m * (p.N >> 1) + (n >> 5) * 16 + (lane & 15)] = __float2bfloat16_rn(silu_mul(v[e], other));
+                            outh[(size_t)m * (p.N >> 1) + (n >> 5) * 16 + (lane & 15)] = __float2bfloat16_rn(gelu ? gelu_mul(v[e], other) : silu_mul(v[e], other));
                     } else if (n < p.N && m < p.M) {
                         const size_t o = (size_t)m * p.N + n;
-                        if (p.out_kind == kStoreBF16) outh[o] = __float2bfloat16_rn(v[e]);
+                        if (p.out_kind == kStoreBF16 || (kAct && p.out_kind == kSquaredBF16)) outh[o] = __float2bfloat16_rn(v[e]);
                         else if (p.out_kind == kAddF32) red_add_f32(outf + o, v[e]);      // one add per element: the same sum, no load to wait for
                         else outf[o] = v[e];
                     }
@@ -555,11 +593,11 @@ static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, b
     return pl;
 }
 
-template <int BN, bool kSwapped>
-static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
+template <int BN, bool kSwapped, bool kAct>
+static int launch_form(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
     constexpr int stages = stages_for<BN>(kSwapped);
     const size_t smem = (size_t)stages * (kBM * kBK * 2 + BN * kBK * 2) + (kSwapped ? (BN < 128 ? BN * 512 + 4096 : 0) : 8 * kEpilogueStageBytes) + 1024;      // ring, split-K receive area behind it, alignment
-    auto kernel = gemm_tc_kernel<BN, kSwapped>;
+    auto kernel = gemm_tc_kernel<BN, kSwapped, kAct>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -573,6 +611,12 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams
     const int grid = p.splits > 1 ? units : (units < sm_count * per_sm ? units : sm_count * per_sm);
     launch_kernel_clustered(kernel, grid, threads_for(kSwapped, BN), smem, p.splits > 1 ? p.splits : 1, stream, ma, mb, p);
     return CITLALI_LAUNCH_CHECK();
+}
+
+template <int BN, bool kSwapped>
+static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
+    const bool act = p.bias != nullptr || p.out_kind == kSquaredBF16 || p.out_kind == kGeluBF16;
+    return act ? launch_form<BN, kSwapped, true>(ma, mb, p, sm_count, stream) : launch_form<BN, kSwapped, false>(ma, mb, p, sm_count, stream);
 }
 
 }  // namespace tc
@@ -664,17 +708,16 @@ extern "C" int citlali_gemm_tc(const void* x, const void* w, void* y, int y_dtyp
                                   nullptr, 0, 0, 0.0f, stream);
 }
 
-// citlali_gemm_tc for few rows of x (the form with the weights as the 128-row operand: see citlali_gemm_tc_plan) with a
+// citlali_gemm_tc_normed: citlali_gemm_tc for few rows of x (the form with the weights as the 128-row operand: see citlali_gemm_tc_plan) with a
 // layer norm's work in its epilogue.  `emit_rows` / `emit_sumsq` (both or neither; mode bit 0, N a multiple of 32): the
 // product is added to the float32 rows y as always, and the updated rows also go out as bfloat16 [M, N] with the sums of
 // their squares over each 32 consecutive features, float32 [M, N / 32].  `scale_sumsq` (float32 [M, scale_groups], the
 // sums of squares of the rows of x over groups of features): every result row m is multiplied by
 // rsqrt(sum of its groups / scale_dim + scale_eps) before it is stored, gated or added.
-extern "C" int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K,
-                                      int mode, int force_splits, int32_t* error_flag, int sm_count,
-                                      void* emit_rows, float* emit_sumsq, const float* scale_sumsq, int scale_groups,
-                                      int scale_dim, float scale_eps, cudaStream_t stream) {
-    const bool accumulate = (mode & 1) != 0, swiglu = (mode & 2) != 0;
+static int gemm_tc_any(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode, int force_splits,
+                       int32_t* error_flag, int sm_count, void* emit_rows, float* emit_sumsq, const float* scale_sumsq,
+                       int scale_groups, int scale_dim, float scale_eps, const float* bias, cudaStream_t stream) {
+    const bool accumulate = (mode & 1) != 0, gelu = (mode & 4) != 0, squared = (mode & 8) != 0, swiglu = (mode & 2) != 0 || gelu;
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8 != 0) {
         set_last_error("gemm_tc: the inner size %d must be a positive multiple of 8 (rows of 16-byte multiples for TMA)", K);
@@ -713,7 +756,7 @@ extern "C" int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int
             return kBadShape;
         }
     }
-    if (runs_on_pairs(M, N, K, pl)) return citlali_gemm_tc_pair(x, w, y, y_dtype, M, N, K, mode, error_flag, stream);
+    if (runs_on_pairs(M, N, K, pl)) return citlali_gemm_tc_pair_act(x, w, y, y_dtype, M, N, K, mode, bias, error_flag, stream);
     GemmParams p;
     p.emit_rows = (__nv_bfloat16*)emit_rows; p.emit_sumsq = emit_sumsq;
     p.scale_sumsq = scale_sumsq; p.scale_groups = scale_groups; p.scale_dim = scale_dim; p.scale_eps = scale_eps;
@@ -721,7 +764,8 @@ extern "C" int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int
     p.splits = pl.splits;
     p.error_flag = error_flag;
     p.out = y;
-    p.out_kind = swiglu ? kSwigluBF16 : accumulate ? kAddF32 : (y_dtype == kF32 ? kStoreF32 : kStoreBF16);
+    p.bias = bias;
+    p.out_kind = gelu ? kGeluBF16 : squared ? kSquaredBF16 : swiglu ? kSwigluBF16 : accumulate ? kAddF32 : (y_dtype == kF32 ? kStoreF32 : kStoreBF16);
     p.rows_a = pl.swapped ? N : M;
     p.rows_b = pl.swapped ? M : N;
     CUtensorMap ma, mb;
@@ -749,4 +793,29 @@ extern "C" int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int
         }
     }
     return rc;
+}
+
+extern "C" int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K,
+                                      int mode, int force_splits, int32_t* error_flag, int sm_count,
+                                      void* emit_rows, float* emit_sumsq, const float* scale_sumsq, int scale_groups,
+                                      int scale_dim, float scale_eps, cudaStream_t stream) {
+    return gemm_tc_any(x, w, y, y_dtype, M, N, K, mode & 3, force_splits, error_flag, sm_count, emit_rows, emit_sumsq, scale_sumsq,
+                       scale_groups, scale_dim, scale_eps, nullptr, stream);
+}
+
+// citlali_gemm_tc with an activation in its epilogue, on the float32 sums: `bias` (float32 [N], 16-byte aligned, or null) is added to
+// every result row first; mode bit 2 = the gate epilogue of bit 1 with gelu_tanh(gate) * up instead of silu(gate) * up (the bias in the
+// order of w's rows); mode bit 3 = y is bfloat16 max(v, 0)^2.  At most one of the bits 1 to 3, and only bit 0 with none of them.
+extern "C" int citlali_gemm_tc_act(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode, const float* bias,
+                                   int32_t* error_flag, int sm_count, cudaStream_t stream) {
+    const int gates = mode & 14;
+    if ((mode & ~15) || (gates & (gates - 1)) || ((mode & 1) && gates) || ((mode & 8) && y_dtype != kBF16)) {
+        set_last_error("gemm_tc_act: mode %d with output dtype code %d is no form of the epilogue", mode, y_dtype);
+        return kBadShape;
+    }
+    if ((uintptr_t)bias & 15u) {
+        set_last_error("gemm_tc_act: the bias must start on a 16-byte boundary");
+        return kBadAlignment;
+    }
+    return gemm_tc_any(x, w, y, y_dtype, M, N, K, mode, 0, error_flag, sm_count, nullptr, nullptr, nullptr, 0, 0, 0.0f, bias, stream);
 }

@@ -36,13 +36,16 @@ struct Params {
     int out_kind;
     int M, N, K;
     int32_t* error_flag;
+    const float* bias;     // [N] or null (kAct only)
     int band;              // row tiles that are finished across all weight tiles before the next ones begin
 };
 
 template <int BN>
 constexpr int stages_for() { return BN <= 192 ? 7 : 6; }      // 16 KB of x and BN * 64 bytes of w a stage
 
-template <int BN>
+// kAct: the epilogue adds a bias, squares max(v, 0) or gates by the tanh form of GELU (tc_common.cuh); a form of its own, so that
+// the plain epilogue keeps its registers.
+template <int BN, bool kAct>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, Params p) {
     constexpr int kStages = stages_for<BN>();
@@ -160,7 +163,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         wait_for_predecessor();      // the epilogue reads and writes memory other kernels use
 
         auto finish = [&](const float (&v)[16], int i, int j0, int c0) {
-            finish_rows(v, i, j0, c0, gate_keep, p.out, p.out_kind, p.M, p.N, epilogue_stage, lane, out_policy);
+            if constexpr (kAct) {
+                float w[16];
+                with_biases(v, w, p.bias, j0, p.N, p.out_kind);
+                finish_rows<true>(w, i, j0, c0, gate_keep, p.out, p.out_kind == kSquaredBF16 ? (int)kStoreBF16 : p.out_kind, p.M, p.N,
+                                  epilogue_stage, lane, out_policy);
+            } else {
+                finish_rows(v, i, j0, c0, gate_keep, p.out, p.out_kind, p.M, p.N, epilogue_stage, lane, out_policy);
+            }
         };
 
         const uint32_t leader_acc_empty0 = cluster_addr(smem_u32(&acc_empty_bar[0]), 0);
@@ -211,11 +221,11 @@ static int make_map(CUtensorMap* map, const void* base, int rows, int K, int box
 }
 
 // The number of clusters of two that the device runs at once (not every SM has a partner free).
-template <int BN>
+template <int BN, bool kAct = false>
 static int resident_pairs(size_t smem) {
     static int cached = -1;
     if (cached >= 0) return cached;
-    if (cudaFuncSetAttribute(gemm_tc_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(gemm_tc_pair_kernel<BN, kAct>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -231,7 +241,7 @@ static int resident_pairs(size_t smem) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_kernel<BN>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_kernel<BN, kAct>, &cfg) != cudaSuccess || n <= 0) {
         cudaGetLastError();
         n = 0;
     }
@@ -239,12 +249,12 @@ static int resident_pairs(size_t smem) {
     return n;
 }
 
-template <int BN>
+template <int BN, bool kAct>
 static int launch(const void* x, const void* w, const Params& p, cudaStream_t stream) {
     constexpr int stages = stages_for<BN>();
     const size_t smem = (size_t)stages * (kBM * kBK * 2 + (BN / 2) * kBK * 2) + kEpilogueWarps * kEpilogueStageBytes + 1024;
-    auto kernel = gemm_tc_pair_kernel<BN>;
-    const int pairs_max = resident_pairs<BN>(smem);
+    auto kernel = gemm_tc_pair_kernel<BN, kAct>;
+    const int pairs_max = resident_pairs<BN, kAct>(smem);
     if (pairs_max <= 0) {
         set_last_error("gemm_tc_pair: the device runs no cluster of two blocks with %zu bytes of shared memory", smem);
         return kTooLarge;
@@ -289,7 +299,13 @@ extern "C" int citlali_gemm_tc_pair_plan(int M, int N, int K, int* bn, int* pair
 // For many rows of x; it takes every M, N and K that citlali_gemm_tc takes.
 extern "C" int citlali_gemm_tc_pair(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K,
                                     int mode, int32_t* error_flag, cudaStream_t stream) {
-    const bool accumulate = (mode & 1) != 0, swiglu = (mode & 2) != 0;
+    return citlali_gemm_tc_pair_act(x, w, y, y_dtype, M, N, K, mode, nullptr, error_flag, stream);
+}
+
+// The same with a bias and the further `mode` bits of citlali_gemm_tc_act, which checks them.
+extern "C" int citlali_gemm_tc_pair_act(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode,
+                                        const float* bias, int32_t* error_flag, cudaStream_t stream) {
+    const bool accumulate = (mode & 1) != 0, gelu = (mode & 4) != 0, swiglu = (mode & 2) != 0 || gelu;
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8 != 0) {
         set_last_error("gemm_tc_pair: the inner size %d must be a positive multiple of 8 (rows of 16-byte multiples for TMA)", K);
@@ -321,6 +337,8 @@ extern "C" int citlali_gemm_tc_pair(const void* x, const void* w, void* y, int y
     }
     p.error_flag = error_flag;
     p.out = y;
-    p.out_kind = swiglu ? tc::kSwigluBF16 : accumulate ? tc::kAddF32 : (y_dtype == kF32 ? tc::kStoreF32 : tc::kStoreBF16);
-    return N >= 256 ? tc::pair::launch<256>(x, w, p, stream) : tc::pair::launch<128>(x, w, p, stream);
+    p.bias = bias;
+    p.out_kind = gelu ? tc::kGeluBF16 : (mode & 8) ? tc::kSquaredBF16 : swiglu ? tc::kSwigluBF16 : accumulate ? tc::kAddF32 : (y_dtype == kF32 ? tc::kStoreF32 : tc::kStoreBF16);
+    if (bias || (mode & 12)) return N >= 256 ? tc::pair::launch<256, true>(x, w, p, stream) : tc::pair::launch<128, true>(x, w, p, stream);
+    return N >= 256 ? tc::pair::launch<256, false>(x, w, p, stream) : tc::pair::launch<128, false>(x, w, p, stream);
 }

@@ -576,6 +576,24 @@ def gemm_tc(x, w, y, accumulate=False, error_flag=None, swiglu=False, force_spli
            "gemm_tc")
 
 
+_GEMM_ACTS = {None: 0, "gelu_gate": 4, "relu_squared": 8}
+
+
+def gemm_tc_act(x, w, y, accumulate=False, bias=None, act=None, error_flag=None):
+    """:func:`gemm_tc` with an activation in the epilogue, on the float32 sums: ``bias`` (float32 [N]) is added first; ``act``
+    "gelu_gate": ``w``'s rows alternate gate/up in runs of 16 (the bias with them) and ``y`` is bfloat16 [M, N/2] =
+    gelu_tanh(gate) * up; "relu_squared": ``y`` is bfloat16 max(v, 0)^2."""
+    _need_cuda(x, w, y, bias, error_flag)
+    M, K = x.shape
+    N = w.shape[0]
+    require(gemm_tc_accepts(x, w, y) and w.shape[1] == K and y.shape == (M, N // 2 if act == "gelu_gate" else N)
+            and (bias is None or (bias.dtype == torch.float32 and bias.numel() == N)) and act in _GEMM_ACTS,
+            "gemm_tc_act: shapes or dtypes do not fit")
+    _check(lib().citlali_gemm_tc_act(_ptr(x), _ptr(w), _ptr(y), _i(_dtype_code(y)), _i(M), _i(N), _i(K),
+                                     _i(_GEMM_ACTS[act] | (1 if accumulate else 0)), _ptr(bias), _ptr(error_flag), _i(sm_count(x.device)),
+                                     _stream()), "gemm_tc_act")
+
+
 # ---- residual streams --------------------------------------------------------------------------
 
 _sz = ctypes.c_size_t

@@ -7,8 +7,8 @@ and matching gate and up values lie next to each other for the gate kernel.
 Parameters: hidden_size, intermediate_size; optional ``activation`` ("silu", the default, or "gelu_tanh": z / 2 (1 +
 tanh(sqrt(2 / pi) (z + 0.044715 z^3)))), ``biases`` (true: gate, up and down have a bias each) and ``names``: the full
 tensor names by role (gate, up, down, gate_bias, up_bias, down_bias; a bias defaults to its matrix's name with ``.b``).
-With another activation than SiLU, or with biases, the gate and up product keeps its float32 result, and bias,
-activation and gate are one kernel with one rounding at its store.
+With another activation than SiLU, or with biases, bias, activation and gate work on the gate and up product's float32 sums
+with one rounding at the store: in the product's epilogue (GELU, shapes the tensor-core product takes) or in a kernel behind it.
 """
 from __future__ import annotations
 
@@ -83,15 +83,18 @@ class GatedSiluFeedForward:
         ``overwrite``: ``residual`` holds nothing yet and receives the output.  ``defer_bias``: the caller adds
         ``deferred_bias`` (the output's bias) itself."""
         if not self.plain:
-            gu = self.gate_up.forward(h, out_dtype=torch.float32)
-            act = torch.empty((h.shape[0], self.inter), dtype=self.dtype, device=h.device)
-            ops.expert_gate(gu, None, act, 0, 0, 1, self.activation, tail_ff=self.inter, tail_run=self.run, bias=self.bias)
-            if overwrite:
-                self.down.forward(act, out=residual)
-            else:
-                self.down.forward(act, accumulate_into=residual)
-            if self.deferred_bias is not None and not defer_bias:
-                ops.add_row_bias(residual, self.deferred_bias)
+            act = self.gate_up.forward_act(h, "gelu_gate", self.bias) if self.activation == "gelu_tanh" else None
+            if act is None:
+                gu = self.gate_up.forward(h, out_dtype=torch.float32)
+                act = torch.empty((h.shape[0], self.inter), dtype=self.dtype, device=h.device)
+                ops.expert_gate(gu, None, act, 0, 0, 1, self.activation, tail_ff=self.inter, tail_run=self.run, bias=self.bias)
+            bias = None if defer_bias else self.deferred_bias
+            target = {"out": residual} if overwrite else {"accumulate_into": residual}
+            if bias is not None and self.down.forward_act(act, bias=bias, **target) is not None:
+                return residual
+            self.down.forward(act, **target)
+            if bias is not None:
+                ops.add_row_bias(residual, bias)
             return residual
         if isinstance(h, NormedRows):
             act = self.gate_up.forward_gated(h.rows, self.run, row_scale=h.scale)
@@ -130,8 +133,10 @@ class SquaredReluFeedForward:
 
     def forward(self, h, batch, residual, overwrite=False):
         """``overwrite``: ``residual`` holds nothing yet and receives the output instead of being added to."""
-        z = self.up.forward(h)
-        ops.relu_squared(z, z)
+        z = self.up.forward_act(h, "relu_squared")
+        if z is None:
+            z = self.up.forward(h)
+            ops.relu_squared(z, z)
         if overwrite:
             self.down.forward(z, out=residual)
         else:

@@ -105,6 +105,20 @@ class DenseLinear:
         ops.gemm_tc(x, self.weight, act, error_flag=self.error_flag, swiglu=True, row_scale=row_scale)
         return act
 
+    def forward_act(self, x: torch.Tensor, act: Optional[str] = None, bias: Optional[torch.Tensor] = None,
+                    accumulate_into: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None):
+        """The product with a bias and an activation in its epilogue (``ops.gemm_tc_act``), or ``None`` where the tensor-core product
+        does not take it: a new bfloat16 matrix, ``accumulate_into`` or ``out``."""
+        rows = x.shape[0]
+        if (rows == 0 or not self.uses_tensor_cores(x) or (bias is not None and bias.data_ptr() % 16 != 0)
+                or (act == "gelu_gate" and (self.interleave_run != 16 or self.out_features % 32 != 0))):
+            return None
+        y = accumulate_into if accumulate_into is not None else out
+        if y is None:
+            y = torch.empty((rows, self.out_features // 2 if act == "gelu_gate" else self.out_features), dtype=torch.bfloat16, device=x.device)
+        ops.gemm_tc_act(x, self.weight, y, accumulate=accumulate_into is not None, bias=bias, act=act, error_flag=self.error_flag)
+        return y
+
     def forward(self, x: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                 accumulate_into: Optional[torch.Tensor] = None, row_scale=None, emit=None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:

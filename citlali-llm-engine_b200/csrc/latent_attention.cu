@@ -284,6 +284,78 @@ heads_product_mma_kernel(const TX* __restrict__ x, size_t x_row, int x_head, con
         rotate_tail(x, x_row, x_head, y, y_row, y_head, h, row0, 64, rows, K, N, tail, inv_freq, rot_dims, row_pos, rot_halves);
 }
 
+// The same for few rows (decoding), where the kernel above walks k in tiles that nobody hides and pads the rows to 64: a block owns 16
+// rows and 16 columns of a head, its eight warps share k between them, every operand is read from memory straight into an MMA's
+// registers (all of a warp's reads at once), and the warps' sums meet in shared memory, added in warp order.  Matrices whose k lies
+// contiguously, K a multiple of 16, x in float32.  Bound by the latency of one round of reads.
+// 8 rows, 16 heads, K x N = 128 x 512 and 512 x 128: 6.2 and 5.0 us, above 16 and 32 us.
+constexpr int kFewRows = 16;
+
+template <typename TY>
+__global__ void __launch_bounds__(256)
+heads_product_few_kernel(const float* x, size_t x_row, int x_head, const __nv_bfloat16* __restrict__ M, size_t m_head, int m_n,
+                         TY* y, size_t y_row, int y_head, int rows, int K, int N, int tail, const float* inv_freq, int rot_dims,
+                         const int32_t* row_pos, const float* gate, size_t gate_stride, int rot_halves, int gate_per_head) {
+    // (Only the matrix is declared unaliased: a read that the compiler may take for one of constant memory may also be moved ahead
+    // of the wait below, and x, the gate and the positions are the kernels' before this one.)
+    __shared__ float part[8][16][17];
+    dependents_may_launch();
+    const int h = blockIdx.y, row0 = blockIdx.x * 16, n0 = blockIdx.z * 16;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const __nv_bfloat16* Mh = M + (size_t)h * m_head;
+    const int steps = K / 16, per = (steps + 7) / 8, s0 = warp * per, s1 = min(steps, s0 + per);
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    const float* xa = x + (size_t)(row0 + g) * x_row + (size_t)h * x_head;
+    const float* xb = xa + 8 * x_row;
+    const bool on_a = row0 + g < rows, on_b = row0 + g + 8 < rows;
+    bool first = true;
+    for (int s = s0; s < s1; s += 4) {
+        uint32_t b[4][2][2], a[4][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)                           // the matrix is written by no kernel: its first reads go out ahead of the wait
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int n = n0 + j * 8 + g, k = (s + u) * 16 + t * 2;
+                const bool on = s + u < s1 && n < N;
+                const uint32_t* m = reinterpret_cast<const uint32_t*>(Mh + (size_t)n * m_n + k);
+                b[u][j][0] = on ? __ldg(m) : 0u;
+                b[u][j][1] = on ? __ldg(m + 4) : 0u;
+            }
+        if (first) { wait_for_predecessor(); first = false; }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = (s + u) * 16 + t * 2;
+            const bool on = s + u < s1;
+            const float2 zero = make_float2(0.f, 0.f);
+            const float2 v0 = on && on_a ? *reinterpret_cast<const float2*>(xa + k) : zero, v2 = on && on_a ? *reinterpret_cast<const float2*>(xa + k + 8) : zero;
+            const float2 v1 = on && on_b ? *reinterpret_cast<const float2*>(xb + k) : zero, v3 = on && on_b ? *reinterpret_cast<const float2*>(xb + k + 8) : zero;
+            a[u][0] = fa::pack_bf16(v0.x, v0.y); a[u][1] = fa::pack_bf16(v1.x, v1.y);
+            a[u][2] = fa::pack_bf16(v2.x, v2.y); a[u][3] = fa::pack_bf16(v3.x, v3.y);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) fa::mma_16816(acc[j], a[u][0], a[u][1], a[u][2], a[u][3], b[u][j][0], b[u][j][1]);
+    }
+    if (first) wait_for_predecessor();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        part[warp][g][j * 8 + t * 2] = acc[j][0]; part[warp][g][j * 8 + t * 2 + 1] = acc[j][1];
+        part[warp][g + 8][j * 8 + t * 2] = acc[j][2]; part[warp][g + 8][j * 8 + t * 2 + 1] = acc[j][3];
+    }
+    __syncthreads();
+    const int r = threadIdx.x >> 4, c = threadIdx.x & 15, row = row0 + r, n = n0 + c;
+    if (row < rows && n < N) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += part[w][r][c];
+        if (gate) v *= 1.0f / (1.0f + expf(-gate[(size_t)row * gate_stride + (gate_per_head ? (size_t)h : (size_t)h * N + n)]));
+        stf(y, (size_t)row * y_row + (size_t)h * y_head + n, v);
+    }
+    if (tail > 0 && blockIdx.z == 0)
+        rotate_tail(x, x_row, x_head, y, y_row, y_head, h, row0, 16, rows, K, N, tail, inv_freq, rot_dims, row_pos, rot_halves);
+}
+
 // q [rows, H, E] float32 (E = R + P: the query in the latent's coordinates, then its rotated part); the cache's pool
 // [page, page_size, E]; out [rows, H, R] float32 = sum_j p_j c_j.  NC * 32 >= E.
 template <typename TC, int NC>
@@ -379,6 +451,16 @@ extern "C" int citlali_heads_product(const void* x, int x_dtype, size_t x_row, i
     if (tail > 0 && (rot_dims > tail || (rot_dims & 1) || (rot_dims > 0 && (!inv_freq || !row_pos)))) {
         set_last_error("heads_product: %d rotated dimensions of a tail of %d", rot_dims, tail);
         return kBadShape;
+    }
+    // few rows: up to 16, with the alignment that reads of two floats and two bfloat16 want
+    if (m_dtype == kBF16 && x_dtype == kF32 && rows <= kFewRows && m_k == 1 && K % 16 == 0 && m_n % 2 == 0 && m_head % 2 == 0 && x_row % 2 == 0 &&
+        x_head % 2 == 0 && ((uintptr_t)x & 7u) == 0 && ((uintptr_t)M & 3u) == 0 && (N + 15) / 16 <= 65535) {
+        dim3 grid((rows + 15) / 16, heads, (N + 15) / 16);
+        return CITLALI_DISPATCH_FLOAT(y_dtype, TY, [&] {
+            launch_kernel(heads_product_few_kernel<TY>, grid, 256, 0, stream, (const float*)x, x_row, x_head, (const __nv_bfloat16*)M, m_head, m_n,
+                          (TY*)y, y_row, y_head, rows, K, N, tail, inv_freq, rot_dims, row_pos, gate, gate_stride, rot_halves, gate_per_head);
+            return CITLALI_LAUNCH_CHECK();
+        });
     }
     if (m_dtype == kBF16) {
         dim3 grid((rows + 63) / 64, heads, (N + 63) / 64);

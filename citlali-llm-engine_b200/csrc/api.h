@@ -254,7 +254,8 @@ int citlali_delta_prepare(const float* proj, int proj_stride, const float* taps_
                           const int32_t* seq_slot, int sequences, const float* a_log, const float* dt_bias, float* prep,
                           int rows, int H, int KH, int D, int V, float unit_eps, int block_a_segment, int beta_col,
                           int decay_col, const float* decay_in, int decay_stride, int channel_decay, cudaStream_t stream);
-// (beta_col, decay_col: the columns of b and a in a row of proj.  decay_in (rows decay_stride floats apart) given: the
+// (block_a_segment 1: a block a segment, for few rows; 2: the same, for a step of one row a sequence, in one launch.
+// beta_col, decay_col: the columns of b and a in a row of proj.  decay_in (rows decay_stride floats apart) given: the
 // decays' inputs come from there instead of proj.  channel_decay: one decay a head and key channel instead of one a head,
 // g = exp(-exp(a_log[h]) softplus(decay_in[h D + i] + dt_bias[h D + i])); prep is then [rows, C + H + H D].)
 // The recurrence over each sequence's rows, from and into state[slot][0 ...] = S [H, D, V]; out [rows, H V] float32.
@@ -264,6 +265,10 @@ int citlali_delta_prepare(const float* proj, int proj_stride, const float* taps_
 int citlali_delta_rule(const float* prep, int prep_stride, float* state, size_t state_stride, const int32_t* seq_start,
                        const int32_t* seq_slot, int sequences, int H, int KH, int D, int V, float* out, int pairs, int mode,
                        cudaStream_t stream);
+// citlali_delta_rule in mode 0 or 1 and citlali_delta_output for a step in which every sequence brings one token (V at most 128).
+int citlali_delta_step(const float* prep, int prep_stride, float* state, size_t state_stride, const int32_t* seq_start,
+                       const int32_t* seq_slot, int sequences, int H, int KH, int D, int V, int mode, const float* gate,
+                       int gate_stride, const float* weight, void* y, int y_dtype, float eps, int gate_act, cudaStream_t stream);
 // The recurrence in mode 0 over runs of tokens, 32 at a time (the same numbers up to the order of the sums): two launches.  max_new:
 // the longest sequence's rows; D at most 128, and D, V and prep_stride multiples of four.  scratch: 16-byte aligned, as many floats
 // as citlali_delta_chunks_scratch_floats says for the step's rows.

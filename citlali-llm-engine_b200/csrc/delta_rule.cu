@@ -206,13 +206,14 @@ delta_prepare_run_kernel(const float* __restrict__ proj, int proj_stride, const 
 }
 
 // The same with a block of 128 threads a segment, a thread a channel: for steps of few rows, where a row's segments
-// are all the parallelism there is.  (It sums a head's squares in another order than the kernel above.)
+// are all the parallelism there is.  (It sums a head's squares in another order than the kernel above.)  keep: every sequence has one
+// row here, and the channels' kept inputs move on as well (delta_conv_state_kernel's work).
 __global__ void __launch_bounds__(128)
 delta_prepare_block_kernel(const float* __restrict__ proj, int proj_stride, const float* __restrict__ taps_w, int taps,
-                     const float* __restrict__ state, size_t state_stride, size_t conv_off,
+                     float* state, size_t state_stride, size_t conv_off,
                      const int32_t* __restrict__ row_slot, const float* __restrict__ a_log,
                      const float* __restrict__ dt_bias, float* __restrict__ prep, int H, int KH, int D, int V, float unit_eps,
-                     int beta_col, int decay_col, const float* __restrict__ decay_in, int decay_stride, int channel_decay) {
+                     int beta_col, int decay_col, const float* __restrict__ decay_in, int decay_stride, int channel_decay, int keep) {
     extern __shared__ float act[];          // max(D, V) floats
     __shared__ float scratch[32];
     dependents_may_launch();
@@ -225,7 +226,7 @@ delta_prepare_block_kernel(const float* __restrict__ proj, int proj_stride, cons
     const int slot = row_slot[row];
     int in_step = 0;                        // how many of the tokens before this one are rows of this step
     while (in_step < taps - 1 && row - in_step - 1 >= 0 && row_slot[row - in_step - 1] == slot) ++in_step;
-    const float* kept = state + (size_t)slot * state_stride + conv_off;
+    float* kept = state + (size_t)slot * state_stride + conv_off;
     float ss = 0.0f;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int c = c0 + i;
@@ -235,6 +236,10 @@ delta_prepare_block_kernel(const float* __restrict__ proj, int proj_stride, cons
             if (j <= in_step) x = proj[(size_t)(row - j) * proj_stride + c];
             else x = kept[(size_t)(taps - 1 - j + in_step) * C + c];
             acc = fmaf(taps_w[(size_t)c * taps + (taps - 1 - j)], x, acc);
+        }
+        if (keep) {                                           // (the row is its sequence's only one: nobody else reads these inputs)
+            for (int j = 0; j < taps - 2; ++j) kept[(size_t)j * C + c] = kept[(size_t)(j + 1) * C + c];
+            if (taps > 1) kept[(size_t)(taps - 2) * C + c] = proj[(size_t)row * proj_stride + c];
         }
         const float v = siluf_(acc);
         act[i] = v;
@@ -477,6 +482,98 @@ delta_rule_kernel(const float* __restrict__ prep, int prep_stride, float* __rest
     }
 }
 
+// A step in which every sequence brings one token: the recurrence and the output's norm and gate (delta_output) of one (sequence, head)
+// in one block, a warp for eight columns as in delta_rule_kernel, whose numbers these are.  The state is the bulk of what a decoding
+// step moves here (64 KB a head of 128 x 128, in and out): it is on its way to L2 while the kernel ahead still runs, and the output
+// never goes to memory unnormed.  8 sequences, 32 heads of 128 x 128: 14.6 us with caches cold (20 in
+// two kernels); a Lanizen step of three such layers 599 -> 579 us, the preparation in one launch instead of two among it.
+// MODE 0: one decay a head.  MODE 1: a decay a key channel.  V at most 128.
+template <int DP, int MODE, typename TO>
+__global__ void __launch_bounds__(512)
+delta_step_kernel(const float* prep, int prep_stride, float* state, size_t state_stride, const int32_t* __restrict__ seq_start,
+                  const int32_t* __restrict__ seq_slot, int H, int KH, int D, int V, const float* gate, int gate_stride,
+                  const float* __restrict__ weight, TO* y, float eps, int gate_act) {
+    __shared__ __align__(16) float ks[DP], qs[DP], gs[MODE == 1 ? DP : 4];
+    __shared__ float os[128];
+    dependents_may_launch();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = lane & 3;
+    const int head = blockIdx.x, seq = blockIdx.y, row = seq_start[seq];
+    const int col = warp * 8 + (lane >> 2);
+    const bool live = col < V;
+    float* S_h = state + (size_t)seq_slot[seq] * state_stride + (size_t)head * D * V;
+    for (int i = tid * 32; i < D * V; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(S_h + i));
+    wait_for_predecessor();
+    constexpr int GROUPS = DP / 16;
+    float S[GROUPS][4];
+#pragma unroll
+    for (int j = 0; j < GROUPS; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int i = (4 * j + part) * 4 + e;
+            S[j][e] = (live && i < D) ? S_h[(size_t)i * V + col] : 0.0f;
+        }
+    const int C = 2 * KH * D + H * V, kv_head = head / (H / KH);
+    const float* p = prep + (size_t)row * prep_stride;
+    for (int i = tid; i < DP; i += blockDim.x) {
+        ks[i] = i < D ? p[(KH + kv_head) * D + i] : 0.0f;
+        qs[i] = i < D ? p[kv_head * D + i] : 0.0f;
+        if (MODE == 1) gs[i] = i < D ? p[C + H + head * D + i] : 0.0f;
+    }
+    const float v = live ? p[2 * KH * D + head * V + col] : 0.0f, beta = p[C + head];
+    const float g = MODE == 1 ? 1.0f : p[C + H + head];
+    __syncthreads();
+    if (MODE == 1) {
+#pragma unroll
+        for (int j = 0; j < GROUPS; ++j) {
+            const float4 g4 = *reinterpret_cast<const float4*>(gs + (4 * j + part) * 4);
+            S[j][0] *= g4.x; S[j][1] *= g4.y; S[j][2] *= g4.z; S[j][3] *= g4.w;
+        }
+    }
+    float sk0 = 0.0f, sk1 = 0.0f, sk2 = 0.0f, sk3 = 0.0f;
+#pragma unroll
+    for (int j = 0; j < GROUPS; ++j) {
+        const float4 k4 = *reinterpret_cast<const float4*>(ks + (4 * j + part) * 4);
+        sk0 = fmaf(S[j][0], k4.x, sk0); sk1 = fmaf(S[j][1], k4.y, sk1);
+        sk2 = fmaf(S[j][2], k4.z, sk2); sk3 = fmaf(S[j][3], k4.w, sk3);
+    }
+    float sk = (sk0 + sk1) + (sk2 + sk3);
+    sk += __shfl_xor_sync(0xffffffffu, sk, 1);
+    sk += __shfl_xor_sync(0xffffffffu, sk, 2);
+    const float u = beta * (v - g * sk);
+    float o0 = 0.0f, o1 = 0.0f, o2 = 0.0f, o3 = 0.0f;
+#pragma unroll
+    for (int j = 0; j < GROUPS; ++j) {
+        const float4 k4 = *reinterpret_cast<const float4*>(ks + (4 * j + part) * 4);
+        const float4 q4 = *reinterpret_cast<const float4*>(qs + (4 * j + part) * 4);
+        S[j][0] = fmaf(k4.x, u, g * S[j][0]); o0 = fmaf(S[j][0], q4.x, o0);
+        S[j][1] = fmaf(k4.y, u, g * S[j][1]); o1 = fmaf(S[j][1], q4.y, o1);
+        S[j][2] = fmaf(k4.z, u, g * S[j][2]); o2 = fmaf(S[j][2], q4.z, o2);
+        S[j][3] = fmaf(k4.w, u, g * S[j][3]); o3 = fmaf(S[j][3], q4.w, o3);
+    }
+    if (live) {
+#pragma unroll
+        for (int j = 0; j < GROUPS; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = (4 * j + part) * 4 + e;
+                if (i < D) S_h[(size_t)i * V + col] = S[j][e];
+            }
+    }
+    float o = (o0 + o1) + (o2 + o3);
+    o += __shfl_xor_sync(0xffffffffu, o, 1);
+    o += __shfl_xor_sync(0xffffffffu, o, 2);
+    if (live && part == 0) os[col] = o;
+    __syncthreads();
+    float ss = 0.0f;                                          // every warp the whole sum, in delta_output's order
+    for (int i = lane; i < V; i += 32) ss = fmaf(os[i], os[i], ss);
+    ss = warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)V + eps);
+    if (tid < V) {
+        const float z = gate[(size_t)row * gate_stride + head * V + tid];
+        stf(y, ((size_t)row * H + head) * V + tid, os[tid] * inv * weight[tid] * (gate_act == 1 ? sigmoidf_(z) : siluf_(z)));
+    }
+}
+
 // y[row, h, :] = o[row, h, :] / sqrt(mean(o^2) + eps) * weight * act(gate[row, h, :]), act = SiLU (gate_act 0) or the
 // sigmoid (1).  One warp a head.
 template <typename TO>
@@ -509,6 +606,12 @@ extern "C" int citlali_delta_prepare(const float* proj, int proj_stride, const f
                                      int D, int V, float unit_eps, int block_a_segment, int beta_col, int decay_col,
                                      const float* decay_in, int decay_stride, int channel_decay, cudaStream_t stream) {
     if (rows <= 0) return 0;
+    // block_a_segment 2: every sequence has one row, and the same kernel keeps the inputs
+    const bool keeps = block_a_segment == 2;
+    if (keeps && rows != sequences) {
+        set_last_error("delta_prepare: %d rows of %d sequences are not one each", rows, sequences);
+        return kBadShape;
+    }
     if (H <= 0 || KH <= 0 || H % KH != 0 || D <= 0 || V <= 0 || taps < 1 || (channel_decay && !decay_in)) {
         set_last_error("delta_prepare: %d heads over %d key heads of %d, values of %d, %d taps (a decay per channel comes in a buffer of its own)", H, KH, D, V, taps);
         return kBadShape;
@@ -527,8 +630,8 @@ extern "C" int citlali_delta_prepare(const float* proj, int proj_stride, const f
         }
         dim3 prepare_grid(rows, segments);
         launch_kernel(delta_prepare_block_kernel, prepare_grid, 128, smem, stream, proj, proj_stride, taps_w, taps,
-                      (const float*)state, state_stride, conv_off, row_slot, a_log, dt_bias, prep, H, KH, D, V, unit_eps,
-                      beta_col, decay_col, decay_in, decay_stride, channel_decay);
+                      state, state_stride, conv_off, row_slot, a_log, dt_bias, prep, H, KH, D, V, unit_eps,
+                      beta_col, decay_col, decay_in, decay_stride, channel_decay, keeps ? 1 : 0);
     } else if (taps >= 2 && taps <= 4 && D <= 256 && V <= 256) {
         dim3 prepare_grid((rows + kPrepareRun - 1) / kPrepareRun, (segments + 3) / 4);
         const bool narrow = D <= 128 && V <= 128;
@@ -544,7 +647,7 @@ extern "C" int citlali_delta_prepare(const float* proj, int proj_stride, const f
                       decay_in, decay_stride, channel_decay);
     }
     int code = CITLALI_LAUNCH_CHECK();
-    if (code != 0 || taps == 1) return code;
+    if (code != 0 || taps == 1 || keeps) return code;
     dim3 grid(sequences, (C + 127) / 128);
     launch_kernel(delta_conv_state_kernel, grid, 128, 0, stream, proj, proj_stride, taps, state, state_stride, conv_off,
                   seq_start, seq_slot, C);
@@ -598,5 +701,39 @@ extern "C" int citlali_delta_output(const float* o, const float* gate, int gate_
         dim3 grid(rows, (H + 7) / 8 < 64 ? (H + 7) / 8 : 64);             // a warp a head, eight heads a block
         launch_kernel(delta_output_kernel<TO>, grid, 256, 0, stream, o, gate, gate_stride, weight, (TO*)y, H, V, eps, gate_act);
         return CITLALI_LAUNCH_CHECK();
+    });
+}
+
+// delta_rule (mode 0 or 1) and delta_output for a step in which every sequence brings one token; V at most 128, D at most 256.
+template <int MODE, typename TO>
+static int launch_delta_step(const float* prep, int prep_stride, float* state, size_t state_stride, const int32_t* seq_start,
+                             const int32_t* seq_slot, int sequences, int H, int KH, int D, int V, const float* gate, int gate_stride,
+                             const float* weight, void* y, float eps, int gate_act, cudaStream_t stream) {
+    const int threads = 32 * ((V + 7) / 8);
+#define CITLALI_DELTA_STEP(DP)                                                                                                       \
+    launch_kernel(delta_step_kernel<DP, MODE, TO>, dim3(H, sequences), threads, 0, stream, prep, prep_stride, state, state_stride,   \
+                  seq_start, seq_slot, H, KH, D, V, gate, gate_stride, weight, (TO*)y, eps, gate_act)
+    if (D <= 32) CITLALI_DELTA_STEP(32);
+    else if (D <= 64) CITLALI_DELTA_STEP(64);
+    else if (D <= 128) CITLALI_DELTA_STEP(128);
+    else CITLALI_DELTA_STEP(256);
+#undef CITLALI_DELTA_STEP
+    return CITLALI_LAUNCH_CHECK();
+}
+
+extern "C" int citlali_delta_step(const float* prep, int prep_stride, float* state, size_t state_stride, const int32_t* seq_start,
+                                  const int32_t* seq_slot, int sequences, int H, int KH, int D, int V, int mode, const float* gate,
+                                  int gate_stride, const float* weight, void* y, int y_dtype, float eps, int gate_act,
+                                  cudaStream_t stream) {
+    if (sequences <= 0) return 0;
+    if (mode < 0 || mode > 1 || H <= 0 || KH <= 0 || H % KH != 0 || D <= 0 || D > 256 || V <= 0 || V > 128 || sequences > 65535) {
+        set_last_error("delta_step: form %d, %d heads over %d key heads of %d, values of %d", mode, H, KH, D, V);
+        return kBadShape;
+    }
+    return CITLALI_DISPATCH_FLOAT(y_dtype, TO, [&] {
+        return mode == 1 ? launch_delta_step<1, TO>(prep, prep_stride, state, state_stride, seq_start, seq_slot, sequences, H, KH, D, V, gate,
+                                                    gate_stride, weight, y, eps, gate_act, stream)
+                         : launch_delta_step<0, TO>(prep, prep_stride, state, state_stride, seq_start, seq_slot, sequences, H, KH, D, V, gate,
+                                                    gate_stride, weight, y, eps, gate_act, stream);
     });
 }

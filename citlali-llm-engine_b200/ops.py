@@ -655,11 +655,12 @@ def relu_squared(x: torch.Tensor, y: torch.Tensor):
 
 def delta_prepare(proj, taps_w, state, conv_off, row_slot, seq_start, seq_slot, sequences, a_log, dt_bias, prep,
                   H, KH, D, V, unit_eps, block_a_segment=False, beta_col=None, decay_col=None, decay_in=None,
-                  channel_decay=False):
+                  channel_decay=False, one_row_each=False):
     """See ``citlali_delta_prepare`` (csrc/api.h).  ``state`` [slots, n] float32; two launches unless taps == 1.
     ``beta_col`` / ``decay_col``: the columns of b and a in a row of ``proj`` (default: behind q, k, v and a gate of H V
     columns).  ``decay_in``: the decays' inputs in a tensor of their own (a view whose rows may be further apart than its
-    width).  ``channel_decay``: a decay per head and key channel, ``prep`` is then [rows, C + H + H D]."""
+    width).  ``channel_decay``: a decay per head and key channel, ``prep`` is then [rows, C + H + H D].  ``block_a_segment``:
+    for few rows; with ``one_row_each`` (every sequence brings one row) the same launch also keeps the inputs."""
     _need_cuda(proj, taps_w, state, row_slot, seq_start, seq_slot, a_log, dt_bias, prep)
     rows = proj.shape[0]
     C = 2 * KH * D + H * V
@@ -682,10 +683,10 @@ def delta_prepare(proj, taps_w, state, conv_off, row_slot, seq_start, seq_slot, 
     _check(lib().citlali_delta_prepare(_ptr(proj), _i(proj.shape[1]), _ptr(taps_w), _i(taps), _ptr(state),
                                        _sz(state.shape[1]), _sz(conv_off), _ptr(row_slot), _ptr(seq_start), _ptr(seq_slot),
                                        _i(sequences), _ptr(a_log), _ptr(dt_bias), _ptr(prep), _i(rows), _i(H), _i(KH),
-                                       _i(D), _i(V), _f(unit_eps), _i(1 if block_a_segment else 0), _i(beta_col),
+                                       _i(D), _i(V), _f(unit_eps), _i((2 if one_row_each else 1) if block_a_segment else 0), _i(beta_col),
                                        _i(decay_col), _ptr(decay_in), _i(decay_stride), _i(1 if channel_decay else 0),
                                        _stream()),
-           "delta_prepare" if taps == 1 else "delta_prepare_kept")
+           "delta_prepare" if taps == 1 or (block_a_segment and one_row_each) else "delta_prepare_kept")
 
 
 _KERNELS_PER_CALL["delta_prepare_kept"] = 2
@@ -729,6 +730,19 @@ def delta_chunks(prep, state, seq_start, seq_slot, sequences, max_new, H, KH, D,
 
 
 _KERNELS_PER_CALL["delta_chunks"] = 2
+
+
+def delta_step(prep, state, seq_start, seq_slot, sequences, H, KH, D, V, gate, gate_stride, weight, y, eps, gate_act="silu",
+               mode=DELTA_HEAD_DECAY):
+    """:func:`delta_rule` and :func:`delta_output` for a step in which every sequence brings one token; ``V`` at most 128."""
+    _need_cuda(prep, state, seq_start, seq_slot, weight, y)
+    require(prep.dtype == torch.float32 and state.dtype == torch.float32 and prep.shape[0] == sequences and state.shape[1] >= H * D * V
+            and prep.shape[1] == 2 * KH * D + H * V + H + H * (D if mode == DELTA_CHANNEL_DECAY else 1)
+            and gate.is_cuda and gate.dtype == torch.float32 and weight.dtype == torch.float32 and weight.numel() == V
+            and y.shape == (sequences, H * V) and gate_act in ("silu", "sigmoid"), "delta_step: shapes or dtypes do not fit")
+    _check(lib().citlali_delta_step(_ptr(prep), _i(prep.shape[1]), _ptr(state), _sz(state.shape[1]), _ptr(seq_start), _ptr(seq_slot),
+                                    _i(sequences), _i(H), _i(KH), _i(D), _i(V), _i(mode), _ptr(gate), _i(gate_stride), _ptr(weight),
+                                    _ptr(y), _i(_dtype_code(y)), _f(eps), _i(1 if gate_act == "sigmoid" else 0), _stream()), "delta_step")
 
 
 def delta_output(o, gate, gate_stride, weight, y, H, V, eps, gate_act="silu"):

@@ -134,20 +134,27 @@ class GatedDeltaMixer:
         rows, hv = batch.rows, self.H * self.V
         proj = self.proj.forward(h, out_dtype=torch.float32)
         few = self.dtype == torch.bfloat16 and rows < 64
+        each = few and batch.is_decode                     # every sequence brings one row: two kernels do the whole of it
         prep = torch.empty((rows, self.C + self.H + self.H * self.GD), dtype=torch.float32, device=proj.device)
         if self.low1 is None:
             gate, gate_stride = proj[:, self.C:], proj.shape[1]
             ops.delta_prepare(proj, self.conv_w, state, self.H * self.D * self.V, batch.row_slot, batch.seq_start,
                               batch.seq_slot, batch.sequences, self.a_log, self.dt_bias, prep, self.H, self.KH, self.D,
-                              self.V, _UNIT_EPS, block_a_segment=few)
+                              self.V, _UNIT_EPS, block_a_segment=few, one_row_each=each)
         else:
             # the low-rank maps: [a1 h | g1 h] in the compute dtype, then both second halves in one block-diagonal product
             low = self.low2.forward(self.low1.forward(h), out_dtype=torch.float32)      # [rows, H GD | H V]
             gate, gate_stride = low[:, self.H * self.GD:], low.shape[1]
             ops.delta_prepare(proj, self.conv_w, state, self.H * self.D * self.V, batch.row_slot, batch.seq_start,
                               batch.seq_slot, batch.sequences, self.a_log, self.dt_bias, prep, self.H, self.KH, self.D,
-                              self.V, _UNIT_EPS, block_a_segment=few, beta_col=self.C,
+                              self.V, _UNIT_EPS, block_a_segment=few, one_row_each=each, beta_col=self.C,
                               decay_in=low[:, :self.H * self.GD], channel_decay=self.channel_decay)
+        y = torch.empty((rows, hv), dtype=self.dtype, device=proj.device)
+        mode = ops.DELTA_CHANNEL_DECAY if self.channel_decay else ops.DELTA_HEAD_DECAY
+        if each and self.V <= 128:
+            ops.delta_step(prep, state, batch.seq_start, batch.seq_slot, batch.sequences, self.H, self.KH, self.D, self.V, gate, gate_stride,
+                           self.norm_w, y, self.eps, gate_act=self.gate_act, mode=mode)
+            return self._finish(y, residual, overwrite)
         o = torch.empty((rows, hv), dtype=torch.float32, device=proj.device)
         # bfloat16 steps take a sequence's rows 32 or two at a time; the 32-bit path keeps one order of operations for every cut
         if self.dtype == torch.bfloat16 and not self.channel_decay and ops.delta_runs_in_chunks(batch, self.D, self.V, prep.shape[1]):
@@ -155,10 +162,11 @@ class GatedDeltaMixer:
                              self.V, o)
         else:
             ops.delta_rule(prep, state, batch.seq_start, batch.seq_slot, batch.sequences, self.H, self.KH, self.D, self.V, o,
-                           pairs=self.dtype == torch.bfloat16,
-                           mode=ops.DELTA_CHANNEL_DECAY if self.channel_decay else ops.DELTA_HEAD_DECAY)
-        y = torch.empty((rows, hv), dtype=self.dtype, device=proj.device)
+                           pairs=self.dtype == torch.bfloat16, mode=mode)
         ops.delta_output(o, gate, gate_stride, self.norm_w, y, self.H, self.V, self.eps, gate_act=self.gate_act)
+        return self._finish(y, residual, overwrite)
+
+    def _finish(self, y, residual, overwrite):
         if overwrite:
             self.o.forward(y, out=residual)
         else:

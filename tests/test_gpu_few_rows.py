@@ -36,3 +36,39 @@ def test_heads_product_of_few_rows(rows, H, K, N, tail, rot_dims, halves, gate, 
     tol = 2e-6 * K ** 0.5 if out == torch.float32 else 2 ** -8            # sums of K products in float32; one rounding
     assert float((got[rows][..., :N] - want).abs().max()) <= tol * scale
     assert float((got[rows] - got[many]).abs().max()) <= tol * scale and torch.equal(got[rows][..., N:], got[many][..., N:])
+
+
+@pytest.mark.parametrize("D, V, H, KH, mode", [(128, 128, 4, 2, 0), (40, 36, 6, 2, 0), (20, 8, 2, 1, 1), (128, 100, 3, 3, 1), (200, 64, 2, 2, 0)])
+@pytest.mark.parametrize("taps", [1, 2, 4])
+def test_delta_step_against_the_kernels_it_stands_for(D, V, H, KH, mode, taps):
+    """One token a sequence, several steps: the kept inputs, the state and the output of the two launches against those of the four."""
+    B, GD, C = 5, D if mode else 1, 2 * KH * D + H * V
+    g = torch.Generator().manual_seed(D * V + taps)
+    dev = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    taps_w, a_log, bias, weight = dev(C, taps), 0.3 * dev(H), dev(H * GD), dev(V)
+    i32 = lambda v: torch.as_tensor(v, dtype=torch.int32, device=DEV)
+    slots, starts = i32([6, 1, 0, 3, 5]), i32(list(range(B + 1)))
+    first = 0.5 * dev(8, H * D * V + (taps - 1) * C)
+    states = [first.clone(), first.clone()]
+    for step in range(3):
+        proj, decay = dev(B, C + H * V + 2 * H), dev(B, H * GD) if mode else None
+        gate = proj[:, C:]
+        outs = []
+        for kind, state in enumerate(states):
+            prep = torch.empty(B, C + H + H * GD, device=DEV)
+            ops.delta_prepare(proj, taps_w, state, H * D * V, slots, starts, slots, B, a_log, bias, prep, H, KH, D, V, 1e-6,
+                              block_a_segment=True, one_row_each=kind == 1, decay_in=decay, channel_decay=bool(mode))
+            y = torch.full((B, H * V), float("nan"), device=DEV)
+            if kind == 0:
+                o = torch.empty(B, H * V, device=DEV)
+                ops.delta_rule(prep, state, starts, slots, B, H, KH, D, V, o, mode=mode)
+                ops.delta_output(o, gate, proj.shape[1], weight, y, H, V, 1e-5)
+            else:
+                ops.delta_step(prep, state, starts, slots, B, H, KH, D, V, gate, proj.shape[1], weight, y, 1e-5, mode=mode)
+            outs.append((prep.cpu(), y.cpu(), state.cpu()))
+        assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][2][:, H * D * V:], outs[1][2][:, H * D * V:])
+        for a, b in zip(outs[0][1:], outs[1][1:]):         # the same sums in the same order, up to what the compiler fuses
+            assert float((a - b).abs().max()) <= 2e-6 * float(a.abs().max())
+    with pytest.raises(Exception, match="one each"):
+        ops.delta_prepare(proj, taps_w, states[0], H * D * V, slots, i32([0, 2, 2, 3, 4]), slots, B - 1, a_log, bias, prep, H, KH, D, V, 1e-6,
+                          block_a_segment=True, one_row_each=True, decay_in=decay, channel_decay=bool(mode))

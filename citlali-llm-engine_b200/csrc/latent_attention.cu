@@ -38,6 +38,8 @@ __device__ __forceinline__ float rotated_element(const TX* __restrict__ src, int
 }
 
 // proj [rows, proj_stride] float32: query latent (RQ) | c (R) | r (P) | ...   (has_kv = 0: no c and r in the row).
+// A block a row; what a few rows wait for is the chain read, sum, read again: the row is read once and summed once for both norms
+// (each in block_sum's order).
 template <typename TC, typename TQ>
 __global__ void __launch_bounds__(256)
 latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, int RQ, int R, int P, int has_kv,
@@ -50,21 +52,49 @@ latent_prepare_kernel(const float* __restrict__ proj, int proj_stride, int RQ, i
     wait_for_predecessor();
     const int row = blockIdx.x;
     const float* src = proj + (size_t)row * proj_stride;
-    float ss = 0.0f;
-    for (int i = threadIdx.x; i < RQ; i += blockDim.x) ss = fmaf(src[i], src[i], ss);
-    ss = block_sum(ss, scratch);
-    float inv = 1.0f / sqrtf(ss / (float)RQ + eps);
-    for (int i = threadIdx.x; i < RQ; i += blockDim.x) stf(cq, (size_t)row * RQ + i, src[i] * inv * q_weight[i]);
-    if (!has_kv) return;
     const float* c = src + RQ;
-    ss = 0.0f;
-    for (int i = threadIdx.x; i < R; i += blockDim.x) ss = fmaf(c[i], c[i], ss);
-    ss = block_sum(ss, scratch);
-    inv = 1.0f / sqrtf(ss / (float)R + eps);
-    const int pos = row_pos[row];
-    const int page = page_table[(size_t)row_slot[row] * table_stride + pos / page_size];
+    const int Rc = has_kv ? R : 0;
+    // one pass over the row: a thread's first four elements of either part stay in registers, and both sums are taken at once
+    float qv[4], cv[4], ss = 0.0f, sc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = threadIdx.x + j * 256;
+        qv[j] = i < RQ ? src[i] : 0.0f;
+        cv[j] = i < Rc ? c[i] : 0.0f;
+    }
+    const int pos = has_kv ? row_pos[row] : 0;
+    const int page = has_kv ? page_table[(size_t)row_slot[row] * table_stride + pos / page_size] : 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        ss = fmaf(qv[j], qv[j], ss);
+        sc = fmaf(cv[j], cv[j], sc);
+    }
+    for (int i = threadIdx.x + 1024; i < RQ; i += 256) ss = fmaf(src[i], src[i], ss);
+    for (int i = threadIdx.x + 1024; i < Rc; i += 256) sc = fmaf(c[i], c[i], sc);
+    {   // block_sum of both (eight warps)
+        ss = warp_sum(ss); sc = warp_sum(sc);
+        if ((threadIdx.x & 31) == 0) { scratch[threadIdx.x >> 5] = ss; scratch[16 + (threadIdx.x >> 5)] = sc; }
+        __syncthreads();
+        const int lane = threadIdx.x & 31;
+        ss = warp_sum(lane < 8 ? scratch[lane] : 0.0f);
+        sc = warp_sum(lane < 8 ? scratch[16 + lane] : 0.0f);
+    }
+    float inv = 1.0f / sqrtf(ss / (float)RQ + eps);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = threadIdx.x + j * 256;
+        if (i < RQ) stf(cq, (size_t)row * RQ + i, qv[j] * inv * q_weight[i]);
+    }
+    for (int i = threadIdx.x + 1024; i < RQ; i += 256) stf(cq, (size_t)row * RQ + i, src[i] * inv * q_weight[i]);
+    if (!has_kv) return;
+    inv = 1.0f / sqrtf(sc / (float)R + eps);
     TC* dst = pool + ((size_t)page * page_size + pos % page_size) * (R + P);
-    for (int i = threadIdx.x; i < R; i += blockDim.x) stf(dst, i, c[i] * inv * c_weight[i]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = threadIdx.x + j * 256;
+        if (i < R) stf(dst, i, cv[j] * inv * c_weight[i]);
+    }
+    for (int i = threadIdx.x + 1024; i < R; i += 256) stf(dst, i, c[i] * inv * c_weight[i]);
     const float* r = c + R;
     if (rot_halves) {
         for (int i = threadIdx.x; i < P; i += blockDim.x) stf(dst, R + i, rotated_element(r, i, rot_dims, 1, pos, inv_freq));

@@ -8,7 +8,10 @@
 // warp w accumulates the output columns R/4 w .. R/4 (w + 1).  Softmax is float32 (online, base 2); the sink joins
 // the denominator at the end.  In steps of few rows (decoding) a unit's tiles are dealt to several blocks in runs, whose
 // unnormalised sums, maxima and denominators a second kernel merges in run order; the number of runs follows the
-// number of rows in the step alone, so what else is in the step changes a row by rounding at most.  Needs E a multiple of 16 and R a multiple of 64.
+// number of rows in the step alone, so what else is in the step changes a row by rounding at most.  A run's time is the latency of its
+// first reads (the first tile is on its way while the queries are read, six reads a thread at once) and 2 us a tile: with the merge 12.3 us
+// for runs of one tile (queries read one 16-byte piece after another, and before the tile: 16.7 us).
+// Needs E a multiple of 16 and R a multiple of 64.
 #include "api.h"
 #include "common.cuh"
 #include "mma_common.cuh"
@@ -40,17 +43,6 @@ latent_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __
     const int pos = row_pos[row];
     const int32_t* table = page_table + (size_t)row_slot[row] * table_stride;
     const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
-    {   // the queries of the sixteen heads, rounded to bfloat16: 16-byte loads, four elements a thread and turn
-        const int quads = E / 4;
-        for (int hh = 0; hh < 16; ++hh) {
-            const bool real = h0 + hh < H;
-            const float4* src = reinterpret_cast<const float4*>(q + ((size_t)row * H + h0 + hh) * E);
-            for (int i = tid; i < quads; i += 128) {
-                const float4 v = real ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<uint2*>(Qs + hh * ES + i * 4) = make_uint2(fa::pack_bf16(v.x, v.y), fa::pack_bf16(v.z, v.w));
-            }
-        }
-    }
     const float sl2 = scale * 1.4426950408889634f;          // scores in units of log 2
     const int NT = R / 32;                                   // tiles of 8 output columns a warp owns
     const int col0 = warp * (R / 4);
@@ -65,8 +57,8 @@ latent_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __
     const int tiles = (pos - lo) / kTileKeys + 1, per = (tiles + splits - 1) / splits;
     const int first = lo + split * per * kTileKeys;
     const int last = min(pos, first + per * kTileKeys - 1);
-    for (int t0 = first; t0 <= last; t0 += kTileKeys) {
-        __syncthreads();                                     // the tile before is no longer read; Q is in place
+    if (splits > 1 && first > last) return;                 // a run without tiles; the merge counts the runs that have some
+    auto fetch = [&](int t0) {
         for (int kr = tid >> 3; kr < kTileKeys; kr += 16) {      // eight threads a cached vector, sixteen vectors a pass
             const int key = t0 + kr;
             __nv_bfloat16* dst = Ks + kr * ES;
@@ -78,6 +70,33 @@ latent_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __
             }
         }
         fa::cp_async_commit();
+    };
+    // the first tile is on its way while the queries are read and rounded
+    fetch(first);
+    {   // the queries of the sixteen heads, rounded to bfloat16: 16-byte loads, six on their way at once
+        const int quads = E / 4;
+        const float4* src = reinterpret_cast<const float4*>(q + ((size_t)row * H + h0) * E);      // the heads' rows follow one another
+        const int total = 16 * quads, real = min(16, H - h0) * quads;
+        for (int i0 = tid; i0 < total; i0 += 6 * 128) {
+            float4 v[6];
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                const int i = i0 + u * 128;
+                v[u] = i < real ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                const int i = i0 + u * 128;
+                if (i < total)
+                    *reinterpret_cast<uint2*>(Qs + (i / quads) * ES + (i % quads) * 4) = make_uint2(fa::pack_bf16(v[u].x, v[u].y), fa::pack_bf16(v[u].z, v[u].w));
+            }
+        }
+    }
+    for (int t0 = first; t0 <= last; t0 += kTileKeys) {
+        if (t0 != first) {
+            __syncthreads();                                 // the tile before is no longer read
+            fetch(t0);
+        }
         fa::cp_async_wait<0>();
         __syncthreads();
         // scores of this warp's 16 keys
@@ -187,28 +206,40 @@ latent_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __
     }
 }
 
-// The runs of a unit put together in run order: one block a (row, head), a thread a column at a time.
+// The runs of a unit put together in run order: one block a (row, head).  Every warp works the runs' weights out for itself (a lane a
+// run), then a thread takes two neighbouring columns over all runs, several runs' reads at once.  Bound by those reads: 8 rows of 16
+// heads over 17 runs, 10 us with caches cold; over 32 runs, empty ones among them, it was 15 us.
 __global__ void __launch_bounds__(128)
 latent_attention_merge_kernel(const float* __restrict__ partial, const float* __restrict__ sink, float* __restrict__ out,
-                              int H, int R, int splits) {
+                              const int32_t* __restrict__ row_pos, int H, int R, int window, int splits) {
     __shared__ float weight[64];
     dependents_may_launch();
     wait_for_predecessor();
-    const int groups = (H + 15) / 16, row = blockIdx.x / H, h = blockIdx.x % H;
+    const int groups = (H + 15) / 16, row = blockIdx.x / H, h = blockIdx.x % H, lane = threadIdx.x & 31;
     const int unit = row * groups + h / 16, hh = h % 16;
     const float* src = partial + (size_t)unit * splits * 16 * (R + 2) + (size_t)hh * (R + 2);
     const size_t run = (size_t)16 * (R + 2);
-    float top = sink ? sink[h] * 1.4426950408889634f : -INFINITY;
-    const float sk = top;
-    for (int s = 0; s < splits; ++s) top = fmaxf(top, src[s * run + R]);
-    float denom = sink ? fa::fast_exp2(sk - top) : 0.0f;
-    for (int s = 0; s < splits; ++s) denom += src[s * run + R + 1] * fa::fast_exp2(src[s * run + R] - top);   // an empty run: maximum -inf, counts nothing
-    if (threadIdx.x < splits) weight[threadIdx.x] = fa::fast_exp2(src[threadIdx.x * run + R] - top) / denom;
+    // the runs that have tiles (as the walk deals them)
+    const int pos = row_pos[row], lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+    const int tiles = (pos - lo) / kTileKeys + 1, per = (tiles + splits - 1) / splits, runs = (tiles + per - 1) / per;
+    const float sk = sink ? sink[h] * 1.4426950408889634f : -INFINITY;
+    float2 mine[2];                                          // maximum and denominator of runs lane, lane + 32
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        mine[k] = lane + 32 * k < runs ? *reinterpret_cast<const float2*>(src + (lane + 32 * k) * run + R) : make_float2(-INFINITY, 0.0f);
+    const float top = fmaxf(warp_max(fmaxf(mine[0].x, mine[1].x)), sk);
+    const float f0 = fa::fast_exp2(mine[0].x - top), f1 = fa::fast_exp2(mine[1].x - top);
+    const float denom = warp_sum(mine[0].y * f0 + mine[1].y * f1) + (sink ? fa::fast_exp2(sk - top) : 0.0f);
+    if (threadIdx.x < 32) { weight[lane] = f0 / denom; weight[lane + 32] = f1 / denom; }
     __syncthreads();
-    for (int i = threadIdx.x; i < R; i += blockDim.x) {
-        float acc = 0.0f;
-        for (int s = 0; s < splits; ++s) acc = fmaf(src[s * run + i], weight[s], acc);
-        out[((size_t)row * H + h) * R + i] = acc;
+    for (int i = threadIdx.x * 2; i < R; i += blockDim.x * 2) {              // R is a multiple of 64
+        float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll 8
+        for (int s = 0; s < runs; ++s) {
+            const float2 v = *reinterpret_cast<const float2*>(src + s * run + i);
+            acc.x = fmaf(v.x, weight[s], acc.x); acc.y = fmaf(v.y, weight[s], acc.y);
+        }
+        *reinterpret_cast<float2*>(out + ((size_t)row * H + h) * R + i) = acc;
     }
 }
 
@@ -257,6 +288,6 @@ extern "C" int citlali_latent_attention_mma(const float* q, const void* pool, co
 #undef CITLALI_LATENT_MMA
     int code = CITLALI_LAUNCH_CHECK();
     if (code != 0 || splits == 1) return code;
-    launch_kernel(latent_attention_merge_kernel, rows * H, 128, 0, stream, (const float*)partial, sink, out, H, R, splits);
+    launch_kernel(latent_attention_merge_kernel, rows * H, 128, 0, stream, (const float*)partial, sink, out, row_pos, H, R, window, splits);
     return CITLALI_LAUNCH_CHECK();
 }

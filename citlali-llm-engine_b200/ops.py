@@ -1292,7 +1292,12 @@ def latent_attention(q, pool, page_table, row_slot, row_pos, sink, out, H, R, E,
         # follows the number of rows alone and never exceeds the tiles a window (or the longest sequence) has
         units = rows * ((H + 15) // 16)
         longest = int(window) if window else page_table.shape[1] * page_size
-        splits = max(1, min(sm_count(q.device) * 2 // units, (longest + 63) // 64, 32)) if splits is None else int(splits)
+        if splits is None:
+            tiles, sms = (longest + 63) // 64, sm_count(q.device)
+            # two blocks an SM, but a second one only for runs of two tiles and more: a run costs the merge what it saves the walk
+            # (8 units of 32 tiles: 32 runs 18.8 us, 16 runs 16.6; 16 units of 63 tiles: 18 runs 29.3 us, 9 runs 33.9)
+            splits = max(1, min(sms * 2 // units, max(sms // units, (tiles + 1) // 2), tiles, 32))
+        splits = int(splits)
         partial = None
         if splits > 1:
             partial = _scratch(q.device, "latent_attention runs", units * splits * 16 * (R + 2) * 4)

@@ -164,16 +164,18 @@ class SequenceCache:
         self.lengths[slot] = 0
 
     def length(self, slot: int) -> int:
-        require(self.slots.is_held(slot), f"slot {slot} is not held")
+        if not self.slots.is_held(slot):
+            require(False, f"slot {slot} is not held")
         return self.lengths[slot]
 
     # ---- growing a sequence -----------------------------------------------------------
     def reserve(self, slot: int, new_length: int) -> None:
         """Make room for positions below ``new_length`` in every group.  Either all groups get
         their pages or none does."""
-        require(self.slots.is_held(slot), f"slot {slot} is not held")
-        require(new_length <= self.max_sequence_tokens,
-                f"a sequence of {new_length} tokens exceeds the cache's limit of {self.max_sequence_tokens} per sequence")
+        if not self.slots.is_held(slot):
+            require(False, f"slot {slot} is not held")
+        if not (new_length <= self.max_sequence_tokens):
+            require(False, f"a sequence of {new_length} tokens exceeds the cache's limit of {self.max_sequence_tokens} per sequence")
         have = self.lengths[slot]
         if have > 0 and (new_length - 1) // self.page_size == (have - 1) // self.page_size:
             return          # the page that holds the last token also holds the new ones
@@ -209,7 +211,8 @@ class SequenceCache:
 
     def commit(self, slot: int, new_length: int) -> None:
         """The step that wrote positions below ``new_length`` has been issued."""
-        require(self.slots.is_held(slot), f"slot {slot} is not held")
+        if not self.slots.is_held(slot):
+            require(False, f"slot {slot} is not held")
         self.lengths[slot] = new_length
         if not self._has_window:
             return
@@ -226,9 +229,10 @@ class SequenceCache:
     def rewind(self, slot: int, new_length: int) -> None:
         """Forget a sequence's tokens from ``new_length`` on (they will be computed again or replaced).
         Pages stay with the slot.  Not for caches with a window group, whose early pages are already gone."""
-        require(self.slots.is_held(slot), f"slot {slot} is not held")
-        require(0 <= new_length <= self.lengths[slot],
-                f"slot {slot} holds {self.lengths[slot]} tokens and cannot be rewound to {new_length}")
+        if not self.slots.is_held(slot):
+            require(False, f"slot {slot} is not held")
+        if not (0 <= new_length <= self.lengths[slot]):
+            require(False, f"slot {slot} holds {self.lengths[slot]} tokens and cannot be rewound to {new_length}")
         require(not self._has_window, "a cache with a windowed group cannot be rewound")
         self.lengths[slot] = new_length
 
@@ -247,7 +251,8 @@ class SequenceCache:
         return self._view_of(keys)
 
     def _view_of(self, key):
-        require(key in self._where, f"schedule step {key} keeps no cache")
+        if key not in self._where:
+            require(False, f"schedule step {key} keeps no cache")
         kind, gi, j = self._where[key]
         if kind == "kv":
             g = self.kv_groups[gi]

@@ -170,6 +170,25 @@ def build(force: bool = False, verbose: bool = True) -> str:
 
 _BASE = "elementwise"                       # holds what every other source calls (error text, launch mode)
 _ALSO = {"gemm_tcgen05": ("gemm_tcgen05_pair",), "attention_decode_no_alloc": ("attention_decode",)}    # who calls whom besides
+_TYPES = {"int": ctypes.c_int, "float": ctypes.c_float, "size_t": ctypes.c_size_t, "long": ctypes.c_long, "long long": ctypes.c_longlong,
+          "cudaStream_t": ctypes.c_void_p, "void": None, "const char*": ctypes.c_char_p}
+_DECLARED = re.compile(r"([\w ]+[\s*]+)(citlali_\w+)\s*\(([^)]*)\)\s*;")
+
+
+def signatures():
+    """{entry point: (result type, argument types)} as the C headers declare them; any pointer is a ``c_void_p``.  With the types known,
+    a call takes plain Python numbers and addresses: making a ctypes object of every argument took a launch several microseconds."""
+    out = {}
+    for header in ("api.h", "no_alloc.h"):
+        with open(os.path.join(_HERE, header), encoding="utf-8") as fh:
+            code = re.sub(r"//[^\n]*", "", fh.read())
+        for result, name, args in _DECLARED.findall(code):
+            kinds = [ctypes.c_void_p if "*" in a else _TYPES[re.sub(r"\w+$", "", a).strip()] for a in
+                     (a.strip() for a in args.split(",")) if a not in ("", "void")]
+            out[name] = (_TYPES[result.strip()], kinds)
+    return out
+
+
 _ENTRY = re.compile(r'extern "C"[^;{]*?\b(citlali_\w+)\s*\(')
 
 
@@ -183,6 +202,7 @@ class Kernels:
         self._loaded = {}
         self._source_of = {}
         self._lock = threading.RLock()
+        self._signatures = signatures()
         if _stamped(library_path(), _digest()):
             self._whole = self._open(library_path())
             return
@@ -235,6 +255,9 @@ class Kernels:
                 raise AttributeError(f"no kernel source defines {name}")
             self.prepare([stem])
             fn = getattr(self._loaded[stem], name)
+        if name not in self._signatures:
+            raise CitlaliError(f"{name} is defined but no header declares it: its arguments' types are not known")
+        fn.restype, fn.argtypes = self._signatures[name]
         self.__dict__[name] = fn
         return fn
 

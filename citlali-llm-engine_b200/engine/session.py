@@ -142,10 +142,11 @@ class InferenceSession:
         require(len(entries) > 0, "a step needs at least one entry")
         past = []
         for e in entries:
-            require(self.cache.slots.is_held(e.slot), f"slot {e.slot} was not acquired")
+            if not self.cache.slots.is_held(e.slot):
+                require(False, f"slot {e.slot} was not acquired")
             p = self.cache.length(e.slot)
-            require(p + len(e.tokens) <= self.max_context,
-                    f"slot {e.slot}: {p} cached + {len(e.tokens)} new tokens exceed max_context {self.max_context}")
+            if not (p + len(e.tokens) <= self.max_context):
+                require(False, f"slot {e.slot}: {p} cached + {len(e.tokens)} new tokens exceed max_context {self.max_context}")
             past.append(p)
         batch = pack_step(entries, past, self.model.spec.vocab_size, self.model.ctx.device)
         for e, p in zip(entries, past):

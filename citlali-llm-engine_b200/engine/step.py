@@ -10,6 +10,7 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import List, Sequence
 
+import numpy as np
 import torch
 
 from ..errors import require
@@ -23,18 +24,27 @@ class StepEntry:
     want: Sequence[int] = field(default_factory=list)   # places among `tokens` whose logits are asked for
 
 
+def _as_ids(tokens: list) -> np.ndarray:
+    try:
+        return np.array(tokens, dtype=np.int64)
+    except (TypeError, ValueError):                   # numbers that numpy does not read (elements of a tensor on the device)
+        return torch.as_tensor(tokens, dtype=torch.int64).numpy()
+
+
 def pack_step(entries: List[StepEntry], past: List[int], vocab_size: int, device) -> StepBatch:
     """``past[i]`` is the number of tokens entry i's slot already holds."""
     require(len(entries) > 0, "a step needs at least one entry")
     seen = set()
     rows = 0
     for e in entries:
-        require(e.slot not in seen, f"slot {e.slot} appears twice in one step")
+        if e.slot in seen:
+            require(False, f"slot {e.slot} appears twice in one step")
         seen.add(e.slot)
-        require(len(e.tokens) > 0, f"the entry of slot {e.slot} brings no tokens")
+        if len(e.tokens) == 0:
+            require(False, f"the entry of slot {e.slot} brings no tokens")
         for w in e.want:
-            require(0 <= w < len(e.tokens),
-                    f"slot {e.slot}: logits asked at place {w} of {len(e.tokens)} tokens")
+            if not (0 <= w < len(e.tokens)):
+                require(False, f"slot {e.slot}: logits asked at place {w} of {len(e.tokens)} tokens")
         rows += len(e.tokens)
     B = len(entries)
     wanted = sum(len(e.want) for e in entries)
@@ -45,24 +55,26 @@ def pack_step(entries: List[StepEntry], past: List[int], vocab_size: int, device
         offsets.append(offsets[-1] + ((s + 3) // 4) * 4)      # 16-byte aligned pieces
     pin = torch.device(device).type == "cuda"
     host = torch.zeros(max(offsets[-1], 4), dtype=torch.int32, pin_memory=pin)
+    # the same memory written without tensor operations: a few microseconds each, and a step of short prompts waits for the host
+    array = host.numpy()
     tokens, row_slot, row_pos, seq_start, seq_slot, seq_past, want_rows = (
-        host[offsets[i]:offsets[i] + sizes[i]] for i in range(7))
+        array[offsets[i]:offsets[i] + sizes[i]] for i in range(7))
     r = 0
     w = 0
     for b, e in enumerate(entries):
         n = len(e.tokens)
-        ids = torch.as_tensor(list(e.tokens), dtype=torch.int64)
+        ids = _as_ids(list(e.tokens))
         if int(ids.min()) < 0 or int(ids.max()) >= vocab_size:        # as the reference checks (qwen_model.cpp:240-241)
             bad = int(ids[(ids < 0) | (ids >= vocab_size)][0])
             require(False, f"token id {bad} out of vocab range [0, {vocab_size})")
-        tokens[r:r + n] = ids.to(torch.int32)
-        row_slot[r:r + n] = e.slot
-        row_pos[r:r + n] = torch.arange(past[b], past[b] + n, dtype=torch.int32)
+        tokens[r:r + n] = ids
+        row_slot[r:r + n] = int(e.slot)
+        row_pos[r:r + n] = np.arange(past[b], past[b] + n)
         seq_start[b] = r
-        seq_slot[b] = e.slot
+        seq_slot[b] = int(e.slot)
         seq_past[b] = past[b]
         for place in e.want:
-            want_rows[w] = r + place
+            want_rows[w] = r + int(place)
             w += 1
         r += n
     seq_start[B] = r

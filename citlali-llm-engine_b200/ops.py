@@ -8,6 +8,7 @@ CUDA device, they raise.
 from __future__ import annotations
 
 import ctypes
+import operator
 from typing import Optional
 
 import torch
@@ -30,9 +31,7 @@ def lib():
     global _lib
     if _lib is None:
         from .csrc.build import load
-        l = load()
-        l.citlali_last_error.restype = ctypes.c_char_p
-        _lib = l
+        _lib = load()
     return _lib
 
 
@@ -43,20 +42,20 @@ def prepare_kernels(sources) -> None:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    if t is None:
-        return ctypes.c_void_p(0)
-    return ctypes.c_void_p(t.data_ptr())
+    """A tensor's address, for an argument declared as a pointer (csrc/build.py gives every entry point its argument types)."""
+    return None if t is None else t.data_ptr()
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device      # a tensor is on the device: CUDA is up
 
 
 def _stream():
     """The current CUDA stream's handle.  Asked for at every launch, so by the quick route where torch has one
     (a step launches a few hundred kernels and the host must not be what a short prompt waits for)."""
     if _raw_stream is not None:
-        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_current_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 _launches = 0
@@ -86,8 +85,9 @@ def _need_cuda(*tensors):
             require(False, "kernels take contiguous tensors")
 
 
-_i = ctypes.c_int
-_f = ctypes.c_float
+# plain numbers of the kind the C argument wants (an integer argument takes no float)
+_i = _sz = operator.index
+_f = float
 
 
 def embed_rows(table: torch.Tensor, tokens: torch.Tensor, out: torch.Tensor, error_flag: torch.Tensor,
@@ -381,7 +381,6 @@ def attention_decode(q, q_stride, k_pool, v_pool, page_table, row_slot, row_pos,
             "attention_decode: bfloat16 only")
     rows = out.shape[0]
     l = lib()
-    l.citlali_attention_decode_scratch_floats.restype = ctypes.c_size_t
     need = l.citlali_attention_decode_scratch_floats(_i(rows), _i(nq), _i(head_dim), _i(page_size), _i(max_positions))
     ws = _scratch(q.device, "attention_decode", need * 4)
     counters = _scratch(q.device, "attention_decode counters", rows * nq * 4, zeroed=True)
@@ -406,7 +405,6 @@ def attention_decode_with(q, kv, batch, out, nq, nkv, d, vd, window, scale, soft
             and q.shape == (rows, nq * d) and out.shape == (rows, nq * vd), "attention_decode_with: shapes or dtypes do not fit")
     _check_sink_and_turns(sink, turns, nq, rows, vd)
     l = lib()
-    l.citlali_attention_decode_scratch_floats.restype = ctypes.c_size_t
     positions = kv.page_table.shape[1] * kv.page_size
     need = l.citlali_attention_decode_scratch_floats(_i(rows), _i(nq), _i(max(d, vd)), _i(kv.page_size), _i(positions))
     ws = _scratch(q.device, "attention_decode", need * 4)
@@ -596,8 +594,6 @@ def gemm_tc_act(x, w, y, accumulate=False, bias=None, act=None, error_flag=None)
 
 # ---- residual streams --------------------------------------------------------------------------
 
-_sz = ctypes.c_size_t
-
 
 def hyper_read_norm(X: torch.Tensor, w_in: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.Tensor):
     """``out = rms_norm(sum_s w_in[s] X[s]) * gain``; X float32 [streams, rows, width], gain float32."""
@@ -722,7 +718,6 @@ def delta_chunks(prep, state, seq_start, seq_slot, sequences, max_new, H, KH, D,
     require(prep.dtype == torch.float32 and state.dtype == torch.float32 and out.dtype == torch.float32 and out.shape == (rows, H * V)
             and state.shape[1] >= H * D * V and prep.shape[1] == 2 * KH * D + H * V + 2 * H, "delta_chunks: shapes or dtypes do not fit")
     l = lib()
-    l.citlali_delta_chunks_scratch_floats.restype = ctypes.c_size_t
     scratch = torch.empty(l.citlali_delta_chunks_scratch_floats(_i(rows), _i(sequences), _i(H)), dtype=torch.float32, device=prep.device)
     _check(l.citlali_delta_chunks(_ptr(prep), _i(prep.shape[1]), _ptr(state), _sz(state.shape[1]), _ptr(seq_start), _ptr(seq_slot),
                                   _i(sequences), _i(max_new), _i(H), _i(KH), _i(D), _i(V), _ptr(out), _ptr(scratch),

@@ -111,12 +111,13 @@ class GQAttention:
     def forward(self, h, batch, cache_view, residual, write_cache=True, emit=None):
         """``h``: the normed rows, or :class:`~.base.NormedRows` (few rows; after :meth:`fold_norm_gain`).  ``emit``: a pair
         of buffers that the output projection fills with what the next norm needs of the updated residual rows."""
-        require(cache_view is not None, f"{self.prefix}: attention needs a key/value cache")
+        if cache_view is None:
+            require(False, f"{self.prefix}: attention needs a key/value cache")
         req = cache_view.requirement
         nkv_here = self.nkv if self.kv_projection else 0
-        require(req.head_dim == self.d and req.num_kv_heads == self.nkv,
-                f"{self.prefix}: the cache holds {req.num_kv_heads} heads of {req.head_dim}, "
-                f"the layer has {self.nkv} of {self.d}")
+        if not (req.head_dim == self.d and req.num_kv_heads == self.nkv):
+            require(False, f"{self.prefix}: the cache holds {req.num_kv_heads} heads of {req.head_dim}, "
+                           f"the layer has {self.nkv} of {self.d}")
         if isinstance(h, NormedRows):
             qkv = self.qkv.forward(h.rows, row_scale=h.scale)
         else:

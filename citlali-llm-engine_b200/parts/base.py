@@ -126,6 +126,8 @@ class StepBatch:
     # not know of it breaks the chain instead of passing on something stale.
     norm_carry: Optional["NormedRows"] = None
     norm_carry_in: Optional["NormedRows"] = None
+    # the two pairs of buffers such rows take turns in, for the whole step (parts/block.py)
+    norm_buffers: Optional[list] = None
     # A block on several residual streams may leave its last write-back undone, as (y, mix, out), for the next such
     # block to do together with its first read (one pass over the streams instead of two); the model does what is left
     # after the last layer.

@@ -76,17 +76,20 @@ class PreNormResidualBlock:
 
     def _forward_norms_in_products(self, x, batch, cache_view, write_cache):
         rows, hidden = x.shape
-        def buffers():
-            return (torch.empty((rows, hidden), dtype=torch.bfloat16, device=x.device),
-                    torch.empty((rows, hidden // 32), dtype=torch.float32, device=x.device))
+        # Two pairs of buffers serve the whole step: a product reads one pair while a later one fills the other, in stream order
+        # (four tensors a layer took the host an eighth of a short step).
+        pairs = batch.norm_buffers
+        if pairs is None or pairs[0][0].shape != x.shape:
+            pairs = batch.norm_buffers = [(torch.empty((rows, hidden), dtype=torch.bfloat16, device=x.device),
+                                           torch.empty((rows, hidden // 32), dtype=torch.float32, device=x.device)) for _ in range(2)]
+        after_mixer, after_ff = pairs
         carried = batch.norm_carry_in
         if carried is None or carried.rows.shape != (rows, hidden):
-            rows_bf16, sumsq = buffers()                   # the rows came from somewhere that emitted nothing
-            ops.norm_inputs(x, rows_bf16, sumsq)
-            carried = NormedRows(rows_bf16, sumsq, hidden)
-        after_mixer = buffers()
+            ops.norm_inputs(x, *after_ff)                  # the rows came from somewhere that emitted nothing
+            carried = NormedRows(*after_ff, hidden)
+        elif carried.rows is after_mixer[0]:
+            after_mixer, after_ff = after_ff, after_mixer
         self.mixer.forward(carried.with_eps(self.mixer_norm.eps), batch, cache_view, x, write_cache, emit=after_mixer)
-        after_ff = buffers()
         self.feed_forward.forward(NormedRows(after_mixer[0], after_mixer[1], hidden, self.feed_forward_norm.eps), batch, x,
                                   emit=after_ff)
         batch.norm_carry = NormedRows(after_ff[0], after_ff[1], hidden)

@@ -96,3 +96,20 @@ def test_stream_writes_against_float64(S, rows, W):
     u = torch.einsum("s,srw->rw", w_in.double(), want)
     ref = u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-5) * gain.double()
     assert float((h.cpu().double() - ref).abs().max()) <= 2e-5 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("V, H, extra", [(128, 5, 0), (36, 9, 4), (512, 2, 8), (300, 3, 0), (7, 4, 1), (516, 2, 0), (128, 3, 2)])
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_delta_output_against_float64(V, H, extra, act, dtype):
+    """Values in fours and others, gates on 16-byte boundaries and off them (rows a little wider than the gates)."""
+    rows = 11
+    g = torch.Generator().manual_seed(V * H)
+    o, wide, w = torch.randn(rows, H * V, generator=g), torch.randn(rows, extra + H * V, generator=g), torch.randn(V, generator=g)
+    z = wide.to(DEV)
+    y = torch.full((rows, H * V), float("nan"), dtype=dtype, device=DEV)
+    ops.delta_output(o.to(DEV), z[:, extra:], z.shape[1], w.to(DEV), y, H, V, 1e-5, gate_act=act)
+    v, t = o.double().view(rows, H, V), wide[:, extra:].double().view(rows, H, V)
+    s = torch.sigmoid(t)
+    want = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double() * (s if act == "sigmoid" else t * s)
+    assert float((y.double().cpu().view(rows, H, V) - want).abs().max()) <= (3e-6 if dtype == torch.float32 else 2 ** -8) * float(want.abs().max())

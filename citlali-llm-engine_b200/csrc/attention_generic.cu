@@ -357,11 +357,11 @@ attention_rows_grouped_kernel(const T* __restrict__ q, int q_stride, const T* __
     const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
     const int n = pos - lo + 1;
     float* sc = smem;                                         // [n][HB]
-    int* at = reinterpret_cast<int*>(smem + (size_t)n * HB);  // [n]: the key's row in the pools
+    uint32_t* at = reinterpret_cast<uint32_t*>(smem + (size_t)n * HB);      // [n]: the key's row in the pools
     const int32_t* pages = page_table + (size_t)row_slot[row] * page_table_stride;
     for (int t = tid; t < n; t += 128) {
         const int key = lo + t;
-        at[t] = (pages[key / page_size] * nkv + g) * page_size + key % page_size;
+        at[t] = ((uint32_t)pages[key / page_size] * nkv + g) * page_size + key % page_size;
     }
     float qv[HB][EPL];
 #pragma unroll

@@ -73,7 +73,7 @@ gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __restr
 // [k][row] in shared memory, put there element by element by asynchronous copies (any alignment, any K) three tiles deep.
 // TN = 128 for matrices with tiles enough for every SM, TN = 64 below that (see launch_wide).
 // A four-layer model of width 1,024 over 682 rows with logits of each (17 products, 54 G multiply-adds): 6.9 ms in the kernel
-// above, 2.5 ms here.
+// above, 3.2 ms here (of 1.5 that the FMA units need).
 __device__ __forceinline__ void cp_async4_or_zero(uint32_t dst, const float* src, bool there) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(there ? 4 : 0) : "memory");
 }

@@ -707,7 +707,7 @@ def delta_runs_in_chunks(batch, D, V, width) -> bool:
     sequence on, for sizes the chunks' 16-byte pieces take.  32 heads of 128 x 128, walk against chunks in us: one sequence of 24 / 48 /
     256 / 2,048 rows 20 / 39 / 184 / 1,420 against 19 / 23 / 52 / 318; sixteen of 32 / 33 / 48 / 256 rows 136 / 140 / 196 / 967 against
     108 / 172 / 172 / 588 (a chunk that begins is paid for whole)."""
-    return (batch.rows >= 48 * batch.sequences and D <= 128 and D % 4 == 0 and V % 4 == 0 and width % 4 == 0
+    return (batch.rows >= 48 * batch.sequences and batch.sequences <= 65535 and D <= 128 and D % 4 == 0 and V % 4 == 0 and width % 4 == 0
             and not torch.cuda.is_current_stream_capturing())
 
 
@@ -1328,7 +1328,7 @@ def latent_runs_as_attention(batch, dtype, H, R, P, D, V, window, gate, gate_per
     tokens in all, keep the walk: the rounding of the values averages out over the keys a row sees, and over a single key the walk has
     none (a lone row: 0.0031 against 0.0023 off float64)."""
     if (dtype != torch.bfloat16 or (window is not None and 0 < int(window) < 64) or D != 128 or V != 128 or R % 8 != 0 or P % 8 != 0 or P > 64
-            or batch.rows < 64 * batch.sequences or torch.cuda.is_current_stream_capturing()):
+            or batch.rows < 64 * batch.sequences or batch.sequences > 65535 or torch.cuda.is_current_stream_capturing()):
         return False
     if not gate_per_head and (gate.data_ptr() % 16 != 0 or gate.stride(0) % 4 != 0):
         return False

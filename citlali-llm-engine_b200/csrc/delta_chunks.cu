@@ -146,7 +146,25 @@ delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const f
     ScanShared<VS>& sm = *reinterpret_cast<ScanShared<VS>*>(smem_raw);
     dependents_may_launch();
     wait_for_predecessor();
-    const int tid = threadIdx.x, seq = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * VS;
+    const int tid = threadIdx.x, h = blockIdx.y, v0 = blockIdx.x * VS;
+    // the longest sequences' blocks first: where there are more blocks than SMs, the last ones to begin are then the shortest (five
+    // sequences of 155 to 540 tokens, 16 heads: a step of three such layers 1.70 -> 1.63 ms)
+    int seq = blockIdx.z;
+    const int sequences = gridDim.z;
+    if (sequences > 1 && sequences <= 256) {
+        __shared__ int chosen;
+        if (tid < sequences) {
+            const int n = seq_start[tid + 1] - seq_start[tid];
+            int rank = 0;
+            for (int s = 0; s < sequences; ++s) {
+                const int m = seq_start[s + 1] - seq_start[s];
+                rank += m > n || (m == n && s < tid);
+            }
+            if (rank == (int)blockIdx.z) chosen = tid;
+        }
+        __syncthreads();
+        seq = chosen;
+    }
     const int row0 = seq_start[seq], tokens = seq_start[seq + 1] - row0;
     if (tokens <= 0) return;
     const int kh = h / (H / KH);

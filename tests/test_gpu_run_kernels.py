@@ -113,3 +113,23 @@ def test_delta_output_against_float64(V, H, extra, act, dtype):
     s = torch.sigmoid(t)
     want = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double() * (s if act == "sigmoid" else t * s)
     assert float((y.double().cpu().view(rows, H, V) - want).abs().max()) <= (3e-6 if dtype == torch.float32 else 2 ** -8) * float(want.abs().max())
+
+
+@pytest.mark.parametrize("N, K, odd", [(48, 64, False), (130, 1000, False), (17, 333, False), (1024, 1024, False), (70, 128, True), (1, 1, False)])
+def test_32_bit_products_give_a_row_the_same_bits_in_steps_of_any_size(N, K, odd):
+    """Few rows, many rows and operands off 16-byte boundaries run different kernels with one chain an element."""
+    g = torch.Generator().manual_seed(N + K)
+    x, base = torch.randn(97, K, generator=g), torch.randn(97, N, generator=g).to(DEV)
+    store = torch.zeros(N * K + 1, device=DEV)
+    w = store[1:].view(N, K) if odd else store[:-1].view(N, K)
+    w.copy_(torch.randn(N, K, generator=g))
+    x, want = x.to(DEV), None
+    for rows in (97, 1, 7, 8, 9, 31, 32, 65):
+        y = torch.full((rows, N), float("nan"), device=DEV)
+        ops.gemm_simt(x[:rows].contiguous(), w, y)
+        added = base[:rows].clone()
+        ops.gemm_simt(x[:rows].contiguous(), w, added, accumulate=True)
+        if want is None:
+            want, exact = y, x.double() @ w.double().T
+            assert float((y.double() - exact).abs().max()) <= 2e-6 * K ** 0.5 * max(1.0, float(exact.abs().max()))
+        assert torch.equal(y, want[:rows]) and torch.equal(added, base[:rows] + y)

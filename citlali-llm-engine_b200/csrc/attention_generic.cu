@@ -457,15 +457,14 @@ attention_rows_grouped_kernel(const T* __restrict__ q, int q_stride, const T* __
     }
 }
 
+constexpr size_t kGroupedShared = 56 * 1024;                 // the most this form asks for: a quarter of an SM's
+
 template <typename T, int HB>
 static int launch_grouped(const void* q, int q_stride, const void* k_pool, const void* v_pool, const int32_t* page_table,
                           int page_table_stride, const int32_t* row_slot, const int32_t* row_pos, void* out, int out_stride, int rows,
                           int nq, int nkv, int d, int page_size, int window, size_t smem, float scale, cudaStream_t stream) {
     auto kernel = d <= 128 ? attention_rows_grouped_kernel<T, HB, 4> : attention_rows_grouped_kernel<T, HB, 8>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
+    if (int e = raise_shared_limit(kernel, smem, kGroupedShared)) return e;
     launch_kernel(kernel, dim3(rows, nq / HB), 128, smem, stream, (const T*)q, q_stride, (const T*)k_pool, (const T*)v_pool, page_table,
                   page_table_stride, row_slot, row_pos, (T*)out, out_stride, nq, nkv, d, page_size, window, scale);
     return CITLALI_LAUNCH_CHECK();
@@ -564,7 +563,7 @@ extern "C" int citlali_attention_rows(const void* q, int q_stride, int dtype,
         return kBadShape;
     }
     const size_t smem = (size_t)(head_dim + max_keys) * sizeof(float);
-    if (smem > 200 * 1024) {
+    if (smem > kRowShared) {
         set_last_error("attention_rows: %d keys for one row need %zu bytes of shared memory, more than 204800",
                        max_keys, smem);
         return kTooLarge;
@@ -573,7 +572,7 @@ extern "C" int citlali_attention_rows(const void* q, int q_stride, int dtype,
     // rows and heads above 256 go one head at a time.
     const int group = nq / nkv, hb = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
     const size_t grouped = (size_t)max_keys * (hb + 1) * sizeof(float);
-    if (head_dim <= 256 && grouped <= 56 * 1024) {
+    if (head_dim <= 256 && grouped <= kGroupedShared) {
         return CITLALI_DISPATCH_FLOAT(dtype, T, [&] {
             auto launch = hb == 4 ? launch_grouped<T, 4> : hb == 2 ? launch_grouped<T, 2> : launch_grouped<T, 1>;
             return launch(q, q_stride, k_pool, v_pool, page_table, page_table_stride, row_slot, row_pos, out, out_stride, rows, nq, nkv,
@@ -582,10 +581,7 @@ extern "C" int citlali_attention_rows(const void* q, int q_stride, int dtype,
     }
     return CITLALI_DISPATCH_FLOAT(dtype, T, [&] {
         auto kernel = attention_rows_kernel<T>;
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-        }
+        if (int e = raise_shared_limit(kernel, smem, kRowShared)) return e;
         dim3 grid(rows, nq);
         launch_kernel(kernel, grid, 128, smem, stream, (const T*)q, q_stride, (const T*)k_pool, (const T*)v_pool, page_table,
                                              page_table_stride, row_slot, row_pos, (T*)out, out_stride, nq, nkv,

@@ -52,6 +52,17 @@ inline int device_sm_count() {
     return cached[device];
 }
 
+// Before a launch with `bytes` of dynamic shared memory, at most `most` for any launch of this kernel.  Without more ado a block gets
+// 48 KB, and a kernel's own __shared__ arrays count among them (none here takes 8 KB).  The limit is always raised to `most`, so that
+// of two threads launching with different sizes neither takes the other's away.
+constexpr size_t kSharedWithoutRaise = 40 * 1024;
+constexpr size_t kRowShared = 200 * 1024;       // the most that kernels with a whole row in shared memory ask for
+template <typename Kernel>
+inline int raise_shared_limit(Kernel kernel, size_t bytes, size_t most) {
+    if (bytes <= kSharedWithoutRaise) return 0;
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg = {};

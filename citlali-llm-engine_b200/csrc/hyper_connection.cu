@@ -202,13 +202,12 @@ extern "C" int citlali_hyper_read_norm(const float* X, size_t stream_stride, int
                                        cudaStream_t stream) {
     if (rows <= 0) return 0;
     const size_t smem = (size_t)width * sizeof(float);
-    if (streams < 1 || smem > 200 * 1024) {
+    if (streams < 1 || smem > kRowShared) {
         set_last_error("hyper_read_norm: %d streams of width %d", streams, width);
         return kBadShape;
     }
     return CITLALI_DISPATCH_FLOAT(out_dtype, TO, [&] {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(hyper_read_norm_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (int e = raise_shared_limit(hyper_read_norm_kernel<TO>, smem, kRowShared)) return e;
         // few rows in bfloat16 (decoding): a row is spread over more threads; 32-bit keeps one order of summation
         launch_kernel(hyper_read_norm_kernel<TO>, rows, (sizeof(TO) == 2 && rows < 128 && width >= 2048) ? 1024 : 256, smem, stream, X, stream_stride, streams, w_in, gain, (TO*)out,
                       width, eps);
@@ -235,14 +234,14 @@ extern "C" int citlali_hyper_write_read_norm(float* X, size_t stream_stride, int
                                              int out_dtype, int rows, int width, float eps, cudaStream_t stream) {
     if (rows <= 0) return 0;
     const size_t smem = (size_t)width * sizeof(float);
-    if (streams < 1 || streams > kMaxStreams || smem > 200 * 1024) {
+    if (streams < 1 || streams > kMaxStreams || smem > kRowShared) {
         set_last_error("hyper_write_read_norm: %d streams of width %d", streams, width);
         return kBadShape;
     }
     return CITLALI_DISPATCH_FLOAT(out_dtype, TO, [&] {
         auto kernel = streams == 4 ? hyper_write_read_norm_kernel<TO, 4> : streams == 2 ? hyper_write_read_norm_kernel<TO, 2>
                                                                                         : hyper_write_read_norm_kernel<TO, 0>;
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (int e = raise_shared_limit(kernel, smem, kRowShared)) return e;
         launch_kernel(kernel, rows, (sizeof(TO) == 2 && rows < 128 && width >= 2048) ? 1024 : 256, smem, stream, X, stream_stride, streams, y,
                       w_mix, w_out, w_in, gain, (TO*)out, width, eps);
         return CITLALI_LAUNCH_CHECK();

@@ -326,6 +326,7 @@ extern "C" int citlali_lru_gates(const float* u, const float* wa_t, const float*
         set_last_error("lru_gates: gate blocks of %d channels exceed the kernel's 1536", bw);
         return kTooLarge;
     }
+    if (int e = raise_shared_limit(lru_gates_kernel, smem, 48 * 1024)) return e;
     dim3 grid((rows + kGateRows - 1) / kGateRows, blocks, (bw + 31) / 32);
     launch_kernel(lru_gates_kernel, grid, 128, smem, stream, u, wa_t, ba, wi_t, bi, lam, a_out, coef_out, rows, width, bw);
     return CITLALI_LAUNCH_CHECK();

@@ -446,7 +446,7 @@ extern "C" int citlali_layer_norm_add(const float* y, const void* gain, int gain
                                       int rows, int hidden, float eps, cudaStream_t stream) {
     if (rows <= 0) return 0;
     const size_t smem = (size_t)hidden * sizeof(float);
-    if (hidden <= 0 || smem > 200 * 1024) {
+    if (hidden <= 0 || smem > kRowShared) {
         set_last_error("layer_norm_add: rows of %d elements do not fit a block's shared memory", hidden);
         return kTooLarge;
     }
@@ -462,10 +462,7 @@ extern "C" int citlali_layer_norm_add(const float* y, const void* gain, int gain
     return CITLALI_DISPATCH_FLOAT(gain_dtype, TG, [&] {
         return CITLALI_DISPATCH_FLOAT(emit_dtype, TE, [&] {
             auto kernel = layer_norm_add_kernel<TG, TE>;
-            if (smem > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (e != cudaSuccess) return (int)e;
-            }
+            if (int e = raise_shared_limit(kernel, smem, kRowShared)) return e;
             launch_kernel(kernel, rows, 256, smem, stream, y, (const TG*)gain, x, (TE*)emit, hidden, eps);
             return CITLALI_LAUNCH_CHECK();
         });
@@ -476,7 +473,7 @@ extern "C" int citlali_layer_norm_rows(const float* x, const void* gain, const v
                                        void* out, int out_dtype, int rows, int hidden, float eps, cudaStream_t stream) {
     if (rows <= 0) return 0;
     const size_t smem = (size_t)hidden * sizeof(float);
-    if (hidden <= 0 || smem > 200 * 1024) {
+    if (hidden <= 0 || smem > kRowShared) {
         set_last_error("layer_norm_rows: rows of %d elements do not fit a block's shared memory", hidden);
         return kTooLarge;
     }
@@ -492,10 +489,7 @@ extern "C" int citlali_layer_norm_rows(const float* x, const void* gain, const v
     return CITLALI_DISPATCH_FLOAT(gain_dtype, TG, [&] {
         return CITLALI_DISPATCH_FLOAT(out_dtype, TO, [&] {
             auto kernel = layer_norm_rows_kernel<TG, TO>;
-            if (smem > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (e != cudaSuccess) return (int)e;
-            }
+            if (int e = raise_shared_limit(kernel, smem, kRowShared)) return e;
             launch_kernel(kernel, rows, 256, smem, stream, x, (const TG*)gain, (const TG*)bias, row_index, (TO*)out, hidden, eps);
             return CITLALI_LAUNCH_CHECK();
         });
@@ -521,7 +515,7 @@ extern "C" int citlali_layer_norm_chain(const float* y, const float* in_bias, co
                                         int hidden, float eps1, float eps2, cudaStream_t stream) {
     if (rows <= 0) return 0;
     const size_t smem = (size_t)hidden * sizeof(float);
-    if (hidden <= 0 || smem > 200 * 1024 || g1 == nullptr || (g2 != nullptr && out2 == nullptr)) {
+    if (hidden <= 0 || smem > kRowShared || g1 == nullptr || (g2 != nullptr && out2 == nullptr)) {
         set_last_error("layer_norm_chain: rows of %d elements; the first gain and, with a second norm, its output are needed", hidden);
         return kBadShape;
     }
@@ -540,10 +534,7 @@ extern "C" int citlali_layer_norm_chain(const float* y, const float* in_bias, co
     }
     return CITLALI_DISPATCH_FLOAT(out_dtype, TE, [&] {
         auto kernel = layer_norm_chain_kernel<TE>;
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-        }
+        if (int e = raise_shared_limit(kernel, smem, kRowShared)) return e;
         launch_kernel(kernel, rows, threads, smem, stream, y, in_bias, g1, b1, x, (TE*)emit, g2, b2, (TE*)out2, hidden, eps1, eps2);
         return CITLALI_LAUNCH_CHECK();
     });

@@ -1,5 +1,8 @@
 """Kernels that take several rows, heads or streams at once against plain float64, and against the forms they stand beside."""
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -133,3 +136,64 @@ def test_32_bit_products_give_a_row_the_same_bits_in_steps_of_any_size(N, K, odd
             want, exact = y, x.double() @ w.double().T
             assert float((y.double() - exact).abs().max()) <= 2e-6 * K ** 0.5 * max(1.0, float(exact.abs().max()))
         assert torch.equal(y, want[:rows]) and torch.equal(added, base[:rows] + y)
+
+
+_SHARED_MEMORY_LIMITS = """
+import sys
+sys.path.insert(0, {root!r})
+import torch
+import citlali_b200
+from citlali_b200 import ops
+DEV, d, page = torch.device("cuda:0"), 128, 64
+g = torch.Generator().manual_seed(1)
+pool = torch.randn(191, 1, page, d, generator=g).to(DEV)
+table = torch.arange(191, dtype=torch.int32, device=DEV)[None].contiguous()
+slot = torch.zeros(1, dtype=torch.int32, device=DEV)
+close = lambda a, b: float((a.double() - b).abs().max()) <= 1e-5 * float(b.abs().max())      # sums of up to 12,289 in float32
+
+
+def attention(nq, keys, room):
+    q = torch.randn(1, nq * d, generator=torch.Generator().manual_seed(keys)).to(DEV)
+    out = torch.full((1, nq * d), float("nan"), device=DEV)
+    ops.attention_rows(q, nq * d, pool, pool, table, slot, slot + (keys - 1), out, nq, 1, d, page, 0, room, d ** -0.5)
+    return out
+
+
+# the form of one head at a time first: the reference below needs more shared memory and leaves a higher limit behind
+lengths = [(nq, keys) for nq in (1, 2, 4) for keys in (12128, 12129, 12144, 12160, 12161)]
+lengths += [(4, n) for n in range(2451, 2459)] + [(2, n) for n in range(4090, 4098)] + [(1, n) for n in range(6140, 6146)]
+for (nq, keys), out in [(c, attention(*c, c[1])) for c in lengths]:
+    assert torch.isfinite(out).all() and torch.equal(out, attention(nq, keys, 40000)), (nq, keys)
+
+for W in (12255, 12256, 12264, 12270, 12288, 12289):          # a row of floats beside a block sum's 128 bytes
+    X, y = torch.randn(3, 2, W, generator=g).to(DEV), torch.randn(2, W, generator=g).to(DEV)
+    ones, eye = torch.ones(3, device=DEV), torch.eye(3, device=DEV)
+    gain = torch.ones(W, device=DEV)
+    norm = lambda x: x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5)
+    h = torch.empty(2, W, device=DEV)
+    ops.hyper_read_norm(X, ones, gain, 1e-5, h)
+    assert close(h, norm(X.double().sum(0))), W
+    wrote = X.clone()
+    ops.hyper_write_read_norm(wrote, y, eye, ones, ones, gain, 1e-5, h)
+    assert close(h, norm((X.double() + y.double()).sum(0))), W
+    x = torch.zeros(2, W, device=DEV)
+    ops.layer_norm_add(y, gain, 1e-5, x)
+    ops.layer_norm_rows(y, gain, 1e-5, h)
+    centred = y.double() - y.double().mean(-1, keepdim=True)
+    assert close(x, norm(centred)) and close(h, norm(centred)), W
+for bw in (1280, 1281, 1536):                                  # eight rows of a gate block beside 8 KB of partial sums
+    u, wa, wi = torch.randn(3, bw, generator=g).to(DEV), *(torch.randn(1, bw, bw, generator=g).to(DEV) / bw ** 0.5 for _ in range(2))
+    zero, a, coef = torch.zeros(bw, device=DEV), torch.empty(3, bw, device=DEV), torch.empty(3, bw, device=DEV)
+    ops.lru_gates(u, wa, zero, wi, zero, zero, a, coef, 1)
+    log_a = -8.0 * torch.sigmoid(u.double() @ wa[0].double()) * torch.log(torch.tensor(2.0, dtype=torch.float64))
+    assert close(a, torch.exp(log_a)) and close(coef, torch.sqrt(-torch.expm1(2 * log_a)) * torch.sigmoid(u.double() @ wi[0].double()) * u.double()), bw
+print("every length ran")
+"""
+
+
+def test_every_length_around_the_default_limit_of_shared_memory_runs():
+    """48 KB a block count a kernel's own arrays too.  In a process of its own: a launch that raises a kernel's limit raises it for later
+    ones, so another test's longer rows would hide what is looked for."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _SHARED_MEMORY_LIMITS.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "every length ran" in r.stdout, r.stdout + r.stderr

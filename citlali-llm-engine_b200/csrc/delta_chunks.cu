@@ -136,6 +136,48 @@ struct ScanShared {
     float r[kChunk][VS], u[kChunk][VS], eu[kChunk][VS];
 };
 
+// N (two or four) floats from their natural boundary.
+template <int N>
+struct Floats { float f[N]; };
+template <int N>
+__device__ __forceinline__ Floats<N> load_floats(const float* p) {
+    Floats<N> r;
+    if constexpr (N == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        r.f[0] = v.x; r.f[1] = v.y; r.f[2] = v.z; r.f[3] = v.w;
+    } else {
+        const float2 v = *reinterpret_cast<const float2*>(p);
+        r.f[0] = v.x; r.f[1] = v.y;
+    }
+    return r;
+}
+template <int N>
+__device__ __forceinline__ void store_floats(float* p, const float (&f)[N]) {
+    if constexpr (N == 4) *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+    else *reinterpret_cast<float2*>(p) = make_float2(f[0], f[1]);
+}
+
+// sum += W[row, 0 .. row] X[0 .. row, col ..], rows in order.  What W holds above its diagonal (zeros, or not a number where a later
+// token is none) and X's later rows must not meet: a token reaches no earlier one, infinite or not.  A warp has four rows, so only its
+// last four of W's columns need to ask.
+template <int N, int VS>
+__device__ __forceinline__ void add_rows_up_to(float (&sum)[N], const float* W, const float (&X)[kChunk][VS], int row, int col) {
+    auto tile = [&](int j, bool ask) {
+        const Floats<4> w = load_floats<4>(W + row * kChunk + j);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const Floats<N> x = load_floats<N>(&X[j + e][col]);
+            if (!ask || j + e <= row) {
+#pragma unroll
+                for (int c = 0; c < N; ++c) sum[c] = fmaf(w.f[e], x.f[c], sum[c]);
+            }
+        }
+    };
+    const int own = row & ~3;
+    for (int j = 0; j < own; j += 4) tile(j, false);
+    tile(own, true);
+}
+
 template <int VS>
 __global__ void __launch_bounds__(256)
 delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const float* __restrict__ coef, float* __restrict__ state,
@@ -203,9 +245,9 @@ delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const f
         }
     // [K; Q] S: slice `slice` of k, columns 4 xc .. 4 xc + 3, rows xr + 8 i (i < 4: keys, else queries)
     const int slice = tid / (8 * CG), xc = tid % CG, xr = (tid / CG) & 7;
-    // the 32 x VS matrices: row `ur`, columns 4 uc .. 4 uc + 3 (VS = 16: the first half of the threads)
-    const int ur = tid / CG, uc = tid % CG;
-    const bool mine = ur < kChunk;
+    // the 32 x VS matrices: row `ur`, UC columns from `uc` (a warp four rows)
+    constexpr int UC = VS / 8;
+    const int ur = tid >> 3, uc = (tid & 7) * UC;
     for (int ch = 0; ch < chunks; ++ch) {
         const int buf = ch & 1;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -238,57 +280,30 @@ delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const f
         const float* M = T + kChunk * kChunk;
         const float* G = M + kChunk * kChunk;
         const float* E = G + kChunk;
-        float y[4] = {0.f, 0.f, 0.f, 0.f};
-        if (mine) {
-            float x[4] = {0.f, 0.f, 0.f, 0.f};
+        float y[UC], r[UC], u[UC], eu[UC];
 #pragma unroll
-            for (int s = 0; s < SLICES; ++s) {
-                const float4 a = *reinterpret_cast<const float4*>(&sm.part[s][ur][uc * 4]);
-                const float4 b = *reinterpret_cast<const float4*>(&sm.part[s][kChunk + ur][uc * 4]);
-                x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
-                y[0] += b.x; y[1] += b.y; y[2] += b.z; y[3] += b.w;
-            }
-            const float Gi = G[ur];
-            const float4 v = *reinterpret_cast<const float4*>(&sm.v[buf][ur][uc * 4]);
-            *reinterpret_cast<float4*>(&sm.r[ur][uc * 4]) = make_float4(fmaf(-Gi, x[0], v.x), fmaf(-Gi, x[1], v.y), fmaf(-Gi, x[2], v.z), fmaf(-Gi, x[3], v.w));
+        for (int c = 0; c < UC; ++c) r[c] = y[c] = u[c] = 0.0f;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) y[e] *= Gi;
+        for (int s = 0; s < SLICES; ++s) {
+            const Floats<UC> a = load_floats<UC>(&sm.part[s][ur][uc]), b = load_floats<UC>(&sm.part[s][kChunk + ur][uc]);
+#pragma unroll
+            for (int c = 0; c < UC; ++c) { r[c] += a.f[c]; y[c] += b.f[c]; }
         }
+        const float Gi = G[ur], Ei = E[ur];
+        const Floats<UC> v = load_floats<UC>(&sm.v[buf][ur][uc]);
+#pragma unroll
+        for (int c = 0; c < UC; ++c) { r[c] = fmaf(-Gi, r[c], v.f[c]); y[c] *= Gi; }
+        store_floats<UC>(&sm.r[ur][uc], r);
         __syncthreads();
-        // the rows a warp has end here (T and M are zero above the diagonal)
-        const int last = min(kChunk, ((tid | 31) / CG) + 1);
-        if (mine) {
-            float u[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int j = 0; j < last; j += 4) {
-                const float4 t = *reinterpret_cast<const float4*>(T + ur * kChunk + j);
-                const float tj[4] = {t.x, t.y, t.z, t.w};
+        add_rows_up_to<UC>(u, T, sm.r, ur, uc);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float4 r = *reinterpret_cast<const float4*>(&sm.r[j + e][uc * 4]);
-                    u[0] = fmaf(tj[e], r.x, u[0]); u[1] = fmaf(tj[e], r.y, u[1]);
-                    u[2] = fmaf(tj[e], r.z, u[2]); u[3] = fmaf(tj[e], r.w, u[3]);
-                }
-            }
-            const float e = E[ur];
-            *reinterpret_cast<float4*>(&sm.u[ur][uc * 4]) = make_float4(u[0], u[1], u[2], u[3]);
-            *reinterpret_cast<float4*>(&sm.eu[ur][uc * 4]) = make_float4(e * u[0], e * u[1], e * u[2], e * u[3]);
-        }
+        for (int c = 0; c < UC; ++c) eu[c] = Ei * u[c];
+        store_floats<UC>(&sm.u[ur][uc], u);
+        store_floats<UC>(&sm.eu[ur][uc], eu);
         __syncthreads();
-        if (mine) {
-            for (int j = 0; j < last; j += 4) {
-                const float4 t = *reinterpret_cast<const float4*>(M + ur * kChunk + j);
-                const float tj[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float4 r = *reinterpret_cast<const float4*>(&sm.u[j + e][uc * 4]);
-                    y[0] = fmaf(tj[e], r.x, y[0]); y[1] = fmaf(tj[e], r.y, y[1]);
-                    y[2] = fmaf(tj[e], r.z, y[2]); y[3] = fmaf(tj[e], r.w, y[3]);
-                }
-            }
-            const int token = ch * kChunk + ur;
-            if (token < tokens && v0 + uc * 4 < V)
-                *reinterpret_cast<float4*>(out + (size_t)(row0 + token) * H * V + h * V + v0 + uc * 4) = make_float4(y[0], y[1], y[2], y[3]);
-        }
+        add_rows_up_to<UC>(y, M, sm.u, ur, uc);
+        const int token = ch * kChunk + ur;
+        if (token < tokens && v0 + uc < V) store_floats<UC>(out + (size_t)(row0 + token) * H * V + h * V + v0 + uc, y);
         const float G_all = G[kChunk - 1];
 #pragma unroll
         for (int i = 0; i < RS; ++i)

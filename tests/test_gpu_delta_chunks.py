@@ -1,5 +1,7 @@
 """The gated delta rule 32 tokens at a time against the recurrence in float64, and no further off than the walk: lengths around a chunk,
 sequences side by side, states carried over, key and value sizes that do not fill the tiles, decays of nothing and of everything."""
+import math
+
 import pytest
 import torch
 
@@ -67,3 +69,33 @@ def test_chunks_against_float64_and_the_walk(D, V, H, KH, lengths, decays):
     # 32-bit sums: a few 2^-24 each, along chains of a chunk's 32 tokens instead of the walk's pairs
     for a, b in zip(off["chunks"], off["walk"]):
         assert a <= 2e-6 and a <= 2.0 * b + 1e-7, off
+
+
+@pytest.mark.parametrize("heads", [4, 64])                    # columns of the values a block: 16, 32
+@pytest.mark.parametrize("part", ["query", "key", "value", "strength", "decay"])
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+def test_a_token_that_is_not_finite_reaches_no_earlier_one(heads, part, bad):
+    """Not even times zero: the rows before it keep their bits, whatever their places in its chunk."""
+    D = V = 128
+    H, KH, T, C = heads, heads // 2, 75, heads * 2 * D
+    assert (2 * H * 4 >= torch.cuda.get_device_properties(0).multi_processor_count * 3 // 4) == (heads == 64)
+    g = torch.Generator().manual_seed(heads)
+    prep = torch.zeros(T, C + 2 * H)
+    prep[:, :2 * KH * D] = torch.nn.functional.normalize(torch.randn(T, 2 * KH, D, generator=g), dim=-1).view(T, -1)
+    prep[:, 2 * KH * D:C] = torch.randn(T, H * V, generator=g)
+    prep[:, C:] = 0.5 + 0.5 * torch.rand(T, 2 * H, generator=g)
+    span = {"query": (0, KH * D), "key": (KH * D, 2 * KH * D), "value": (2 * KH * D, C), "strength": (C, C + H), "decay": (C + H, C + 2 * H)}[part]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    def run(rows):
+        out = torch.full((2 * T, H * V), float("nan"), device=DEV)
+        ops.delta_chunks(torch.cat([rows, prep]).to(DEV), torch.zeros(2, H * D * V, device=DEV), i32([0, T, 2 * T]), i32([1, 0]), 2, T, H, KH, D, V, out)
+        return out[:T].cpu(), out[T:].cpu()
+
+    clean, beside = run(prep)
+    for at in (0, 1, 2, 3, 6, 17, 30, 31, 32, 45, 63, 64, 74):
+        rows = prep.clone()
+        rows[at, span[0]:span[1]] = bad
+        got, other = run(rows)
+        assert torch.equal(got[:at], clean[:at]) and torch.equal(other, beside), (at, int(torch.isfinite(got).all(1).long().argmin()))
+        assert not torch.isfinite(got[at]).all()

@@ -28,12 +28,19 @@ __device__ __forceinline__ int2 seen_tiles(int past, int n, int window) {
     return make_int2(lo / kKeyTile, n > 0 ? (past + n - 1) / kKeyTile + 1 : lo / kKeyTile);
 }
 
+// Whether one of eight bfloat16 has all bits of its exponent set.
+__device__ __forceinline__ bool not_all_finite(uint4 v) {
+    auto pair = [](uint32_t w) { return (w & 0x7f800000u) == 0x7f800000u || (w & 0x7f80u) == 0x7f80u; };
+    return pair(v.x) || pair(v.y) || pair(v.z) || pair(v.w);
+}
+
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, const int32_t* __restrict__ page_table, int table_stride, int page_size,
                      const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_slot, const int32_t* __restrict__ seq_past,
                      int R, int P, int window, __nv_bfloat16* __restrict__ latents, __nv_bfloat16* __restrict__ shared_keys,
                      int32_t* __restrict__ key_rows, int key_total) {
     __shared__ int first_row;
+    __shared__ int spoilt[32];                                // this block's rows whose latents are not all finite
     dependents_may_launch();
     wait_for_predecessor();
     const int seq = blockIdx.y, lane = threadIdx.x & 31;
@@ -42,6 +49,7 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, const int32_t* __re
     const int tile = mine.x + blockIdx.x / 4;                 // four blocks a tile: 32 rows each
     if (tile >= mine.y) return;
     if (threadIdx.x < 32) {                                   // the rows of the sequences before this one
+        spoilt[lane] = 0;
         int before = 0;
         for (int s = lane; s < seq; s += 32) {
             const int2 t = seen_tiles(seq_past[s], seq_start[s + 1] - seq_start[s], window);
@@ -56,15 +64,29 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, const int32_t* __re
     const int lo = window > 0 ? max(0, past - window + 1) : 0, hi = past + n;        // the positions seen
     const int E = R + P, chunks = (R + 64) / 8, r_chunks = R / 8, e_chunks = E / 8;
     const int32_t* table = page_table + (size_t)seq_slot[seq] * table_stride;
+    const int key0 = tile * kKeyTile + (blockIdx.x & 3) * 32;
     for (int i = threadIdx.x; i < 32 * chunks; i += 256) {
-        const int key = tile * kKeyTile + (blockIdx.x & 3) * 32 + i / chunks, ch = i % chunks;
-        const int row = first_row + key;
+        const int r = i / chunks, key = key0 + r, ch = i % chunks, row = first_row + key;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (key >= lo && key < hi && ch < e_chunks)
             v = *reinterpret_cast<const uint4*>(pool + ((size_t)table[key / page_size] * page_size + key % page_size) * E + ch * 8);
         if (row >= key_total) continue;                       // (a caller that counted otherwise: nothing is written past its buffers)
-        if (ch < r_chunks) *reinterpret_cast<uint4*>(latents + (size_t)row * R + ch * 8) = v;
-        else *reinterpret_cast<uint4*>(shared_keys + (size_t)row * 64 + (ch - r_chunks) * 8) = v;
+        if (ch < r_chunks) {
+            *reinterpret_cast<uint4*>(latents + (size_t)row * R + ch * 8) = v;
+            if (not_all_finite(v)) spoilt[r] = 1;
+        } else {
+            *reinterpret_cast<uint4*>(shared_keys + (size_t)row * 64 + (ch - r_chunks) * 8) = v;
+        }
+    }
+    __syncthreads();
+    // A latent that is not all finite (and was written: those rows alone are marked): its values would meet the zeros that rows which do
+    // not see it have for weights.  They become zero, and a key that is not a number says the same to the rows that do see it.
+    for (int r = threadIdx.x >> 5; r < 32; r += 8) {
+        if (!spoilt[r]) continue;
+        const size_t row = first_row + key0 + r;
+        for (int ch = threadIdx.x & 31; ch < r_chunks; ch += 32) *reinterpret_cast<uint4*>(latents + row * R + ch * 8) = make_uint4(0u, 0u, 0u, 0u);
+        if ((threadIdx.x & 31) < 8)
+            *reinterpret_cast<uint4*>(shared_keys + row * 64 + (threadIdx.x & 31) * 8) = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
     }
 }
 

@@ -113,3 +113,32 @@ def test_a_sequence_beside_one_of_infinities():
         a, b, c = cache.acquire(), cache.acquire(), cache.acquire()
         out.append(run_steps(mixer, cache, HIDDEN, [[(a, other[:200]), (b, x[:130]), (c, other)]], torch.bfloat16)[b])
     assert torch.isfinite(out[1]).all() and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("window, sink", [(None, True), (100, True), (None, False)])
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("walk", [False, True])
+def test_a_token_that_is_not_finite_reaches_the_rows_that_see_it_and_no_others(window, sink, bad, walk):
+    """Rows before it, and rows whose window has left it behind, stay what they are (up to the order of a sum, which the prompt kernel
+    chooses for 32 rows together); no row that sees it has a finite result."""
+    mixer, _ = mixer_for(heads=2, window=window, sink=sink)
+    w = weights_for(mixer, 8, {"_norm": lambda r: 1 + 0.3 * r, "sink": lambda r: r})
+    mixer.bind(handles(w, torch.bfloat16), ctx_for(torch.bfloat16))
+    if walk:
+        mixer.kv_up = None
+    x = torch.randn(420, HIDDEN, generator=torch.Generator().manual_seed(9)).to(torch.bfloat16).float()
+
+    def run(rows):
+        cache = SequenceCache([mixer.cache_requirement()], 2, 2048, 512, torch.bfloat16, DEV)
+        a = cache.acquire()
+        return run_steps(mixer, cache, HIDDEN, [[(a, rows[:260])], [(a, rows[260:])]], torch.bfloat16)[a]
+
+    clean = run(x)
+    for at in (1, 77, 127, 128, 250, 300):
+        rows = x.clone()
+        rows[at] = bad
+        got = run(rows)
+        sees = torch.zeros(420, dtype=torch.bool)
+        sees[at:at + (window or 420)] = True
+        assert float((got - clean)[~sees].abs().max()) <= 2 ** -8 * float(clean.abs().max()), at
+        assert not torch.isfinite(got[sees]).any(), at

@@ -25,10 +25,14 @@ class StepEntry:
 
 
 def _as_ids(tokens: list) -> np.ndarray:
+    """The ids as torch reads them.  numpy is quicker and reads whole numbers alike, but takes strings of digits for numbers too."""
     try:
-        return np.array(tokens, dtype=np.int64)
-    except (TypeError, ValueError):                   # numbers that numpy does not read (elements of a tensor on the device)
+        ids = np.array(tokens)
+    except (TypeError, ValueError, RuntimeError):     # what numpy does not read (elements of a tensor on the device)
+        ids = None
+    if ids is None or ids.dtype.kind not in "ib":
         return torch.as_tensor(tokens, dtype=torch.int64).numpy()
+    return ids.astype(np.int64, copy=False)
 
 
 def pack_step(entries: List[StepEntry], past: List[int], vocab_size: int, device) -> StepBatch:

@@ -808,14 +808,6 @@ extern "C" int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int
 // order of w's rows); mode bit 3 = y is bfloat16 max(v, 0)^2.  At most one of the bits 1 to 3, and only bit 0 with none of them.
 extern "C" int citlali_gemm_tc_act(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode, const float* bias,
                                    int32_t* error_flag, int sm_count, cudaStream_t stream) {
-    const int gates = mode & 14;
-    if ((mode & ~15) || (gates & (gates - 1)) || ((mode & 1) && gates) || ((mode & 8) && y_dtype != kBF16)) {
-        set_last_error("gemm_tc_act: mode %d with output dtype code %d is no form of the epilogue", mode, y_dtype);
-        return kBadShape;
-    }
-    if ((uintptr_t)bias & 15u) {
-        set_last_error("gemm_tc_act: the bias must start on a 16-byte boundary");
-        return kBadAlignment;
-    }
+    if (int code = tc::check_epilogue("gemm_tc_act", mode, y_dtype, bias)) return code;
     return gemm_tc_any(x, w, y, y_dtype, M, N, K, mode, 0, error_flag, sm_count, nullptr, nullptr, nullptr, 0, 0, 0.0f, bias, stream);
 }

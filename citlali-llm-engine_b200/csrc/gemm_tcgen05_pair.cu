@@ -295,18 +295,19 @@ extern "C" int citlali_gemm_tc_pair_plan(int M, int N, int K, int* bn, int* pair
     return 0;
 }
 
-// y = x . w^T as citlali_gemm_tc computes it (same `mode` bits, same outputs), on pairs of SMs.
+// y = x . w^T as citlali_gemm_tc computes it (same `mode` bits 0 and 1, same outputs), on pairs of SMs.
 // For many rows of x; it takes every M, N and K that citlali_gemm_tc takes.
 extern "C" int citlali_gemm_tc_pair(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K,
                                     int mode, int32_t* error_flag, cudaStream_t stream) {
-    return citlali_gemm_tc_pair_act(x, w, y, y_dtype, M, N, K, mode, nullptr, error_flag, stream);
+    return citlali_gemm_tc_pair_act(x, w, y, y_dtype, M, N, K, mode & 3, nullptr, error_flag, stream);
 }
 
-// The same with a bias and the further `mode` bits of citlali_gemm_tc_act, which checks them.
+// The same with a bias and the further `mode` bits of citlali_gemm_tc_act.
 extern "C" int citlali_gemm_tc_pair_act(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode,
                                         const float* bias, int32_t* error_flag, cudaStream_t stream) {
     const bool accumulate = (mode & 1) != 0, gelu = (mode & 4) != 0, swiglu = (mode & 2) != 0 || gelu;
     if (M <= 0 || N <= 0) return 0;
+    if (int code = tc::check_epilogue("gemm_tc_pair", mode, y_dtype, bias)) return code;
     if (K <= 0 || K % 8 != 0) {
         set_last_error("gemm_tc_pair: the inner size %d must be a positive multiple of 8 (rows of 16-byte multiples for TMA)", K);
         return kBadShape;

@@ -29,6 +29,21 @@ inline EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
+// Whether `mode` (bit 0 adds, 1 gates by SiLU, 2 gates by GELU, 3 squares max(v, 0)), the output and the bias make a form of a product's
+// epilogue: at most one of the bits 1 to 3, bit 0 with none of them, squares in bfloat16, and a bias that is read in 16-byte pieces.
+inline int check_epilogue(const char* who, int mode, int y_dtype, const float* bias) {
+    const int gates = mode & 14;
+    if ((mode & ~15) || (gates & (gates - 1)) || ((mode & 1) && gates) || ((mode & 8) && y_dtype != kBF16)) {
+        set_last_error("%s: mode %d with output dtype code %d is no form of the epilogue", who, mode, y_dtype);
+        return kBadShape;
+    }
+    if ((uintptr_t)bias & 15u) {
+        set_last_error("%s: the bias must start on a 16-byte boundary", who);
+        return kBadAlignment;
+    }
+    return 0;
+}
+
 // A [rows, row_elems] bfloat16 matrix with a row pitch of `pitch_elems` elements as tiles of [box_rows, 64] with
 // 128-byte swizzle; outside the matrix a tile reads zeros.  `who` names the caller in the error text.
 //

@@ -7,11 +7,15 @@ import pytest
 from citlali_b200 import ops
 
 
-def plan(M, N, K, sms=148, force=0):
+def library():
     try:
-        lib = ops.lib()
+        return ops.lib()
     except Exception as e:                       # no compiler on this machine
         pytest.skip(f"the kernel library cannot be built here: {e}")
+
+
+def plan(M, N, K, sms=148, force=0):
+    lib = library()
     swapped, bn, splits = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
     lib.citlali_gemm_tc_plan(M, N, K, sms, force, ctypes.byref(swapped), ctypes.byref(bn), ctypes.byref(splits))
     return bool(swapped.value), bn.value, splits.value
@@ -57,3 +61,19 @@ def test_the_plan_depends_on_the_number_of_sms():
     assert plan(8, 6144, 4096, sms=148)[2] == 4
     assert plan(8, 6144, 4096, sms=64)[2] == 2           # 128 places for 48 tiles
     assert plan(8, 6144, 4096, sms=20)[2] == 1
+
+
+F32, BF16 = 0, 1
+
+
+@pytest.mark.parametrize("entry", ["citlali_gemm_tc_act", "citlali_gemm_tc_pair_act"])
+@pytest.mark.parametrize("mode, y_dtype, bias, code", [
+    (8, F32, 0, -2), (1 | 8, F32, 0, -2), (1 | 8, BF16, 0, -2), (2 | 4, BF16, 0, -2), (2 | 8, BF16, 0, -2), (1 | 4, F32, 0, -2), (16, F32, 0, -2),
+    (0, F32, 4100, -4), (8, BF16, 4104, -4), (4, BF16, 4108, -4)])
+def test_epilogues_that_are_none_are_refused_before_any_launch(entry, mode, y_dtype, bias, code):
+    """Addresses nobody reads: the answer comes from the arguments alone."""
+    lib = library()
+    args = [4096, 4096, 4096, y_dtype, 600, 64, 64, mode, bias, None]
+    args += [148, None] if entry == "citlali_gemm_tc_act" else [None]
+    assert getattr(lib, entry)(*args) == code
+    assert (b"no form of the epilogue" if code == -2 else b"16-byte boundary") in lib.citlali_last_error()

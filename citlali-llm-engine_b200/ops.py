@@ -87,7 +87,11 @@ def _need_cuda(*tensors):
 
 # plain numbers of the kind the C argument wants (an integer argument takes no float)
 _i = _sz = operator.index
-_f = float
+
+
+def _f(number):
+    """A float argument as it is: its declared type takes numbers alone, where ``float`` would read a text."""
+    return number
 
 
 def embed_rows(table: torch.Tensor, tokens: torch.Tensor, out: torch.Tensor, error_flag: torch.Tensor,

@@ -63,3 +63,16 @@ def test_an_entry_point_compiles_its_own_source_only(tmp_path, monkeypatch):
     again = build.Kernels()                                # nothing is compiled twice
     again.prepare(["sampling"])
     assert os.path.getmtime(tmp_path / "sampling.o") == stamp
+
+
+@pytest.mark.parametrize("number", ["-1.0", b"-1", None, [-1.0]], ids=repr)
+def test_a_float_argument_takes_numbers_alone(number):
+    """(A cap below zero is refused by the entry point itself: nothing is launched either way.)"""
+    from citlali_b200 import ops
+    try:
+        lib = ops.lib()
+    except Exception as e:                       # no compiler on this machine
+        pytest.skip(f"the kernel library cannot be built here: {e}")
+    assert lib.citlali_soft_cap(None, ops._sz(4), ops._f(-1), None) < 0
+    with pytest.raises((TypeError, ctypes.ArgumentError)):
+        lib.citlali_soft_cap(None, ops._sz(4), ops._f(number), None)

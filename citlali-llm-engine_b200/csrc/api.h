@@ -254,6 +254,8 @@ int citlali_delta_prepare(const float* proj, int proj_stride, const float* taps_
                           const int32_t* seq_slot, int sequences, const float* a_log, const float* dt_bias, float* prep,
                           int rows, int H, int KH, int D, int V, float unit_eps, int block_a_segment, int beta_col,
                           int decay_col, const float* decay_in, int decay_stride, int channel_decay, cudaStream_t stream);
+// Whether the form of a warp a head works through runs of eight rows or has a warp a row (the same bits).
+int citlali_delta_prepare_in_runs(int rows, int H, int KH, int D, int V, int taps, int channel_decay);
 // (block_a_segment 1: a block a segment, for few rows; 2: the same, for a step of one row a sequence, in one launch.
 // beta_col, decay_col: the columns of b and a in a row of proj.  decay_in (rows decay_stride floats apart) given: the
 // decays' inputs come from there instead of proj.  channel_decay: one decay a head and key channel instead of one a head,

@@ -114,7 +114,7 @@ delta_prepare_kernel(const float* __restrict__ proj, int proj_stride, const floa
 // The same for TAPS taps and segments of at most 32 CPL channels, RUN rows a warp: an input is read once, for the RUN rows whose
 // convolution it enters, instead of once a tap, and the taps once for all of them (the kernel above reads eight numbers for every one
 // it writes).  The same operations in the same order, so the same bits.  Bound by the bytes of proj and prep: 2,048 rows of 8,192
-// channels, four taps: 54 us, above 123 us.
+// channels, four taps: 55 us, above 121 us.  (For many rows: see citlali_delta_prepare_in_runs.)
 constexpr int kPrepareRun = 8;
 
 template <int TAPS, int CPL>
@@ -656,6 +656,17 @@ delta_output_vec_kernel(const float* __restrict__ o, const float* __restrict__ g
 
 using namespace citlali;
 
+// Many segments: runs of rows, a warp for eight rows of one.  Fewer leave the device waiting for a warp's eight rows one after the other,
+// where a warp a row has them all at once (same bits); one or two rows are such a run's own length.  A decay a channel is D more numbers
+// a row for a warp, so its line lies higher.  us, a warp a row / runs, four taps: 128 x 128, 32 segments of 8, 64, 192, 320, 2,048 rows
+// 6.0 / 8.4, 7.3 / 8.8, 9.8 / 9.5, 12.2 / 10.3, 58 / 26; 64 x 64, 8 segments of 512, 1,024, 1,280, 2,048 rows 6.1 / 8.0, 7.9 / 8.4,
+// 9.1 / 8.9, 12.5 / 9.3; one row of 32 segments 6.4 / 4.9; a decay a channel, 128 x 128, 48 segments of 1, 2, 256, 341, 682 rows
+// 7.0 / 5.9, 6.9 / 7.6, 15 / 21, 18 / 21, 32 / 29.
+extern "C" int citlali_delta_prepare_in_runs(int rows, int H, int KH, int D, int V, int taps, int channel_decay) {
+    if (taps < 2 || taps > 4 || D > 256 || V > 256) return 0;
+    return rows <= (channel_decay ? 1 : 2) || (long)rows * (2 * KH + H) >= (channel_decay ? 32768 : 10240) ? 1 : 0;
+}
+
 extern "C" int citlali_delta_prepare(const float* proj, int proj_stride, const float* taps_w, int taps, float* state,
                                      size_t state_stride, size_t conv_off, const int32_t* row_slot,
                                      const int32_t* seq_start, const int32_t* seq_slot, int sequences,
@@ -689,7 +700,7 @@ extern "C" int citlali_delta_prepare(const float* proj, int proj_stride, const f
         launch_kernel(delta_prepare_block_kernel, prepare_grid, 128, smem, stream, proj, proj_stride, taps_w, taps,
                       state, state_stride, conv_off, row_slot, a_log, dt_bias, prep, H, KH, D, V, unit_eps,
                       beta_col, decay_col, decay_in, decay_stride, channel_decay, keeps ? 1 : 0);
-    } else if (taps >= 2 && taps <= 4 && D <= 256 && V <= 256) {
+    } else if (citlali_delta_prepare_in_runs(rows, H, KH, D, V, taps, channel_decay)) {
         dim3 prepare_grid((rows + kPrepareRun - 1) / kPrepareRun, (segments + 3) / 4);
         const bool narrow = D <= 128 && V <= 128;
         auto kernel = taps == 4 ? (narrow ? delta_prepare_run_kernel<4, 4> : delta_prepare_run_kernel<4, 8>)

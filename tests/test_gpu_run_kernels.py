@@ -83,6 +83,41 @@ def test_delta_prepare_against_float64(taps, D, V, channel):
         assert torch.equal(kept[s, H * D * V:].cpu().view(taps - 1, C), torch.cat([before, proj[lo:hi, :C]])[n:])
 
 
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("D, V, channel", [(128, 128, False), (20, 40, False), (160, 72, False), (48, 256, True)])
+def test_delta_prepare_has_the_same_bits_in_steps_of_any_size(taps, D, V, channel):
+    """Runs of rows and a warp a row: sequences in one step, and cut into steps of few rows and of a hundred."""
+    H, KH, lengths, slots = 4, 2, [1, 700, 9, 2, 588], [3, 0, 4, 2, 1]
+    if channel:                                                # more heads, for a step that takes runs
+        H, KH = 14, 7
+    T, C, GD = sum(lengths), 2 * KH * D + H * V, D if channel else 1
+    takes_runs = lambda rows: bool(ops.lib().citlali_delta_prepare_in_runs(rows, H, KH, D, V, taps, int(channel)))
+    assert takes_runs(T) and takes_runs(1) and takes_runs(2) != channel and not takes_runs(100)
+    g = torch.Generator().manual_seed(taps * D + 1)
+    dev = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    proj, decay = dev(T, C + H * V + 2 * H), dev(T, H * GD) if channel else None
+    w, a_log, bias, state = dev(C, taps), 0.3 * dev(H), dev(H * GD), dev(5, H * D * V + (taps - 1) * C)
+    i32 = lambda t: torch.as_tensor(t, dtype=torch.int32, device=DEV)
+
+    def run(kept, rows, counts, of_slots):
+        bounds = [sum(counts[:i]) for i in range(len(counts) + 1)]
+        prep = torch.full((bounds[-1], C + H + H * GD), float("nan"), device=DEV)
+        ops.delta_prepare(proj[rows].contiguous(), w, kept, H * D * V, i32([s for s, n in zip(of_slots, counts) for _ in range(n)]), i32(bounds),
+                          i32(of_slots), len(counts), a_log, bias, prep, H, KH, D, V, 1e-6,
+                          decay_in=None if decay is None else decay[rows].contiguous(), channel_decay=channel)
+        return prep
+
+    kept = state.clone()
+    whole = run(kept, slice(0, T), lengths, slots)
+    assert torch.isfinite(whole).all()
+    for cut in (100, 1 if channel else 2):
+        at, parts, part_kept = 0, [], state.clone()
+        for n, s in zip(lengths, slots):
+            parts += [run(part_kept, slice(at + i, at + min(i + cut, n)), [min(cut, n - i)], [s]) for i in range(0, n, cut)]
+            at += n
+        assert torch.equal(torch.cat(parts), whole) and torch.equal(part_kept, kept)
+
+
 @pytest.mark.parametrize("S", [1, 2, 3, 4, 8])
 @pytest.mark.parametrize("rows, W", [(3, 64), (5, 30), (130, 2048)])
 def test_stream_writes_against_float64(S, rows, W):

@@ -63,6 +63,15 @@ def test_the_plan_depends_on_the_number_of_sms():
     assert plan(8, 6144, 4096, sms=20)[2] == 1
 
 
+@pytest.mark.parametrize("rows, H, KH, D, V, taps, channel, runs", [case[:6] + (0,) + case[6:] for case in [
+    (1, 16, 8, 128, 128, 4, True), (2, 2, 1, 32, 32, 4, True), (3, 16, 8, 128, 128, 4, False), (64, 32, 16, 128, 128, 4, False),
+    (319, 16, 8, 128, 128, 4, False), (320, 16, 8, 128, 128, 4, True), (1279, 4, 2, 64, 64, 2, False), (1280, 4, 2, 64, 64, 2, True),
+    (4096, 16, 8, 128, 128, 5, False), (4096, 16, 8, 128, 257, 4, False), (4096, 16, 8, 128, 128, 1, False)]] + [
+    (1, 4, 4, 64, 64, 4, 1, True), (2, 4, 4, 64, 64, 4, 1, False), (682, 16, 16, 128, 128, 4, 1, False), (683, 16, 16, 128, 128, 4, 1, True)])
+def test_the_delta_rules_preparation_takes_runs_of_rows_where_there_are_many(rows, H, KH, D, V, taps, channel, runs):
+    assert bool(library().citlali_delta_prepare_in_runs(rows, H, KH, D, V, taps, channel)) == runs
+
+
 F32, BF16 = 0, 1
 
 

@@ -89,6 +89,8 @@ int citlali_attention_rows(const void* q, int q_stride, int dtype,
                            void* out, int out_stride, int rows, int nq, int nkv, int head_dim,
                            int page_size, int window, int max_keys, float scale,
                            cudaStream_t stream);
+// How many heads of a group it takes together, 0: one head at a time (the same bits).
+int citlali_attention_rows_heads(int nq, int nkv, int head_dim, int max_keys);
 
 // Attention of single new tokens (bfloat16) split over the context; positions are read on the
 // device, `max_positions` bounds them and fixes the grid.  `partial` is float scratch of

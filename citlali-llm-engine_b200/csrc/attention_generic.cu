@@ -545,6 +545,15 @@ extern "C" int citlali_qk_norm_rope_cache(void* qkv, int dtype, const void* q_ga
     });
 }
 
+// Heads of a group together (four, two or one) where the scores of a row's keys fit a quarter of an SM's shared memory; longer rows and
+// heads above 256 go one head at a time (0).  So do rows of fewer than eight keys where heads have no others to share a key with: most of
+// the sixteen scores on their way are then of no key.  8 heads of 128 with a key head each, 1,000 rows of 1, 4, 6, 8 keys, one head at a
+// time / a head's scores together: 15.5 / 26, 22 / 27, 29 / 29, 33 / 27 us; 16 of 64: 27 / 48, 34 / 48, 43 / 52, 49 / 49.
+extern "C" int citlali_attention_rows_heads(int nq, int nkv, int head_dim, int max_keys) {
+    const int group = nq / nkv, hb = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
+    return head_dim <= 256 && (size_t)max_keys * (hb + 1) * sizeof(float) <= kGroupedShared && (hb > 1 || max_keys >= 8) ? hb : 0;
+}
+
 extern "C" int citlali_attention_rows(const void* q, int q_stride, int dtype,
                                       const void* k_pool, const void* v_pool, int cache_dtype,
                                       const int32_t* page_table, int page_table_stride,
@@ -568,11 +577,9 @@ extern "C" int citlali_attention_rows(const void* q, int q_stride, int dtype,
                        max_keys, smem);
         return kTooLarge;
     }
-    // Heads of a group together (four, two or one) where the scores of a row's keys fit a quarter of an SM's shared memory; longer
-    // rows and heads above 256 go one head at a time.
-    const int group = nq / nkv, hb = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
-    const size_t grouped = (size_t)max_keys * (hb + 1) * sizeof(float);
-    if (head_dim <= 256 && grouped <= kGroupedShared) {
+    const int hb = citlali_attention_rows_heads(nq, nkv, head_dim, max_keys);
+    if (hb > 0) {
+        const size_t grouped = (size_t)max_keys * (hb + 1) * sizeof(float);
         return CITLALI_DISPATCH_FLOAT(dtype, T, [&] {
             auto launch = hb == 4 ? launch_grouped<T, 4> : hb == 2 ? launch_grouped<T, 2> : launch_grouped<T, 1>;
             return launch(q, q_stride, k_pool, v_pool, page_table, page_table_stride, row_slot, row_pos, out, out_stride, rows, nq, nkv,

@@ -47,6 +47,26 @@ def test_attention_rows_of_a_group_have_the_bits_of_single_heads(nq, nkv, d, win
         at += n
 
 
+@pytest.mark.parametrize("nq, nkv, d", [(8, 8, 128), (6, 2, 20), (8, 2, 128), (16, 8, 64), (3, 3, 256)])
+def test_attention_over_a_few_keys_has_the_bits_of_single_heads(nq, nkv, d):
+    g = torch.Generator().manual_seed(nq + d)
+    k, v = (torch.randn(1, nkv, 64, d, generator=g).to(DEV) for _ in range(2))
+    table = torch.zeros(1, 1, dtype=torch.int32, device=DEV)
+    for keys in (1, 2, 7, 8, 9, 17):
+        slot, pos = torch.zeros(keys, dtype=torch.int32, device=DEV), torch.arange(keys, dtype=torch.int32, device=DEV)
+        q, outs = torch.randn(keys, nq * d, generator=g).to(DEV), []
+        for room in (keys, 8, 40000):
+            if room < keys:
+                continue
+            outs.append(torch.full((keys, nq * d), float("nan"), device=DEV))
+            ops.attention_rows(q, nq * d, k, v, table, slot, pos, outs[-1], nq, nkv, d, 64, 0, room, d ** -0.5)
+        assert all(torch.equal(o, outs[-1]) for o in outs)
+        s = torch.einsum("ihd,hjd->hij", q.double().view(keys, nq, d), k[0, :, :keys].double().repeat_interleave(nq // nkv, 0)) * d ** -0.5
+        s = s.masked_fill(torch.ones(keys, keys, device=DEV).triu(1).bool(), -math.inf)
+        want = torch.einsum("hij,hjd->ihd", torch.softmax(s, -1), v[0, :, :keys].double().repeat_interleave(nq // nkv, 0)).flatten(1)
+        assert float((outs[0].double() - want).abs().max()) <= 2e-6 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("taps", [1, 2, 3, 4, 5])
 @pytest.mark.parametrize("D, V, channel", [(128, 128, False), (20, 40, False), (160, 72, False), (48, 256, True)])
 def test_delta_prepare_against_float64(taps, D, V, channel):

@@ -72,6 +72,13 @@ def test_the_delta_rules_preparation_takes_runs_of_rows_where_there_are_many(row
     assert bool(library().citlali_delta_prepare_in_runs(rows, H, KH, D, V, taps, channel)) == runs
 
 
+@pytest.mark.parametrize("nq, nkv, d, keys, heads", [
+    (8, 8, 128, 1, 0), (8, 8, 128, 7, 0), (8, 8, 128, 8, 1), (6, 2, 64, 7, 0), (6, 2, 64, 8, 1), (8, 2, 128, 1, 4), (16, 8, 128, 1, 2), (12, 1, 128, 1, 4),
+    (8, 2, 128, 2867, 4), (8, 2, 128, 2868, 0), (16, 8, 128, 4778, 2), (16, 8, 128, 4779, 0), (8, 8, 128, 7168, 1), (8, 8, 128, 7169, 0), (8, 2, 257, 100, 0)])
+def test_heads_that_32_bit_attention_takes_together(nq, nkv, d, keys, heads):
+    assert library().citlali_attention_rows_heads(nq, nkv, d, keys) == heads
+
+
 F32, BF16 = 0, 1
 
 
@@ -85,4 +92,3 @@ def test_epilogues_that_are_none_are_refused_before_any_launch(entry, mode, y_dt
     args = [4096, 4096, 4096, y_dtype, 600, 64, 64, mode, bias, None]
     args += [148, None] if entry == "citlali_gemm_tc_act" else [None]
     assert getattr(lib, entry)(*args) == code
-    assert (b"no form of the epilogue" if code == -2 else b"16-byte boundary") in lib.citlali_last_error()

@@ -706,12 +706,43 @@ def delta_rule(prep, state, seq_start, seq_slot, sequences, H, KH, D, V, out, pa
                                     _i(1 if pairs else 0), _i(mode), _stream()), "delta_rule")
 
 
-def delta_runs_in_chunks(batch, D, V, width) -> bool:
-    """Whether a step of the recurrence (one decay a head) runs 32 tokens at a time (:func:`delta_chunks`) or walks: from 48 rows a
-    sequence on, for sizes the chunks' 16-byte pieces take.  32 heads of 128 x 128, walk against chunks in us: one sequence of 24 / 48 /
-    256 / 2,048 rows 20 / 39 / 184 / 1,420 against 19 / 23 / 52 / 318; sixteen of 32 / 33 / 48 / 256 rows 136 / 140 / 196 / 967 against
-    108 / 172 / 172 / 588 (a chunk that begins is paid for whole)."""
-    return (batch.rows >= 48 * batch.sequences and batch.sequences <= 65535 and D <= 128 and D % 4 == 0 and V % 4 == 0 and width % 4 == 0
+def delta_rule_times(n_new, H, D, V, sms):
+    """About how long the recurrence (one decay a head) over sequences of ``n_new`` rows takes, in us: as a walk of two tokens a step, and
+    32 tokens at a time (:func:`delta_chunks`).  Either is the longest sequence's chain or the work spread over the SMs, whichever is
+    longer, and some of the other.  A walk's work follows the sizes of a head; a chunk's coefficients are made once a head, its blocks
+    have 16 or 32 columns of the values and room for keys of 128, and a chunk that begins is paid for whole.
+
+    Fitted to 1,182 steps: 1 to 300 sequences, equal and unequal, 2 to 32 heads of 16 x 16 to 128 x 128.  Choosing by them with 8 % to spare
+    (:func:`delta_chunks_pay`) is 0.4 % slower on average than the quicker form, and slower than the walk by more than 3 % once (5 %).
+    Walk / chunks measured: 16 heads of 128 x 128, one sequence of 33 / 48 / 256 / 2,048 rows 18 / 17, 25 / 17, 107 / 40, 812 / 233, 64 of
+    48 / 64 390 / 387, 509 / 389, 47 of one row beside one of 3,000 1,690 / 493; of 96 x 96, 64 of 48 / 64 241 / 293, 314 / 296; 4 heads of
+    64 x 64, 16 of 48 / 64 / 96 rows 21 / 23, 26 / 23, 38 / 29, 64 of 48 / 128 / 512 40 / 63, 96 / 104, 365 / 359; of 16 x 16, 64 of
+    48 / 512 18 / 41, 159 / 201."""
+    rows, longest, chunks = sum(n_new), max(n_new), sum((n + 31) // 32 for n in n_new)
+    chain = (0.30 if D <= 32 else 0.34 if D <= 64 else 0.395) * longest
+    work = (28e-6 if D <= 32 else 38e-6 if D <= 64 else 48e-6 if D <= 96 else 59e-6) * rows * H * ((V + 7) // 8 * 8)
+    walk = 4.0 + max(chain, work) + 0.5 * min(chain, work)
+    units = len(n_new) * H
+    if units * ((V + 31) // 32) >= sms * 3 // 4:                           # as citlali_delta_chunks picks a block's columns
+        chain, work = 5.0 * ((longest + 31) // 32), 2.0 + 5.4 * ((V + 31) // 32)
+    else:
+        blocks = (V + 15) // 16
+        chain, work = 3.7 * ((longest + 31) // 32) * (2 if units * blocks > sms else 1), 2.0 + 3.7 * blocks
+    work *= chunks * H / sms
+    return walk, 10.5 + max(chain, work) + 0.2 * min(chain, work)
+
+
+def delta_chunks_pay(n_new, H, D, V, width, sms) -> bool:
+    """Whether 32 tokens at a time is quicker, for sizes that the chunks' 16-byte pieces take."""
+    if len(n_new) > 65535 or D > 128 or D % 4 != 0 or V % 4 != 0 or width % 4 != 0:
+        return False
+    walk, chunks = delta_rule_times(n_new, H, D, V, sms)
+    return 1.08 * chunks <= walk
+
+
+def delta_runs_in_chunks(batch, H, D, V, width, device) -> bool:
+    """Whether a step of the recurrence runs in chunks (:func:`delta_chunks`)."""
+    return (batch.max_new > 1 and delta_chunks_pay(batch.n_new, H, D, V, width, sm_count(device))
             and not torch.cuda.is_current_stream_capturing())
 
 

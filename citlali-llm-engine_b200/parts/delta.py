@@ -157,7 +157,8 @@ class GatedDeltaMixer:
             return self._finish(y, residual, overwrite)
         o = torch.empty((rows, hv), dtype=torch.float32, device=proj.device)
         # bfloat16 steps take a sequence's rows 32 or two at a time; the 32-bit path keeps one order of operations for every cut
-        if self.dtype == torch.bfloat16 and not self.channel_decay and ops.delta_runs_in_chunks(batch, self.D, self.V, prep.shape[1]):
+        if (self.dtype == torch.bfloat16 and not self.channel_decay
+                and ops.delta_runs_in_chunks(batch, self.H, self.D, self.V, prep.shape[1], proj.device)):
             ops.delta_chunks(prep, state, batch.seq_start, batch.seq_slot, batch.sequences, batch.max_new, self.H, self.KH, self.D,
                              self.V, o)
         else:

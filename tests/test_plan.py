@@ -79,6 +79,25 @@ def test_heads_that_32_bit_attention_takes_together(nq, nkv, d, keys, heads):
     assert library().citlali_attention_rows_heads(nq, nkv, d, keys) == heads
 
 
+@pytest.mark.parametrize("lengths, H, D, V, chunks", [
+    # the longest sequence's chain
+    ([1], 16, 128, 128, False), ([24], 32, 128, 128, False), ([33], 16, 128, 128, False), ([48], 16, 128, 128, True), ([65], 16, 128, 128, True),
+    ([2048], 2, 16, 4, True), ([56], 4, 16, 16, True), ([64] * 16, 2, 64, 64, True),
+    # the work, where there is more of it than SMs
+    ([33] * 16, 32, 128, 128, False), ([64] * 64, 16, 128, 128, True), ([65] * 64, 16, 128, 128, False), ([80] * 64, 16, 128, 128, True),
+    ([48] * 64, 16, 96, 96, False), ([256] * 64, 16, 96, 96, True), ([48] * 64, 16, 128, 32, False), ([64] * 300, 16, 128, 64, True),
+    # smaller heads: a chunk's blocks are full-sized all the same
+    ([64] * 64, 4, 64, 64, False), ([128] * 64, 4, 64, 64, False), ([512] * 300, 4, 16, 16, False), ([96] * 16, 4, 64, 64, True),
+    ([128] * 64, 16, 100, 36, False),
+    # unequal lengths: neither the mean nor the longest alone
+    ([540, 155, 300, 420, 200], 16, 128, 128, True), ([1] * 47 + [3000], 32, 128, 128, True), ([1] * 47 + [800], 16, 128, 128, True),
+    ([1] * 300 + [64], 16, 128, 128, False)])
+def test_the_delta_rule_runs_in_chunks_where_that_is_quicker(lengths, H, D, V, chunks):
+    assert ops.delta_chunks_pay(lengths, H, D, V, 4 * H, 148) == chunks
+    for no_pieces in ((D + 2, V, 4 * H), (D, V + 2, 4 * H), (D, V, 4 * H + 2), (132, V, 4 * H)):
+        assert not ops.delta_chunks_pay([2048], H, *no_pieces, 148)
+
+
 F32, BF16 = 0, 1
 
 

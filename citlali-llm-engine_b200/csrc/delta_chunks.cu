@@ -56,26 +56,43 @@ delta_chunk_coefficients_kernel(const float* __restrict__ prep, int prep_stride,
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    {   // 4 x 4 outputs a thread: threads 0-63 K K^T, 64-127 Q K^T; rows and columns eight apart
+    {   // 4 x 4 outputs a thread: threads 0-63 K K^T, 64-127 Q K^T; rows and columns eight apart.  An output is a sum of sums of 16
+        // products.  Off float64, one chain of 128 / this / the walk's sums, in 1e-7: random keys 2.2 / 1.3 / 1.2, decays near zero
+        // 2.1 / 0.9 / 0.9, keys that lean one way 3.3 / 3.2 / 3.1, one key over and over, now and then turned round, 5.9 / 4.6 / 2.6.
+        // 32 heads of 128 x 128: 64 rows 22.7 -> 23.7 us in both kernels, 2,048 rows 322 as before.
         const int a0 = (tid >> 6) * kChunk + ((tid >> 3) & 7), b0 = tid & 7;
         float acc[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-#pragma unroll 4
-        for (int k = 0; k < kHead; k += 4) {
-            float4 a[4], b[4];
+#pragma unroll 1
+        for (int k0 = 0; k0 < D; k0 += 32) {                  // (zeros behind D)
+            float part[4][4][2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i] = *reinterpret_cast<const float4*>(&kq[a0 + 8 * i][k]);
-                b[i] = *reinterpret_cast<const float4*>(&kq[b0 + 8 * i][k]);
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) part[i][j][0] = part[i][j][1] = 0.0f;
+#pragma unroll
+            for (int k = k0; k < k0 + 32; k += 4) {
+                float4 a[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    a[i] = *reinterpret_cast<const float4*>(&kq[a0 + 8 * i][k]);
+                    b[i] = *reinterpret_cast<const float4*>(&kq[b0 + 8 * i][k]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        part[i][j][0] = fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, part[i][j][0]));
+                        part[i][j][1] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, part[i][j][1]));
+                    }
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, acc[i][j]))));
+                for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j][0] + part[i][j][1];
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)

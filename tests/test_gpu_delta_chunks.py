@@ -71,6 +71,36 @@ def test_chunks_against_float64_and_the_walk(D, V, H, KH, lengths, decays):
         assert a <= 2e-6 and a <= 2.0 * b + 1e-7, off
 
 
+@pytest.mark.parametrize("kind", ["random", "leaning", "repeated", "silu", "fast"])
+def test_chunks_are_as_near_float64_as_the_walk(kind):
+    """Means over four seeds of 640 rows; the sums' orders differ, so the two distances do by some tenths."""
+    H, KH, D, V, T = 4, 2, 128, 128, 640
+    C, off = 2 * KH * D + H * V, {"chunks": 0.0, "walk": 0.0}
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    for seed in range(4):
+        g = torch.Generator().manual_seed(seed)
+        keys, beta, decay = torch.randn(T, KH, D, generator=g), torch.rand(T, H, generator=g), torch.rand(T, H, generator=g)
+        if kind == "repeated":
+            keys, beta = keys[:1].expand(T, -1, -1), torch.ones(T, H)
+        keys = {"leaning": keys + 0.3, "silu": torch.nn.functional.silu(keys)}.get(kind, keys)
+        decay = {"random": decay ** 0.1, "silu": 1 - 1e-3 * decay, "fast": 0.1 * decay}.get(kind, torch.ones(T, H))
+        prep = torch.zeros(T, C + 2 * H)
+        prep[:, :KH * D] = torch.nn.functional.normalize(torch.randn(T, KH, D, generator=g), dim=-1).view(T, -1) * D ** -0.5
+        prep[:, KH * D:2 * KH * D] = torch.nn.functional.normalize(keys, dim=-1).reshape(T, -1)
+        prep[:, 2 * KH * D:C] = torch.randn(T, H * V, generator=g)
+        prep[:, C:C + H], prep[:, C + H:] = beta, decay
+        want = recurrence(prep, [T], H, KH, D, V, torch.zeros(1, H, D, V, dtype=torch.float64))
+        for name in off:
+            state, out = torch.zeros(1, H * D * V, device=DEV), torch.empty(T, H * V, device=DEV)
+            if name == "chunks":
+                ops.delta_chunks(prep.to(DEV), state, i32([0, T]), i32([0]), 1, T, H, KH, D, V, out)
+            else:
+                ops.delta_rule(prep.to(DEV), state, i32([0, T]), i32([0]), 1, H, KH, D, V, out, pairs=True)
+            off[name] += float((out.cpu().double() - want).norm() / want.norm()) / 4
+    print(f"[{kind}] chunks {off['chunks']:.2e}, walk {off['walk']:.2e} off float64")
+    assert off["chunks"] <= 1.3 * off["walk"], off
+
+
 @pytest.mark.parametrize("heads", [4, 64])                    # columns of the values a block: 16, 32
 @pytest.mark.parametrize("part", ["query", "key", "value", "strength", "decay"])
 @pytest.mark.parametrize("bad", [math.nan, math.inf])

@@ -98,6 +98,19 @@ def test_the_delta_rule_runs_in_chunks_where_that_is_quicker(lengths, H, D, V, c
         assert not ops.delta_chunks_pay([2048], H, *no_pieces, 148)
 
 
+@pytest.mark.parametrize("units, tiles, runs", [(1, 1, 1), (1, 63, 32), (8, 33, 17), (8, 32, 32), (24, 8, 8), (16, 12, 12), (32, 5, 5), (64, 3, 3), (16, 63, 16),
+                                                (17, 32, 16), (126, 63, 2), (300, 63, 1)])
+def test_runs_of_the_latent_walk(units, tiles, runs):
+    assert ops.latent_runs(units, tiles, 148) == runs
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 5, 12, 33, 64, 100])
+def test_every_run_of_the_latent_walk_has_a_tile(tiles):
+    for units in range(1, 400):
+        runs = ops.latent_runs(units, tiles, 148)
+        assert 1 <= runs <= 32 and (runs - 1) * -(-tiles // runs) < tiles
+
+
 F32, BF16 = 0, 1
 
 

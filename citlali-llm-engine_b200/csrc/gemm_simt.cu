@@ -179,9 +179,12 @@ gemm_simt_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, 
 
 // The same product for float32 operands and few rows (decoding, short ends of prompts): the same chains again.  One output a thread, 8 rows
 // x 16 columns a block, so that a matrix of 1,024 rows reaches 64 blocks and every k costs a thread half of a 16-byte read; four tiles of
-// 64 k are on their way.  Bound by the chain (four clocks a k) and, for large matrices, by the bytes of w.  kPieces: K a multiple of four
-// and operands on 16-byte boundaries, copied in 16-byte pieces, else element by element.
-// 8 rows, K 1,024, N 1,024 / 5,632 / 32,768: 10 / 23 / 56 us (the 64 x 64 tiles above: 105 / 106 / 361).
+// 64 k are on their way.  kPieces: K a multiple of four and operands on 16-byte boundaries, copied in 16-byte pieces, else element by
+// element.  Few blocks wait for their rounds of copies and the chain (four clocks a k); many are bound by shared memory, three
+// wavefronts of reads for every four multiply-adds of a warp (by count 28 us at N 32,768, beside 20 for the bytes of w).  Every eight rows of x
+// read w again.
+// 8 rows, K 1,024, N 1,024 / 5,632 / 32,768: 7 / 16 / 56 us (the first kernel here: 103 / 104 / 342), 16 rows 7 / 29 / 105, 31 rows
+// 11 / 39 / 203.
 template <bool kPieces, bool kAccumulate>
 __global__ void __launch_bounds__(128)
 gemm_simt_few_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K) {
@@ -243,8 +246,10 @@ static int launch_few(const float* x, const float* w, float* y, int M, int N, in
     return CITLALI_LAUNCH_CHECK();
 }
 
-// From kWideRows rows on (below, a 64-row tile is mostly empty: the kernel above).  Tiles of 64 x 128 where they
-// give every SM at least two, else 64 x 64, so that products of few columns still reach every SM.
+// From kWideRows rows on.  A tile of 64 rows takes the same time however few of them are there: K 1,024, N 1,024 / 5,632 / 32,768, 31
+// rows 41 / 41 / 122 us and 64 rows 43 / 43 / 127, where the kernel above takes 11 / 39 / 203 and 21 / 74 / 398.  So the line lies where
+// the two meet for matrices of some 5,000 rows; narrow ones would keep the kernel above to 64 rows and more, the widest to 16.
+// Tiles of 64 x 128 where they give every SM at least two, else 64 x 64, so that products of few columns still reach every SM.
 constexpr int kWideRows = 32;
 
 static int launch_wide(const float* x, const float* w, float* y, int M, int N, int K, int accumulate, cudaStream_t stream) {

@@ -318,7 +318,9 @@ heads_product_mma_kernel(const TX* __restrict__ x, size_t x_row, int x_head, con
 // rows and 16 columns of a head, its eight warps share k between them, every operand is read from memory straight into an MMA's
 // registers (all of a warp's reads at once), and the warps' sums meet in shared memory, added in warp order.  Matrices whose k lies
 // contiguously, K a multiple of 16, x in float32.  Bound by the latency of one round of reads.
-// 8 rows, 16 heads, K x N = 128 x 512 and 512 x 128: 6.2 and 5.0 us, above 16 and 32 us.
+// K x N = 128 x 512 and 512 x 128, back to back, 16 heads: 8 rows 3.7 and 3.0 us (above 8.2 and 18.6), 16 rows 3.7 and 3.4 (9.2 and
+// 22.8).  To kFewRows rows, one tile of them: more read the matrices again (32 rows 6.3 and 4.7 against 11.4 and 25.5, 63 rows of 32 heads
+// 20.2 and 12.0 against 16.7 and 31.8), and steps of more rows keep the sums that they have above.
 constexpr int kFewRows = 16;
 
 template <typename TY>

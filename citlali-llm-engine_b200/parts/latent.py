@@ -111,7 +111,8 @@ class LatentAttention:
         self.q_weight = bind_float32(weights, nm["dq_norm"], (self.RQ,), ctx)
         self.c_weight = bind_float32(weights, nm["dkv_norm"], (self.R,), ctx) if self.kv_projection else None
         self.sink = bind_float32(weights, nm["sink"], (self.H,), ctx) if nm["sink"] is not None else None
-        # one buffer [W_uk of every head; W_uv of every head]: as a whole it makes keys and values of cached vectors
+        # one buffer [W_uk of every head; W_uv of every head]: as a whole it makes keys and values of cached vectors (W_uk is then
+        # held in both layouts, 4 MB more a layer of 32 heads with latents of 512)
         both = torch.empty((self.H * (self.D + self.V), self.R), dtype=ctx.dtype, device=ctx.device)
         uk, self.uv = both[:self.H * self.D], both[self.H * self.D:]
         self.kv_up = both if self._writes_keys_out(ctx.dtype) else None

@@ -71,6 +71,15 @@ def test_chunks_against_float64_and_the_walk(D, V, H, KH, lengths, decays):
         assert a <= 2e-6 and a <= 2.0 * b + 1e-7, off
 
 
+@pytest.mark.parametrize("D, V, H, KH, lengths, decays", [
+    (128, 128, 16, 8, [33, 5, 70, 150, 64], "mixed"), (96, 36, 16, 8, [40, 129, 32, 5, 1], "mixed"), (20, 40, 16, 16, [31, 64, 1, 200], "slow"),
+    (64, 4, 2, 1, [1, 2, 33, 3, 7, 64] * 50, "mixed")], ids=["five", "columns left over", "small", "300"])
+def test_blocks_of_32_columns_and_many_sequences(D, V, H, KH, lengths, decays):
+    """Above: blocks of 16 columns mostly.  Several sequences, the longest first, and so many that they are not sorted."""
+    assert len(lengths) * H * ((V + 31) // 32) >= torch.cuda.get_device_properties(0).multi_processor_count * 3 // 4
+    test_chunks_against_float64_and_the_walk(D, V, H, KH, lengths, decays)
+
+
 @pytest.mark.parametrize("kind", ["random", "leaning", "repeated", "silu", "fast"])
 def test_chunks_are_as_near_float64_as_the_walk(kind):
     """Means over four seeds of 640 rows; the sums' orders differ, so the two distances do by some tenths."""

@@ -7,6 +7,7 @@ the rows goes to the device in one copy from pinned memory.
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 from typing import List, Sequence
 
@@ -25,14 +26,11 @@ class StepEntry:
 
 
 def _as_ids(tokens: list) -> np.ndarray:
-    """The ids as torch reads them.  numpy is quicker and reads whole numbers alike, but takes strings of digits for numbers too."""
+    """The ids as torch reads them; whole numbers by the quick way, which takes nothing else."""
     try:
-        ids = np.array(tokens)
-    except (TypeError, ValueError, RuntimeError):     # what numpy does not read (elements of a tensor on the device)
-        ids = None
-    if ids is None or ids.dtype.kind not in "ib":
+        return np.frombuffer(array("q", tokens), dtype=np.int64)
+    except (TypeError, ValueError, OverflowError):
         return torch.as_tensor(tokens, dtype=torch.int64).numpy()
-    return ids.astype(np.int64, copy=False)
 
 
 def pack_step(entries: List[StepEntry], past: List[int], vocab_size: int, device) -> StepBatch:

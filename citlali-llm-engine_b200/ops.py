@@ -87,11 +87,7 @@ def _need_cuda(*tensors):
 
 # plain numbers of the kind the C argument wants (an integer argument takes no float)
 _i = _sz = operator.index
-
-
-def _f(number):
-    """A float argument as it is: its declared type takes numbers alone, where ``float`` would read a text."""
-    return number
+_f = operator.pos          # (the number as it is, no text; its declared type does the rest)
 
 
 def embed_rows(table: torch.Tensor, tokens: torch.Tensor, out: torch.Tensor, error_flag: torch.Tensor,
@@ -742,8 +738,13 @@ def delta_chunks_pay(n_new, H, D, V, width, sms) -> bool:
 
 def delta_runs_in_chunks(batch, H, D, V, width, device) -> bool:
     """Whether a step of the recurrence runs in chunks (:func:`delta_chunks`)."""
-    return (batch.max_new > 1 and delta_chunks_pay(batch.n_new, H, D, V, width, sm_count(device))
-            and not torch.cuda.is_current_stream_capturing())
+    if batch.max_new == 1 or torch.cuda.is_current_stream_capturing():
+        return False
+    sizes = (H, D, V, width)
+    pays = batch.delta_in_chunks.get(sizes)
+    if pays is None:
+        pays = batch.delta_in_chunks[sizes] = delta_chunks_pay(batch.n_new, H, D, V, width, sm_count(device))
+    return pays
 
 
 def delta_chunks(prep, state, seq_start, seq_slot, sequences, max_new, H, KH, D, V, out):

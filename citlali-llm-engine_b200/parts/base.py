@@ -30,7 +30,7 @@ Interfaces (all tensors are on the model's device; ``x`` is the float32 residual
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import Dict, List, Optional
 
 import torch
@@ -128,6 +128,8 @@ class StepBatch:
     norm_carry_in: Optional["NormedRows"] = None
     # the two pairs of buffers such rows take turns in, for the whole step (parts/block.py)
     norm_buffers: Optional[list] = None
+    # by a delta rule's sizes: whether it runs in chunks in this step (``ops.delta_runs_in_chunks``; its layers ask one by one)
+    delta_in_chunks: dict = field(default_factory=dict)
     # A block on several residual streams may leave its last write-back undone, as (y, mix, out), for the next such
     # block to do together with its first read (one pass over the streams instead of two); the model does what is left
     # after the last layer.

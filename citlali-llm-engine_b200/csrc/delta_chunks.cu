@@ -15,9 +15,9 @@
 //   delta_chunk_scan           one block a (sequence, head, VS columns of the values): the chunks in order, S in registers and in shared
 //                              memory.  [K; Q] S is the bulk: 256 threads, 8 x 4 outputs each over a slice of the 128 k, the slices'
 //                              sums added through shared memory; the next chunk's rows arrive meanwhile.  VS is 32, or 16 where that
-//                              leaves SMs idle.  It is bound by shared memory and the FMA units in turn: 6,000 wavefronts and 3,600
-//                              FMA issues a scheduler in a chunk's 9,000 clocks.
-// One sequence of 2,048 tokens, 32 heads over 16 key heads, 128 x 128: 322 us for both kernels (31 of them the coefficients); the walk of
+//                              leaves SMs idle.  Two warps a scheduler and five barriers a chunk: latency, beside 4,100 wavefronts of
+//                              shared memory and 3,600 FMA issues a scheduler in a chunk's 8,800 clocks.
+// One sequence of 2,048 tokens, 32 heads over 16 key heads, 128 x 128: 316 us for both kernels (31 of them the coefficients); the walk of
 // two tokens a step 948.
 #include "api.h"
 #include "common.cuh"
@@ -27,6 +27,7 @@ namespace citlali {
 constexpr int kChunk = 32, kHead = 128;                      // tokens a chunk; key size (smaller ones are filled up with zeros)
 constexpr int kCoef = 2 * kChunk * kChunk + 2 * kChunk;      // floats a (chunk, head): T | M | G | e
 constexpr int kRow = kHead + 4;                              // a key's stride in shared memory: rows side by side in different banks
+constexpr int kMatRow = kChunk + 4;                          // a row of T's and M's in shared memory, for the same reason
 static_assert(4 * kChunk * (kChunk + 4) <= 2 * kChunk * kRow, "four warps' A lie over the keys and queries");
 
 // The first chunk of a sequence among all chunks' places: sequences of n tokens have at most n / 32 + 1 (rounded down) of them.
@@ -146,7 +147,7 @@ delta_chunk_coefficients_kernel(const float* __restrict__ prep, int prep_stride,
 template <int VS>
 struct ScanShared {
     float kq[2][2 * kChunk][kRow];        // the chunk's keys and queries, and the next one's
-    float coef[2][kCoef];
+    float coef[2][2 * kChunk * kMatRow + 2 * kChunk];           // T | M, rows kMatRow apart | G | e
     float v[2][kChunk][VS];
     float s[kHead][VS];
     float part[128 / VS][2 * kChunk][VS]; // [K; Q] S over a slice of k
@@ -180,7 +181,7 @@ __device__ __forceinline__ void store_floats(float* p, const float (&f)[N]) {
 template <int N, int VS>
 __device__ __forceinline__ void add_rows_up_to(float (&sum)[N], const float* W, const float (&X)[kChunk][VS], int row, int col) {
     auto tile = [&](int j, bool ask) {
-        const Floats<4> w = load_floats<4>(W + row * kChunk + j);
+        const Floats<4> w = load_floats<4>(W + row * kMatRow + j);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const Floats<N> x = load_floats<N>(&X[j + e][col]);
@@ -243,14 +244,25 @@ delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const f
                 const bool there = token < n && v0 + c < V;
                 cp_async16_or_zero(&sm.v[buf][token][c], there ? prep + (size_t)(r0 + token) * prep_stride + 2 * KH * D + h * V + v0 + c : prep, there);
             }
-            for (int i = tid; i < kCoef / 4; i += 256)
-                cp_async16_or_zero(&sm.coef[buf][i * 4], coef_h + (size_t)ch * H * kCoef + i * 4, true);
+            for (int i = tid; i < kCoef / 4; i += 256) {
+                const int row = i / (kChunk / 4), at = row < 2 * kChunk ? row * kMatRow + (i % (kChunk / 4)) * 4 : i * 4 + 2 * kChunk * (kMatRow - kChunk);
+                cp_async16_or_zero(&sm.coef[buf][at], coef_h + (size_t)ch * H * kCoef + i * 4, true);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     fetch(0);
+    // Where a warp's lanes stand in a product.  Of a 16-byte read of shared memory two neighbours (or two lanes two apart) that read the
+    // same place are served together, lanes further apart are not: columns in the lane's low bits and rows above them cost the columns'
+    // operand four wavefronts a read, columns in every other bit and rows in those between cost either operand two.  (The scan's reads
+    // 4,100 wavefronts a chunk instead of 5,900; with the coefficients, columns in the low bits -> every other bit: one sequence of
+    // 2,048 tokens, 32 heads 323 -> 316 us, 8 heads (16 columns a block) 232 -> 214, five of 155 to 540 tokens, 16 heads 149 -> 145.)
+    const int lane = tid & 31, warp = tid >> 5;
+    const int even = (lane & 1) | ((lane >> 1) & 2) | ((lane >> 2) & 4), odd = ((lane >> 1) & 1) | ((lane >> 2) & 2);    // bits 0 2 4; 1 3
+    const int lane_c = CG == 8 ? even : even & 3, lane_r = CG == 8 ? odd : odd | ((lane >> 2) & 4);
+    constexpr int LR = 32 / CG;                // rows a warp has beside its CG columns
     // this thread's part of S: rows sk .. sk + RS - 1, columns 4 sc .. 4 sc + 3
-    const int sc = tid % CG, sk = (tid / CG) * RS;
+    const int sc = lane_c, sk = (warp * LR + lane_r) * RS;
     float* S_g = state + (size_t)seq_slot[seq] * state_stride + (size_t)h * D * V + v0 + sc * 4;
     float S[RS][4];
 #pragma unroll
@@ -261,10 +273,10 @@ delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const f
             sm.s[sk + i][sc * 4 + e] = S[i][e];
         }
     // [K; Q] S: slice `slice` of k, columns 4 xc .. 4 xc + 3, rows xr + 8 i (i < 4: keys, else queries)
-    const int slice = tid / (8 * CG), xc = tid % CG, xr = (tid / CG) & 7;
+    const int slice = warp * LR / 8, xc = lane_c, xr = (warp * LR + lane_r) & 7;
     // the 32 x VS matrices: row `ur`, UC columns from `uc` (a warp four rows)
     constexpr int UC = VS / 8;
-    const int ur = tid >> 3, uc = (tid & 7) * UC;
+    const int ur = warp * 4 + odd, uc = even * UC;
     for (int ch = 0; ch < chunks; ++ch) {
         const int buf = ch & 1;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -294,8 +306,8 @@ delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const f
         }
         __syncthreads();
         const float* T = sm.coef[buf];
-        const float* M = T + kChunk * kChunk;
-        const float* G = M + kChunk * kChunk;
+        const float* M = T + kChunk * kMatRow;
+        const float* G = M + kChunk * kMatRow;
         const float* E = G + kChunk;
         float y[UC], r[UC], u[UC], eu[UC];
 #pragma unroll

@@ -68,12 +68,11 @@ gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __restr
 
 // The same product for float32 operands and many rows: the same chain an element (k ascending, the last 16 k filled up with
 // zeros), so the same bits as the kernel above.
-// What bounds it: the FMA units.  A thread owns 8 x RN outputs, so that a k costs it four (three) 16-byte reads of shared memory
-// for 64 (32) multiply-adds, two of them an instruction (fma.rn.f32x2 rounds each half like fmaf); both operands lie transposed
+// What bounds it: the FMA units.  A thread owns 8 x 8 outputs, so that a k costs it four 16-byte reads of shared memory
+// for 64 multiply-adds, two of them an instruction (fma.rn.f32x2 rounds each half like fmaf); both operands lie transposed
 // [k][row] in shared memory, put there element by element by asynchronous copies (any alignment, any K) three tiles deep.
-// TN = 128 for matrices with tiles enough for every SM, TN = 64 below that (see launch_wide).
-// A four-layer model of width 1,024 over 682 rows with logits of each (17 products, 54 G multiply-adds): 6.9 ms in the kernel
-// above, 3.2 ms here (of 1.5 that the FMA units need).
+// For matrices with tiles enough for every SM twice; fewer run the kernel behind this one (see launch_wide).  682 rows, K 1,024: N 5,632
+// 212 us, N 32,768 977 (18.6 and 23.4 T multiply-adds a second of 37).
 __device__ __forceinline__ void cp_async4_or_zero(uint32_t dst, const float* src, bool there) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(there ? 4 : 0) : "memory");
 }
@@ -88,10 +87,10 @@ __device__ __forceinline__ unsigned long long both(float v) {
     return d;
 }
 
-template <int TN, bool kAccumulate>
+template <bool kAccumulate>
 __global__ void __launch_bounds__(128, 3)
 gemm_simt_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K) {
-    constexpr int TM = 64, STAGES = 3, TX = 16, RN = TN / TX, LX = TM + 4, LW = TN + 4;
+    constexpr int TM = 64, TN = 128, STAGES = 3, TX = 16, RN = TN / TX, LX = TM + 4, LW = TN + 4;
     __shared__ __align__(16) float xs[STAGES][kTileK][LX];
     __shared__ __align__(16) float ws[STAGES][kTileK][LW];
     dependents_may_launch();
@@ -177,6 +176,111 @@ gemm_simt_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, 
     }
 }
 
+// The same product again, the same chains, for matrices of few tiles: 64 rows x 16 RN columns a block of
+// 2 x 2 warps, RN chosen so that the tiles go round the SMs as evenly as they can (narrow_columns).
+// What bounds it: a block or two an SM, a warp or two a scheduler, so the chain of reads and multiply-adds of a thread.  Rows of both
+// operands lie in shared memory as they do in memory, 32 k of each, copied in 16-byte pieces (kPieces; else element by element) three
+// tiles deep; a thread's 16-byte reads are four k of a row, so a copy costs a quarter of the instructions, and 8 RN multiply-adds a k
+// need no moves.  Lanes are placed as in the delta rule's scan: two that read the same place are neighbours or two apart, and a read
+// costs two wavefronts.
+// 682 rows one product after another, 64 x 64 tiles of the kernel above -> here: N 1,024, K 1,024 / 2,816 (143 tiles of 64 x 80 instead of
+// 176) 94 / 254 -> 43 / 111 us; N 1,536, K 1,024 97 -> 62; 200 rows, N 1,024 / 1,536 47 / 71 -> 22 / 29; 33 rows, N 1,024 41 -> 21.
+template <int RN, bool kPieces, bool kAccumulate>
+__global__ void __launch_bounds__(128, 3)
+gemm_simt_narrow_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K) {
+    constexpr int RM = 8, TM = 64, TN = 16 * RN, TK = 32, LD = TK + 4, STAGES = 3;
+    constexpr int kCopies = (TM + TN) / 16;                 // pieces a thread and tile: 16 rows of 8 pieces a pass
+    extern __shared__ __align__(16) float narrow_tiles[];   // [STAGES][rows of x, rows of w][LD]
+    dependents_may_launch();
+    wait_for_predecessor();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = (lane & 1) | ((lane >> 1) & 2) | ((lane >> 2) & 4), ty = ((lane >> 1) & 1) | ((lane >> 2) & 2);    // lane bits 0 2 4; 1 3
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    const int count = (K + TK - 1) / TK;
+    const int lk = (tid & 7) * 4, lr = tid >> 3;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(narrow_tiles) + (uint32_t)((lr * LD + lk) * 4);
+    const float* src[kCopies];
+    bool in[kCopies];
+#pragma unroll
+    for (int i = 0; i < kCopies; ++i) {
+        const int r = 16 * i + lr, row = r < TM ? m0 + r : n0 + r - TM;      // (TM a multiple of 16: a pass is all x or all w)
+        in[i] = row < (r < TM ? M : N);
+        src[i] = (r < TM ? x : w) + (in[i] ? (size_t)row * K : 0) + lk;
+    }
+    auto fetch = [&](int tile) {
+        if (tile < count) {
+            const uint32_t dst = base + (uint32_t)((tile % STAGES) * (TM + TN) * LD * 4);
+            const int k = tile * TK;
+#pragma unroll
+            for (int i = 0; i < kCopies; ++i) {
+                if constexpr (kPieces) {
+                    const bool there = in[i] && k + lk < K;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(i * 16 * LD * 4)),
+                                 "l"(there ? src[i] + k : src[i] - lk), "r"(there ? 16 : 0) : "memory");
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const bool there = in[i] && k + lk + e < K;
+                        cp_async4_or_zero(dst + (uint32_t)((i * 16 * LD + e) * 4), there ? src[i] + k + e : src[i] - lk, there);
+                    }
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[RM][RN];
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = 0.0f;
+    for (int s = 0; s < STAGES - 1; ++s) fetch(s);
+    // rows ty + 4 i of this warp's 32, columns tx + 8 j of its 8 RN
+    const int row0 = (warp >> 1) * 32 + ty, col0 = (warp & 1) * 8 * RN + tx;
+    for (int t = 0; t < count; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                          // the tile has landed for every thread; the one before it is no longer read
+        fetch(t + STAGES - 1);
+        const float* xs = narrow_tiles + (t % STAGES) * (TM + TN) * LD + row0 * LD;
+        const float* ws = narrow_tiles + (t % STAGES) * (TM + TN) * LD + (TM + col0) * LD;
+#pragma unroll
+        for (int k = 0; k < TK; k += 4) {
+            float4 a[RM], b[RN];
+#pragma unroll
+            for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * 4 * LD + k);
+#pragma unroll
+            for (int j = 0; j < RN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + j * 8 * LD + k);
+#pragma unroll
+            for (int j = 0; j < RN; ++j)
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+#pragma unroll
+            for (int j = 0; j < RN; ++j)
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+#pragma unroll
+            for (int j = 0; j < RN; ++j)
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+#pragma unroll
+            for (int j = 0; j < RN; ++j)
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+        const int gm = m0 + row0 + 4 * i;
+        if (gm >= M) continue;
+#pragma unroll
+        for (int j = 0; j < RN; ++j) {
+            const int gn = n0 + col0 + 8 * j;
+            if (gn >= N) continue;
+            float* dst = y + (size_t)gm * N + gn;
+            *dst = kAccumulate ? *dst + acc[i][j] : acc[i][j];
+        }
+    }
+}
+
 // The same product for float32 operands and few rows (decoding, short ends of prompts): the same chains again.  One output a thread, 8 rows
 // x 16 columns a block, so that a matrix of 1,024 rows reaches 64 blocks and every k costs a thread half of a 16-byte read; four tiles of
 // 64 k are on their way.  kPieces: K a multiple of four and operands on 16-byte boundaries, copied in 16-byte pieces, else element by
@@ -246,25 +350,63 @@ static int launch_few(const float* x, const float* w, float* y, int M, int N, in
     return CITLALI_LAUNCH_CHECK();
 }
 
-// From kWideRows rows on.  A tile of 64 rows takes the same time however few of them are there: K 1,024, N 1,024 / 5,632 / 32,768, 31
-// rows 41 / 41 / 122 us and 64 rows 43 / 43 / 127, where the kernel above takes 11 / 39 / 203 and 21 / 74 / 398.  So the line lies where
-// the two meet for matrices of some 5,000 rows; narrow ones would keep the kernel above to 64 rows and more, the widest to 16.
-// Tiles of 64 x 128 where they give every SM at least two, else 64 x 64, so that products of few columns still reach every SM.
+// From kWideRows rows on.  A tile of 64 rows takes the same time however few of them are there: K 1,024, N 1,024 / 5,632 / 32,768, 33
+// to 64 rows 21 / 29 / 112 us, where the kernel above takes 11 / 39 / 203 (31 rows) and 21 / 74 / 398 (64).  So the line lies where
+// the two meet for matrices of some 5,000 rows; narrow ones would keep the kernel above to 64 rows, the widest to 16.
+// Tiles of 64 x 128 where they give every SM at least two, else narrower ones.
 constexpr int kWideRows = 32;
+
+// Columns a thread of the narrow kernel: the RN of 2 to 6 that gives an SM the shortest share, tiles times a tile's time (four k: 32 RN
+// issues of multiply-adds a scheduler or 8 (8 + RN) wavefronts of reads, whichever is longer); of equal ones the widest, which reads x
+// less often (682 rows, N 1,536: two tiles of 64 columns an SM 62 us, four of 32 66).
+static int narrow_columns(long rows, int N, int sm_count) {
+    int best = 2;
+    long least = -1;
+    for (int rn = 2; rn <= 6; ++rn) {
+        const long tiles = rows * ((N + 16 * rn - 1) / (16 * rn));
+        const long share = (tiles + sm_count - 1) / sm_count * (4 * rn > 8 + rn ? 4 * rn : 8 + rn);
+        if (least < 0 || share <= least) { least = share; best = rn; }
+    }
+    return best;
+}
+
+template <int RN, bool kPieces>
+static int launch_narrow(const float* x, const float* w, float* y, int M, int N, int K, int accumulate, cudaStream_t stream) {
+    // The blocks begin while the kernel ahead still runs, on whichever SMs have room by then, and stay there: an SM that was idle takes
+    // several of them and works as many times as long.  So a block asks for as much shared memory as leaves an SM no room for more than
+    // its even share of the blocks (682 rows, N 1,024, one after another: K 1,024 86 -> 43 us, K 2,816 229 -> 111).
+    constexpr size_t needed = (size_t)3 * (64 + 16 * RN) * 36 * 4, of_an_sm = 228 * 1024, alone = of_an_sm / 2 + 256;
+    dim3 grid((N + 16 * RN - 1) / (16 * RN), (M + 63) / 64);
+    const long tiles = (long)grid.x * grid.y, sms = device_sm_count();
+    const size_t spread = of_an_sm / (size_t)((tiles + sms - 1) / sms + 1) + 256, smem = spread > needed ? spread : needed;
+    auto kernel = accumulate ? gemm_simt_narrow_kernel<RN, kPieces, true> : gemm_simt_narrow_kernel<RN, kPieces, false>;
+    if (int code = raise_shared_limit(kernel, alone, alone)) return code;
+    launch_kernel(kernel, grid, 128, smem, stream, x, w, y, M, N, K);
+    return CITLALI_LAUNCH_CHECK();
+}
+
+template <bool kPieces>
+static int launch_narrow(int rn, const float* x, const float* w, float* y, int M, int N, int K, int accumulate, cudaStream_t stream) {
+    switch (rn) {
+        case 2: return launch_narrow<2, kPieces>(x, w, y, M, N, K, accumulate, stream);
+        case 3: return launch_narrow<3, kPieces>(x, w, y, M, N, K, accumulate, stream);
+        case 4: return launch_narrow<4, kPieces>(x, w, y, M, N, K, accumulate, stream);
+        case 5: return launch_narrow<5, kPieces>(x, w, y, M, N, K, accumulate, stream);
+        default: return launch_narrow<6, kPieces>(x, w, y, M, N, K, accumulate, stream);
+    }
+}
 
 static int launch_wide(const float* x, const float* w, float* y, int M, int N, int K, int accumulate, cudaStream_t stream) {
     const long rows = (M + 63) / 64;
-    const bool broad = rows * ((N + 127) / 128) >= 2L * device_sm_count();
-    const int tn = broad ? 128 : 64;
-    dim3 grid((N + tn - 1) / tn, (unsigned)rows);
-    if (broad) {
-        if (accumulate) launch_kernel(gemm_simt_wide_kernel<128, true>, grid, 128, 0, stream, x, w, y, M, N, K);
-        else launch_kernel(gemm_simt_wide_kernel<128, false>, grid, 128, 0, stream, x, w, y, M, N, K);
-    } else {
-        if (accumulate) launch_kernel(gemm_simt_wide_kernel<64, true>, grid, 128, 0, stream, x, w, y, M, N, K);
-        else launch_kernel(gemm_simt_wide_kernel<64, false>, grid, 128, 0, stream, x, w, y, M, N, K);
+    if (rows * ((N + 127) / 128) >= 2L * device_sm_count()) {
+        dim3 grid((N + 127) / 128, (unsigned)rows);
+        if (accumulate) launch_kernel(gemm_simt_wide_kernel<true>, grid, 128, 0, stream, x, w, y, M, N, K);
+        else launch_kernel(gemm_simt_wide_kernel<false>, grid, 128, 0, stream, x, w, y, M, N, K);
+        return CITLALI_LAUNCH_CHECK();
     }
-    return CITLALI_LAUNCH_CHECK();
+    const int rn = narrow_columns(rows, N, device_sm_count());
+    const bool pieces = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15u) == 0;
+    return pieces ? launch_narrow<true>(rn, x, w, y, M, N, K, accumulate, stream) : launch_narrow<false>(rn, x, w, y, M, N, K, accumulate, stream);
 }
 
 template <typename TX, typename TW, typename TY>

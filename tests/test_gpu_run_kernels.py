@@ -193,6 +193,26 @@ def test_32_bit_products_give_a_row_the_same_bits_in_steps_of_any_size(N, K, odd
         assert torch.equal(y, want[:rows]) and torch.equal(added, base[:rows] + y)
 
 
+@pytest.mark.parametrize("M, N, K, odd", [(64, 1024, 96, False), (65, 1531, 100, False), (682, 1024, 68, False), (500, 1100, 33, False),
+                                          (130, 2300, 64, True), (273, 2400, 40, False), (1200, 1024, 36, False)])
+def test_narrow_32_bit_products_give_the_bits_of_few_rows(M, N, K, odd):
+    """Every width of the narrow tiles (32 to 96 columns), ragged rows, columns and last tiles of k, in pieces and element by element."""
+    g = torch.Generator().manual_seed(M + N + K)
+    store = torch.zeros(N * K + 1, device=DEV)
+    w = store[1:].view(N, K) if odd else store[:-1].view(N, K)
+    w.copy_(torch.randn(N, K, generator=g))
+    x, base = torch.randn(M, K, generator=g).to(DEV), torch.randn(M, N, generator=g).to(DEV)
+    y, added = torch.full((M, N), float("nan"), device=DEV), base.clone()
+    ops.gemm_simt(x, w, y)
+    ops.gemm_simt(x, w, added, accumulate=True)
+    few = torch.empty(31, N, device=DEV)
+    for r in range(0, M, 31):
+        n = min(31, M - r)
+        ops.gemm_simt(x[r:r + n].contiguous(), w, few[:n])
+        assert torch.equal(y[r:r + n], few[:n])
+    assert torch.equal(added, base + y)
+
+
 _SHARED_MEMORY_LIMITS = """
 import sys
 sys.path.insert(0, {root!r})

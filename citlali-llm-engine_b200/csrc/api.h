@@ -199,6 +199,25 @@ int citlali_gemm_tc_normed(const void* x, const void* w, void* y, int y_dtype, i
                            int mode, int force_splits, int32_t* error_flag, int sm_count,
                            void* emit_rows, float* emit_sumsq, const float* scale_sumsq, int scale_groups,
                            int scale_dim, float scale_eps, cudaStream_t stream);
+// A layer of a dense decoder over at most 128 rows, its six launches from one call (dense_layer.cu): gated feed-forward (gate and up
+// rows in runs of 16), both norms in the products (their gains in the weights; see citlali_gemm_tc_normed), keys and values into pages.
+// qkv [rows, (nq + 2 nkv) head_dim], heads [rows, nq head_dim] and act [rows, inter] are scratch, bfloat16; in_rows / in_sumsq stand for
+// the rows of x (citlali_norm_inputs, or the layer before), out_rows / out_sumsq for the updated ones.  q_gain and k_gain may be null.
+typedef struct {
+    const void *qkv, *o, *gate_up, *down;          // bfloat16
+    const void *q_gain, *k_gain;
+    const float* inv_freq;
+    void *k_pool, *v_pool;                         // bfloat16
+    const int32_t* page_table;
+    int gain_dtype, rotary_dim, page_table_stride, pool_pages, page_size, hidden, inter, nq, nkv, head_dim, window;
+    float head_eps, scale, mixer_eps, ff_eps;
+} CitlaliDenseLayer;
+int citlali_dense_layer_supports(int nq, int nkv, int head_dim, int page_size, int max_new);
+int citlali_dense_layer(const CitlaliDenseLayer* layer, float* x, void* qkv, void* heads, void* act, const void* in_rows,
+                        const float* in_sumsq, void* mid_rows, float* mid_sumsq, void* out_rows, float* out_sumsq,
+                        const int32_t* row_slot, const int32_t* row_pos, const int32_t* seq_start, const int32_t* seq_slot,
+                        const int32_t* seq_past, int rows, int sequences, int max_new, int32_t* error_flag, int sm_count,
+                        cudaStream_t stream);
 // The same with a bias (float32 [N] or null) and an activation on the float32 sums: mode bit 2 gates by gelu_tanh instead of SiLU, bit 3
 // stores bfloat16 max(v, 0)^2.
 int citlali_gemm_tc_act(const void* x, const void* w, void* y, int y_dtype, int M, int N, int K, int mode, const float* bias,

@@ -169,7 +169,8 @@ def build(force: bool = False, verbose: bool = True) -> str:
 
 
 _BASE = "elementwise"                       # holds what every other source calls (error text, launch mode)
-_ALSO = {"gemm_tcgen05": ("gemm_tcgen05_pair",), "attention_decode_no_alloc": ("attention_decode",)}    # who calls whom besides
+_ALSO = {"gemm_tcgen05": ("gemm_tcgen05_pair",), "attention_decode_no_alloc": ("attention_decode",),
+         "dense_layer": ("gemm_tcgen05_pair", "gemm_tcgen05", "attention_generic", "attention_prefill", "attention_prefill_tc")}    # who calls whom besides
 _TYPES = {"int": ctypes.c_int, "float": ctypes.c_float, "size_t": ctypes.c_size_t, "long": ctypes.c_long, "long long": ctypes.c_longlong,
           "cudaStream_t": ctypes.c_void_p, "void": None, "const char*": ctypes.c_char_p}
 _DECLARED = re.compile(r"([\w ]+[\s*]+)(citlali_\w+)\s*\(([^)]*)\)\s*;")

@@ -8,6 +8,7 @@ CUDA device, they raise.
 from __future__ import annotations
 
 import ctypes
+import math
 import operator
 from typing import Optional
 
@@ -573,6 +574,47 @@ def gemm_tc(x, w, y, accumulate=False, error_flag=None, swiglu=False, force_spli
                                         _ptr(emit_sumsq), _ptr(scale_sumsq), _i(groups), _i(int(dim)), _f(float(eps)), _stream()),
            "gemm_tc")
 
+
+class DenseLayer(ctypes.Structure):
+    """``CitlaliDenseLayer`` of csrc/api.h."""
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("qkv", "o", "gate_up", "down", "q_gain", "k_gain", "inv_freq", "k_pool", "v_pool", "page_table")]
+                + [(n, ctypes.c_int) for n in ("gain_dtype", "rotary_dim", "page_table_stride", "pool_pages", "page_size", "hidden", "inter",
+                                               "nq", "nkv", "head_dim", "window")]
+                + [(n, ctypes.c_float) for n in ("head_eps", "scale", "mixer_eps", "ff_eps")])
+
+
+def dense_layer_supports(nq, nkv, head_dim, page_size, max_new) -> bool:
+    return bool(lib().citlali_dense_layer_supports(_i(nq), _i(nkv), _i(head_dim), _i(page_size), _i(max_new)))
+
+
+def dense_layer(weights, gains, inv_freq, rotary_dim, cache_view, sizes, eps, x, scratch, normed_in, normed_mid, normed_out, batch,
+                error_flag):
+    """A whole layer over at most 128 rows (csrc/dense_layer.cu): ``weights`` (qkv, o, gate_up, down), ``gains`` of the head norms,
+    ``sizes`` (hidden, inter, query heads, key heads, head size, window), ``eps`` (head norms, mixer's norm, feed-forward's norm),
+    ``scratch`` (qkv rows, heads, activations), three pairs (rows, sums of squares).  The parts it stands for have checked their
+    tensors where they were bound; what a step brings is checked here."""
+    _need_cuda(x, cache_view.keys, cache_view.values, cache_view.page_table, batch.row_slot, error_flag, *weights, *scratch, *normed_in,
+               *normed_mid, *normed_out)
+    qkv, o, gate_up, down = weights
+    hidden, inter, nq, nkv, d, window = sizes
+    q_gain, k_gain = gains
+    rows, table = x.shape[0], cache_view.page_table
+    require(qkv.shape == ((nq + 2 * nkv) * d, hidden) and o.shape == (hidden, nq * d) and gate_up.shape == (2 * inter, hidden)
+            and down.shape == (hidden, inter) and x.dtype == torch.float32 and x.shape[1] == hidden and batch.rows == rows <= 128
+            and cache_view.keys.dtype == torch.bfloat16 and normed_in[0].shape == x.shape and normed_mid[0].shape == x.shape
+            and normed_out[0].shape == x.shape and inv_freq.numel() == rotary_dim // 2, "dense_layer: shapes or dtypes do not fit")
+    layer = DenseLayer(qkv.data_ptr(), o.data_ptr(), gate_up.data_ptr(), down.data_ptr(), _ptr(q_gain), _ptr(k_gain), inv_freq.data_ptr(),
+                       cache_view.keys.data_ptr(), cache_view.values.data_ptr(), table.data_ptr(),
+                       _F32 if q_gain is None else _dtype_code(q_gain), rotary_dim, table.shape[1], cache_view.keys.shape[0],
+                       cache_view.page_size, hidden, inter, nq, nkv, d, window, eps[0], 1.0 / math.sqrt(d), eps[1], eps[2])
+    _check(lib().citlali_dense_layer(
+        ctypes.byref(layer), x.data_ptr(), scratch[0].data_ptr(), scratch[1].data_ptr(), scratch[2].data_ptr(), normed_in[0].data_ptr(),
+        normed_in[1].data_ptr(), normed_mid[0].data_ptr(), normed_mid[1].data_ptr(), normed_out[0].data_ptr(), normed_out[1].data_ptr(),
+        batch.row_slot.data_ptr(), batch.row_pos.data_ptr(), batch.seq_start.data_ptr(), batch.seq_slot.data_ptr(),
+        batch.seq_past.data_ptr(), rows, batch.sequences, batch.max_new, _ptr(error_flag), sm_count(x.device), _stream()), "dense_layer")
+
+
+_KERNELS_PER_CALL["dense_layer"] = 6
 
 _GEMM_ACTS = {None: 0, "gelu_gate": 4, "relu_squared": 8}
 

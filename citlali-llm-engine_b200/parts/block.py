@@ -24,7 +24,9 @@ import torch
 from .. import ops
 from ..errors import require
 from ..weights.loader import TensorSpec
+from .attention import GQAttention
 from .base import NormedRows, build_part, register_part
+from .feed_forward import GatedSiluFeedForward
 from .linear import DenseLinear
 from .norm import RMSNorm
 
@@ -41,6 +43,10 @@ class PreNormResidualBlock:
         if has("feed_forward"):
             self.feed_forward_norm = build_part("norm", layer_spec.part("feed_forward_norm"))
             self.feed_forward = build_part("feed_forward", layer_spec.part("feed_forward"))
+
+    def kernel_sources(self, dtype):
+        whole = type(self.mixer) is GQAttention and type(self.feed_forward) is GatedSiluFeedForward
+        return ("dense_layer",) if whole and dtype == torch.bfloat16 else ()
 
     def parts(self):
         return [p for p in (self.mixer_norm, self.mixer, self.feed_forward_norm, self.feed_forward) if p is not None]
@@ -64,6 +70,18 @@ class PreNormResidualBlock:
         if self.norms_in_products:
             self.mixer.fold_norm_gain(self.mixer_norm.gain_moves_downstream())
             self.feed_forward.fold_norm_gain(self.feed_forward_norm.gain_moves_downstream())
+        self.error_flag = ctx.error_flag
+
+    def _from_one_call(self, batch, cache_view, write_cache) -> bool:
+        """Whether this layer's launches over a run of few new rows can be made by one call (``ops.dense_layer``): plain attention with
+        the rotation in the cache's kernel and a plain gated feed-forward."""
+        mixer, ff = self.mixer, self.feed_forward
+        if (type(mixer) is not GQAttention or type(ff) is not GatedSiluFeedForward or not write_cache or not mixer.kv_projection
+                or not mixer.fused_position or cache_view is None or batch.is_decode or torch.cuda.is_current_stream_capturing()):
+            return False
+        req = cache_view.requirement
+        return (req.head_dim == mixer.d and req.num_kv_heads == mixer.nkv and cache_view.keys.dtype == torch.bfloat16
+                and ops.dense_layer_supports(mixer.nq, mixer.nkv, mixer.d, cache_view.page_size, batch.max_new))
 
     def forward(self, x, batch, cache_view, write_cache=True):
         if getattr(self, "norms_in_products", False) and 0 < batch.rows <= _FEW_ROWS:
@@ -89,6 +107,19 @@ class PreNormResidualBlock:
             carried = NormedRows(*after_ff, hidden)
         elif carried.rows is after_mixer[0]:
             after_mixer, after_ff = after_ff, after_mixer
+        if self._from_one_call(batch, cache_view, write_cache):
+            mixer, ff = self.mixer, self.feed_forward
+            widths = (mixer.qkv.out_features, mixer.nq * mixer.d, ff.inter)
+            scratch = batch.layer_scratch
+            if scratch is None or tuple(t.shape[1] for t in scratch) != widths:
+                scratch = batch.layer_scratch = tuple(torch.empty((rows, w), dtype=torch.bfloat16, device=x.device) for w in widths)
+            ops.dense_layer((mixer.qkv.weight, mixer.o.weight, ff.gate_up.weight, ff.down.weight), (mixer.q_gain, mixer.k_gain),
+                            mixer.inv_freq, mixer.rotary_dim, cache_view,
+                            (hidden, ff.inter, mixer.nq, mixer.nkv, mixer.d, int(mixer.window or 0)),
+                            (float(mixer.eps or 0.0), self.mixer_norm.eps, self.feed_forward_norm.eps), x, scratch,
+                            (carried.rows, carried.sumsq), after_mixer, after_ff, batch, self.error_flag)
+            batch.norm_carry = NormedRows(after_ff[0], after_ff[1], hidden)
+            return x
         self.mixer.forward(carried.with_eps(self.mixer_norm.eps), batch, cache_view, x, write_cache, emit=after_mixer)
         self.feed_forward.forward(NormedRows(after_mixer[0], after_mixer[1], hidden, self.feed_forward_norm.eps), batch, x,
                                   emit=after_ff)

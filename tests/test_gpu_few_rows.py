@@ -3,6 +3,7 @@ sizes that do not fill the tiles, both gates, both rotation layouts, outputs in 
 import pytest
 import torch
 
+import citlali_b200 as cb
 from citlali_b200 import ops
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +73,38 @@ def test_delta_step_against_the_kernels_it_stands_for(D, V, H, KH, mode, taps):
     with pytest.raises(Exception, match="one each"):
         ops.delta_prepare(proj, taps_w, states[0], H * D * V, slots, i32([0, 2, 2, 3, 4]), slots, B - 1, a_log, bias, prep, H, KH, D, V, 1e-6,
                           block_a_segment=True, one_row_each=True, decay_in=decay, channel_decay=bool(mode))
+
+
+@pytest.mark.parametrize("d, heads, kv", [(128, 4, 2), (64, 6, 3), (80, 4, 4)])
+@pytest.mark.parametrize("lengths", [(2,), (47,), (48,), (128,), (5, 1, 60, 3), (1, 31, 32, 33, 31)])
+def test_a_layer_from_one_call_gives_the_bits_of_its_launches_one_by_one(d, heads, kv, lengths, monkeypatch):
+    """Few new rows of one or several sequences, at their start and behind cached tokens, either side of the tcgen05 attention's 48 rows."""
+    from citlali_b200.engine.step import StepEntry
+    from citlali_b200.parts.block import PreNormResidualBlock
+    config = cb.config_from_dict(dict(
+        architectures=["Qwen3ForCausalLM"], num_hidden_layers=3, hidden_size=256, num_attention_heads=heads, num_key_value_heads=kv,
+        head_dim=d, intermediate_size=352, vocab_size=500, rope_theta=1e4, rms_norm_eps=1e-6, tie_word_embeddings=True,
+        max_position_embeddings=512))
+    session = cb.InferenceSession().load_random(config, seed=3, max_context=400, dtype="bfloat16", device=DEV, max_batch=len(lengths),
+                                                gain_spread=0.1)
+    calls = []
+    whole = ops.dense_layer
+    monkeypatch.setattr(ops, "dense_layer", lambda *a: (calls.append(1), whole(*a)))
+
+    def steps():
+        g = torch.Generator().manual_seed(7)
+        slots = [session.acquire() for _ in lengths]
+        out = []
+        for _ in range(2):
+            tokens = [torch.randint(0, 500, (n,), generator=g).tolist() for n in lengths]
+            out.append(session.step([StepEntry(s, t, list(range(len(t)))) for s, t in zip(slots, tokens)]))
+        for s in slots:
+            session.release(s)
+        return out
+
+    got = steps()
+    assert len(calls) == 6
+    monkeypatch.setattr(PreNormResidualBlock, "_from_one_call", lambda *a: False)
+    want = steps()
+    session.check_device_errors()
+    assert len(calls) == 6 and all(torch.equal(a, b) for a, b in zip(got, want))

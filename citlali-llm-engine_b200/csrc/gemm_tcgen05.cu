@@ -552,9 +552,10 @@ struct Plan {
 // 20 + 0.03 x width microseconds at K = 4096).
 // Swapped form: up to 128 rows of x always; up to kMaxSwappedRows rows (one tile of 256 rows of x) when the
 // normal form would leave SMs without a tile, i.e. against a narrow weight matrix: a tile's K loop of 26 us
-// would then bound the product, while here every weight tile is streamed once and K is split over the SMs.
+// would then bound the product, while here every weight tile is streamed once and K is split over the SMs; unless K is short.
 // The split aims at a block (two for narrow tiles) on every SM and keeps at least four K blocks per block.
-static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, bool gate_runs = false) {
+// `normed`: the epilogue does a norm's work, which the normal form's does not.
+static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, bool gate_runs = false, bool normed = false) {
     Plan pl;
     pl.swapped = false;
     pl.bn = 128;
@@ -572,6 +573,7 @@ static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, b
         }
         pl.cost = best;
     }
+    const int normal_bn = pl.bn;
     if (M <= 128 || (M <= kMaxSwappedRows && normal_tiles < sm_count)) {
         pl.swapped = true;
         pl.bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
@@ -585,6 +587,22 @@ static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, b
         int pow2 = 1;
         while (pow2 * 2 <= s) pow2 *= 2;
         s = pow2;
+        // tiles of 256 rows of x fill an SM: of clusters of eight such blocks the device does not hold sixteen at once (130 to 256 rows,
+        // N 2,048, K 6,144 / 8,192: 27 / 30 -> 19 / 22 us)
+        if (pl.bn == 256 && s == 8 && tiles > 8) s = 4;
+        // more than 128 rows: the normal form instead, where a tile's whole K costs less than this form's share of it, its sums and their
+        // exchange (both in us; 130 / 256 rows, this form -> the normal one: K 1,024, N 5,632 17 / 19 -> 9; K 2,048, N 2,048 21 -> 14,
+        // N 8,192 19 / 20 -> 15, N 12,288 25 / 28 -> 15; K 4,096, N 6,144 24 / 25 -> 23, N 12,288 35 / 37 -> 26 / 27; this form stays at
+        // K 4,096, N 4,096, 18 us, where the normal one takes 28)
+        if (M > 128 && N >= 192 && force_splits <= 0 && !normed) {
+            const double here = 8.0 + 0.55 * ((kblocks + s - 1) / s) + (s > 1 ? 6.0 : 0.0);
+            const double there = 4.0 + (0.07 + 0.0017 * normal_bn) * (double)((normal_tiles + sm_count - 1) / sm_count) * kblocks;
+            if (there < here) {
+                pl.swapped = false;
+                pl.bn = normal_bn;
+                return pl;
+            }
+        }
         if (force_splits > 0) s = force_splits > kMaxSplits ? kMaxSplits : force_splits;
         if (s > kblocks) s = kblocks;
         if (s < 1) s = 1;
@@ -740,8 +758,8 @@ static int gemm_tc_any(const void* x, const void* w, void* y, int y_dtype, int M
         return kBadShape;
     }
     if (sm_count <= 0) sm_count = device_sm_count();
-    const Plan pl = make_plan(M, N, K, sm_count, force_splits, swiglu);
     const bool normed = emit_rows != nullptr || emit_sumsq != nullptr || scale_sumsq != nullptr;
+    const Plan pl = make_plan(M, N, K, sm_count, force_splits, swiglu, normed);
     if (normed) {
         if (!pl.swapped) {
             set_last_error("gemm_tc_normed: %d rows of x run the prompt form of the product, whose epilogue does no norm work", M);

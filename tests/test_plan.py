@@ -28,6 +28,15 @@ def test_few_rows_put_the_weights_on_the_wide_side(M, bn):
     assert splits in (1, 2, 4, 8)
 
 
+@pytest.mark.parametrize("N, K, form", [(12288, 2048, (False, 192, 1)), (2048, 2048, (False, 192, 1)), (5632, 1024, (False, 192, 1)),
+                                        (2048, 6144, (True, 256, 4)), (4096, 4096, (True, 256, 4)), (1024, 4096, (True, 256, 8)),
+                                        (4096, 12288, (True, 256, 4))])
+def test_more_than_128_rows_take_the_weights_wide_side_only_where_k_is_long(N, K, form):
+    assert plan(129, N, K) == plan(256, N, K) == form
+    assert plan(128, N, K)[:2] == (True, 128) and not plan(257, N, K)[0]
+    assert plan(200, N, K, force=2)[0]                   # a forced split is one of the few-row form
+
+
 def test_k_is_split_by_shape_alone():
     # 148 SMs, two blocks each: 296 places for (tile, split) pairs; a split keeps four K blocks of 64 at least
     assert plan(8, 6144, 4096) == (True, 16, 4)          # 48 tiles: 6 would fit, powers of two only

@@ -26,6 +26,10 @@ extern "C" int citlali_dense_layer(const CitlaliDenseLayer* l, float* x, void* q
                                    const int32_t* seq_past, int rows, int sequences, int max_new, int32_t* error_flag, int sm_count,
                                    cudaStream_t stream) {
     if (rows <= 0) return 0;
+    if (rows > 128) {       // refused before the first launch: from there on a product may run the form that does no norm's work
+        set_last_error("dense_layer: %d rows (128 at most)", rows);
+        return kBadShape;
+    }
     if (!citlali_dense_layer_supports(l->nq, l->nkv, l->head_dim, l->page_size, max_new) || l->hidden % 32 != 0 || l->inter % 16 != 0) {
         set_last_error("dense_layer: %d heads over %d of %d, pages of %d, width %d, inner width %d", l->nq, l->nkv, l->head_dim,
                        l->page_size, l->hidden, l->inter);

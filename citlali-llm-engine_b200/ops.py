@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import math
 import operator
+import struct
 from typing import Optional
 
 import torch
@@ -575,12 +576,9 @@ def gemm_tc(x, w, y, accumulate=False, error_flag=None, swiglu=False, force_spli
            "gemm_tc")
 
 
-class DenseLayer(ctypes.Structure):
-    """``CitlaliDenseLayer`` of csrc/api.h."""
-    _fields_ = ([(n, ctypes.c_void_p) for n in ("qkv", "o", "gate_up", "down", "q_gain", "k_gain", "inv_freq", "k_pool", "v_pool", "page_table")]
-                + [(n, ctypes.c_int) for n in ("gain_dtype", "rotary_dim", "page_table_stride", "pool_pages", "page_size", "hidden", "inter",
-                                               "nq", "nkv", "head_dim", "window")]
-                + [(n, ctypes.c_float) for n in ("head_eps", "scale", "mixer_eps", "ff_eps")])
+_ONLY_I32, _ONLY_F32, _ONLY_BF16 = {torch.int32}, {torch.float32}, {torch.bfloat16}
+# ``CitlaliDenseLayer`` of csrc/api.h: ten addresses, eleven whole numbers, four floats, filled up to the structure's alignment
+_DENSE_LAYER = struct.Struct("@10P11i4f0P")
 
 
 def dense_layer_supports(nq, nkv, head_dim, page_size, max_new) -> bool:
@@ -591,24 +589,33 @@ def dense_layer(weights, gains, inv_freq, rotary_dim, cache_view, sizes, eps, x,
                 error_flag):
     """A whole layer over at most 128 rows (csrc/dense_layer.cu): ``weights`` (qkv, o, gate_up, down), ``gains`` of the head norms,
     ``sizes`` (hidden, inter, query heads, key heads, head size, window), ``eps`` (head norms, mixer's norm, feed-forward's norm),
-    ``scratch`` (qkv rows, heads, activations), three pairs (rows, sums of squares).  The parts it stands for have checked their
-    tensors where they were bound; what a step brings is checked here."""
-    _need_cuda(x, cache_view.keys, cache_view.values, cache_view.page_table, batch.row_slot, error_flag, *weights, *scratch, *normed_in,
-               *normed_mid, *normed_out)
+    ``scratch`` (qkv rows, heads, activations), three pairs (rows, sums of squares).  Every tensor the kernels read or write is checked
+    here, as the six calls this one stands for check theirs."""
     qkv, o, gate_up, down = weights
     hidden, inter, nq, nkv, d, window = sizes
     q_gain, k_gain = gains
-    rows, table = x.shape[0], cache_view.page_table
-    require(qkv.shape == ((nq + 2 * nkv) * d, hidden) and o.shape == (hidden, nq * d) and gate_up.shape == (2 * inter, hidden)
-            and down.shape == (hidden, inter) and x.dtype == torch.float32 and x.shape[1] == hidden and batch.rows == rows <= 128
-            and cache_view.keys.dtype == torch.bfloat16 and normed_in[0].shape == x.shape and normed_mid[0].shape == x.shape
-            and normed_out[0].shape == x.shape and inv_freq.numel() == rotary_dim // 2, "dense_layer: shapes or dtypes do not fit")
-    layer = DenseLayer(qkv.data_ptr(), o.data_ptr(), gate_up.data_ptr(), down.data_ptr(), _ptr(q_gain), _ptr(k_gain), inv_freq.data_ptr(),
-                       cache_view.keys.data_ptr(), cache_view.values.data_ptr(), table.data_ptr(),
-                       _F32 if q_gain is None else _dtype_code(q_gain), rotary_dim, table.shape[1], cache_view.keys.shape[0],
-                       cache_view.page_size, hidden, inter, nq, nkv, d, window, eps[0], 1.0 / math.sqrt(d), eps[1], eps[2])
+    rows, table, keys, values = x.shape[0], cache_view.page_table, cache_view.keys, cache_view.values
+    indices = (batch.row_slot, batch.row_pos, batch.seq_start, batch.seq_slot, batch.seq_past, table)
+    in_bf16 = (*weights, *scratch, keys, values, normed_in[0], normed_mid[0], normed_out[0])
+    in_f32 = (x, inv_freq, normed_in[1], normed_mid[1], normed_out[1])
+    _need_cuda(*in_bf16, *in_f32, *indices, q_gain, k_gain, error_flag)
+    require({t.dtype for t in indices} == _ONLY_I32, "dense_layer: index tensors are int32")
+    require({t.dtype for t in in_bf16} == _ONLY_BF16, "dense_layer: weights, cache and rows are bfloat16")
+    require({t.dtype for t in in_f32} == _ONLY_F32, "dense_layer: residual rows, frequencies and sums of squares are float32")
+    require(q_gain is None or k_gain is None or q_gain.dtype == k_gain.dtype, "dense_layer: q and k gains differ in dtype")
+    stream, sums, out = x.shape, (rows, hidden // 32), (nq + 2 * nkv) * d
+    require(qkv.shape == (out, hidden) and o.shape == (hidden, nq * d) and gate_up.shape == (2 * inter, hidden)
+            and down.shape == (hidden, inter) and stream == (rows, hidden) and batch.rows == rows <= 128
+            and scratch[0].shape == (rows, out) and scratch[1].shape == (rows, nq * d) and scratch[2].shape == (rows, inter)
+            and normed_in[0].shape == stream and normed_mid[0].shape == stream and normed_out[0].shape == stream
+            and normed_in[1].shape == sums and normed_mid[1].shape == sums and normed_out[1].shape == sums
+            and inv_freq.numel() == rotary_dim // 2, "dense_layer: shapes do not fit")
+    layer = _DENSE_LAYER.pack(
+        qkv.data_ptr(), o.data_ptr(), gate_up.data_ptr(), down.data_ptr(), _ptr(q_gain) or 0, _ptr(k_gain) or 0, inv_freq.data_ptr(),
+        keys.data_ptr(), values.data_ptr(), table.data_ptr(), _F32 if q_gain is None else _dtype_code(q_gain), rotary_dim, table.shape[1],
+        keys.shape[0], cache_view.page_size, hidden, inter, nq, nkv, d, window, eps[0], 1.0 / math.sqrt(d), eps[1], eps[2])
     _check(lib().citlali_dense_layer(
-        ctypes.byref(layer), x.data_ptr(), scratch[0].data_ptr(), scratch[1].data_ptr(), scratch[2].data_ptr(), normed_in[0].data_ptr(),
+        layer, x.data_ptr(), scratch[0].data_ptr(), scratch[1].data_ptr(), scratch[2].data_ptr(), normed_in[0].data_ptr(),
         normed_in[1].data_ptr(), normed_mid[0].data_ptr(), normed_mid[1].data_ptr(), normed_out[0].data_ptr(), normed_out[1].data_ptr(),
         batch.row_slot.data_ptr(), batch.row_pos.data_ptr(), batch.seq_start.data_ptr(), batch.seq_slot.data_ptr(),
         batch.seq_past.data_ptr(), rows, batch.sequences, batch.max_new, _ptr(error_flag), sm_count(x.device), _stream()), "dense_layer")

@@ -128,7 +128,7 @@ class StepBatch:
     norm_carry_in: Optional["NormedRows"] = None
     # the two pairs of buffers such rows take turns in, for the whole step (parts/block.py)
     norm_buffers: Optional[list] = None
-    # the scratch rows of a layer that runs from one call, for the whole step (parts/block.py)
+    # the scratch rows of a layer that runs from one call, behind their place and sizes, for the whole step (parts/block.py)
     layer_scratch: Optional[tuple] = None
     # by a delta rule's sizes: whether it runs in chunks in this step (``ops.delta_runs_in_chunks``; its layers ask one by one)
     delta_in_chunks: dict = field(default_factory=dict)

@@ -109,14 +109,13 @@ class PreNormResidualBlock:
             after_mixer, after_ff = after_ff, after_mixer
         if self._from_one_call(batch, cache_view, write_cache):
             mixer, ff = self.mixer, self.feed_forward
-            widths = (mixer.qkv.out_features, mixer.nq * mixer.d, ff.inter)
-            scratch = batch.layer_scratch
-            if scratch is None or tuple(t.shape[1] for t in scratch) != widths:
-                scratch = batch.layer_scratch = tuple(torch.empty((rows, w), dtype=torch.bfloat16, device=x.device) for w in widths)
+            kind = (x.device, rows, mixer.qkv.out_features, mixer.nq * mixer.d, ff.inter)
+            if batch.layer_scratch is None or batch.layer_scratch[0] != kind:
+                batch.layer_scratch = (kind, [torch.empty((rows, w), dtype=torch.bfloat16, device=x.device) for w in kind[2:]])
             ops.dense_layer((mixer.qkv.weight, mixer.o.weight, ff.gate_up.weight, ff.down.weight), (mixer.q_gain, mixer.k_gain),
                             mixer.inv_freq, mixer.rotary_dim, cache_view,
                             (hidden, ff.inter, mixer.nq, mixer.nkv, mixer.d, int(mixer.window or 0)),
-                            (float(mixer.eps or 0.0), self.mixer_norm.eps, self.feed_forward_norm.eps), x, scratch,
+                            (float(mixer.eps or 0.0), self.mixer_norm.eps, self.feed_forward_norm.eps), x, batch.layer_scratch[1],
                             (carried.rows, carried.sumsq), after_mixer, after_ff, batch, self.error_flag)
             batch.norm_carry = NormedRows(after_ff[0], after_ff[1], hidden)
             return x

@@ -68,10 +68,11 @@ gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __restr
 
 // The same product for float32 operands and many rows: the same chain an element (k ascending, the last 16 k filled up with
 // zeros), so the same bits as the kernel above.
-// What bounds it: the FMA units.  A thread owns 8 x 8 outputs, so that a k costs it four 16-byte reads of shared memory
-// for 64 multiply-adds, two of them an instruction (fma.rn.f32x2 rounds each half like fmaf); both operands lie transposed
+// What bounds it: the FMA units.  A thread owns 8 x RN outputs, so that a k costs it four (three) 16-byte reads of shared memory
+// for 64 (32) multiply-adds, two of them an instruction (fma.rn.f32x2 rounds each half like fmaf); both operands lie transposed
 // [k][row] in shared memory, put there element by element by asynchronous copies (any alignment, any K) three tiles deep.
-// For matrices with tiles enough for every SM twice; fewer run the kernel behind this one (see launch_wide).  682 rows, K 1,024: N 5,632
+// TN = 128 for matrices with tiles enough for every SM twice, TN = 64 for some that cannot be copied in pieces; the others run the
+// kernel behind this one (see launch_wide).  682 rows, K 1,024: N 5,632
 // 212 us, N 32,768 977 (18.6 and 23.4 T multiply-adds a second of 37).
 __device__ __forceinline__ void cp_async4_or_zero(uint32_t dst, const float* src, bool there) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(there ? 4 : 0) : "memory");
@@ -87,10 +88,10 @@ __device__ __forceinline__ unsigned long long both(float v) {
     return d;
 }
 
-template <bool kAccumulate>
+template <int TN, bool kAccumulate>
 __global__ void __launch_bounds__(128, 3)
 gemm_simt_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K) {
-    constexpr int TM = 64, TN = 128, STAGES = 3, TX = 16, RN = TN / TX, LX = TM + 4, LW = TN + 4;
+    constexpr int TM = 64, STAGES = 3, TX = 16, RN = TN / TX, LX = TM + 4, LW = TN + 4;
     __shared__ __align__(16) float xs[STAGES][kTileK][LX];
     __shared__ __align__(16) float ws[STAGES][kTileK][LW];
     dependents_may_launch();
@@ -181,7 +182,7 @@ gemm_simt_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, 
 // What bounds it: a block or two an SM, a warp or two a scheduler, so the chain of reads and multiply-adds of a thread.  Rows of both
 // operands lie in shared memory as they do in memory, 32 k of each, copied in 16-byte pieces (kPieces; else element by element) three
 // tiles deep; a thread's 16-byte reads are four k of a row, so a copy costs a quarter of the instructions, and 8 RN multiply-adds a k
-// need no moves.  Lanes are placed as in the delta rule's scan: two that read the same place are neighbours or two apart, and a read
+// need no moves.  Element by element a warp copies 32 k of one row (eight lanes a row, four k apart: 49 -> 45 us at 682 rows, N 1,024, K 1,022).  Lanes are placed as in the delta rule's scan: two that read the same place are neighbours or two apart, and a read
 // costs two wavefronts.
 // 682 rows one product after another, 64 x 64 tiles of the kernel above -> here: N 1,024, K 1,024 / 2,816 (143 tiles of 64 x 80 instead of
 // 176) 94 / 254 -> 43 / 111 us; N 1,536, K 1,024 97 -> 62; 200 rows, N 1,024 / 1,536 47 / 71 -> 22 / 29; 33 rows, N 1,024 41 -> 21.
@@ -197,32 +198,43 @@ gemm_simt_narrow_kernel(const float* __restrict__ x, const float* __restrict__ w
     const int tx = (lane & 1) | ((lane >> 1) & 2) | ((lane >> 2) & 4), ty = ((lane >> 1) & 1) | ((lane >> 2) & 2);    // lane bits 0 2 4; 1 3
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     const int count = (K + TK - 1) / TK;
-    const int lk = (tid & 7) * 4, lr = tid >> 3;
+    // in pieces: eight threads a row, a thread's rows 16 apart; element by element: a warp a row, so that a copy asks for four or five
+    // sectors, its rows four apart
+    const int lk = kPieces ? (tid & 7) * 4 : lane, lr = kPieces ? tid >> 3 : warp;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(narrow_tiles) + (uint32_t)((lr * LD + lk) * 4);
-    const float* src[kCopies];
-    bool in[kCopies];
+    const float* src[kPieces ? kCopies : 1];
+    bool in[kPieces ? kCopies : 1];
+    if constexpr (kPieces) {
 #pragma unroll
-    for (int i = 0; i < kCopies; ++i) {
-        const int r = 16 * i + lr, row = r < TM ? m0 + r : n0 + r - TM;      // (TM a multiple of 16: a pass is all x or all w)
-        in[i] = row < (r < TM ? M : N);
-        src[i] = (r < TM ? x : w) + (in[i] ? (size_t)row * K : 0) + lk;
+        for (int i = 0; i < kCopies; ++i) {
+            const int r = 16 * i + lr, row = r < TM ? m0 + r : n0 + r - TM;      // (TM a multiple of 16: a pass is all x or all w)
+            in[i] = row < (r < TM ? M : N);
+            src[i] = (r < TM ? x : w) + (in[i] ? (size_t)row * K : 0) + lk;
+        }
     }
     auto fetch = [&](int tile) {
         if (tile < count) {
             const uint32_t dst = base + (uint32_t)((tile % STAGES) * (TM + TN) * LD * 4);
             const int k = tile * TK;
+            if constexpr (kPieces) {
 #pragma unroll
-            for (int i = 0; i < kCopies; ++i) {
-                if constexpr (kPieces) {
+                for (int i = 0; i < kCopies; ++i) {
                     const bool there = in[i] && k + lk < K;
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(i * 16 * LD * 4)),
                                  "l"(there ? src[i] + k : src[i] - lk), "r"(there ? 16 : 0) : "memory");
-                } else {
+                }
+            } else {
+                const bool k_in = k + lk < K;
+                const float *xr = x + (size_t)(m0 + lr) * K + k + lk, *wr = w + (size_t)(n0 + lr) * K + k + lk;
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const bool there = in[i] && k + lk + e < K;
-                        cp_async4_or_zero(dst + (uint32_t)((i * 16 * LD + e) * 4), there ? src[i] + k + e : src[i] - lk, there);
-                    }
+                for (int i = 0; i < TM / 4; ++i, xr += (size_t)4 * K) {
+                    const bool there = k_in && m0 + lr + 4 * i < M;
+                    cp_async4_or_zero(dst + (uint32_t)(i * 4 * LD * 4), there ? xr : x, there);
+                }
+#pragma unroll
+                for (int i = 0; i < TN / 4; ++i, wr += (size_t)4 * K) {
+                    const bool there = k_in && n0 + lr + 4 * i < N;
+                    cp_async4_or_zero(dst + (uint32_t)((TM + i * 4) * LD * 4), there ? wr : w, there);
                 }
             }
         }
@@ -356,19 +368,28 @@ static int launch_few(const float* x, const float* w, float* y, int M, int N, in
 // Tiles of 64 x 128 where they give every SM at least two, else narrower ones.
 constexpr int kWideRows = 32;
 
-// Columns a thread of the narrow kernel: the RN of 2 to 6 that gives an SM the shortest share, tiles times a tile's time (four k: 32 RN
-// issues of multiply-adds a scheduler or 8 (8 + RN) wavefronts of reads, whichever is longer); of equal ones the widest, which reads x
-// less often (682 rows, N 1,536: two tiles of 64 columns an SM 62 us, four of 32 66).
-static int narrow_columns(long rows, int N, int sm_count) {
+// Columns a thread of the narrow kernel: the RN of 2 to 6 that gives an SM the shortest share.  A share costs a first part and a part a
+// tile; measured in pieces at K 1,024 (us; element by element some 15 % more, the order is the same).  An SM with one tile waits for its
+// one warp a scheduler, hence the first part: two tiles of 48 columns beat one of 96 where K is short (130 rows, N 4,096, K 64 / 96
+// 7.4 / 8.8 -> 4.9 / 6.3 us) and come out even where it is long.
+constexpr int kNarrowTile[5] = {15, 21, 27, 32, 39}, kNarrowFirst[5] = {5, 5, 7, 7, 9};
+static int narrow_columns(long rows, int N, int sm_count, long* least) {
     int best = 2;
-    long least = -1;
+    *least = -1;
     for (int rn = 2; rn <= 6; ++rn) {
         const long tiles = rows * ((N + 16 * rn - 1) / (16 * rn));
-        const long share = (tiles + sm_count - 1) / sm_count * (4 * rn > 8 + rn ? 4 * rn : 8 + rn);
-        if (least < 0 || share <= least) { least = share; best = rn; }
+        const long share = (tiles + sm_count - 1) / sm_count * kNarrowTile[rn - 2] + kNarrowFirst[rn - 2];
+        if (*least < 0 || share < *least) { *least = share; best = rn; }
     }
     return best;
 }
+
+// Operands that cannot be copied in pieces: whether the transposed tiles of 64 columns are quicker than the narrow kernel, whose deeper
+// tiles are filled up further and take an SM's shared memory, so that short products end before they pay.  `share`: the narrow kernel's.
+// Narrow -> transposed at 26 (260 rows, N 1,280), K 33 / 50 5.1 / 5.0 -> 4.5 / 6.7 us; 88, three tiles of 64 columns an SM (1,400 rows,
+// N 1,280), K 130 / 333 18.1 / 35.9 -> 16.3 / 34.9; 103, three of 80 (1,000 rows, N 2,048), K 130 / 333 22.7 / 43.8 -> 21.2 / 45.6; 115, four of
+// 64 (N 2,304), K 130 / 333 / 667 28 / 58 / 88 -> 21 / 46 / 87.
+static bool transposed_tiles_are_quicker(long share, int K) { return K < (share >= 104 ? 640 : share >= 88 ? 160 : 49); }
 
 template <int RN, bool kPieces>
 static int launch_narrow(const float* x, const float* w, float* y, int M, int N, int K, int accumulate, cudaStream_t stream) {
@@ -396,17 +417,23 @@ static int launch_narrow(int rn, const float* x, const float* w, float* y, int M
     }
 }
 
+template <int TN>
 static int launch_wide(const float* x, const float* w, float* y, int M, int N, int K, int accumulate, cudaStream_t stream) {
-    const long rows = (M + 63) / 64;
-    if (rows * ((N + 127) / 128) >= 2L * device_sm_count()) {
-        dim3 grid((N + 127) / 128, (unsigned)rows);
-        if (accumulate) launch_kernel(gemm_simt_wide_kernel<true>, grid, 128, 0, stream, x, w, y, M, N, K);
-        else launch_kernel(gemm_simt_wide_kernel<false>, grid, 128, 0, stream, x, w, y, M, N, K);
-        return CITLALI_LAUNCH_CHECK();
-    }
-    const int rn = narrow_columns(rows, N, device_sm_count());
+    dim3 grid((N + TN - 1) / TN, (M + 63) / 64);
+    if (accumulate) launch_kernel(gemm_simt_wide_kernel<TN, true>, grid, 128, 0, stream, x, w, y, M, N, K);
+    else launch_kernel(gemm_simt_wide_kernel<TN, false>, grid, 128, 0, stream, x, w, y, M, N, K);
+    return CITLALI_LAUNCH_CHECK();
+}
+
+static int launch_wide(const float* x, const float* w, float* y, int M, int N, int K, int accumulate, cudaStream_t stream) {
+    const long rows = (M + 63) / 64, sms = device_sm_count();
+    if (rows * ((N + 127) / 128) >= 2 * sms) return launch_wide<128>(x, w, y, M, N, K, accumulate, stream);
     const bool pieces = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15u) == 0;
-    return pieces ? launch_narrow<true>(rn, x, w, y, M, N, K, accumulate, stream) : launch_narrow<false>(rn, x, w, y, M, N, K, accumulate, stream);
+    long share;
+    const int rn = narrow_columns(rows, N, (int)sms, &share);
+    if (pieces) return launch_narrow<true>(rn, x, w, y, M, N, K, accumulate, stream);
+    if (transposed_tiles_are_quicker(share, K)) return launch_wide<64>(x, w, y, M, N, K, accumulate, stream);
+    return launch_narrow<false>(rn, x, w, y, M, N, K, accumulate, stream);
 }
 
 template <typename TX, typename TW, typename TY>

@@ -213,6 +213,28 @@ def test_narrow_32_bit_products_give_the_bits_of_few_rows(M, N, K, odd):
     assert torch.equal(added, base + y)
 
 
+@pytest.mark.parametrize("M, N, K, odd", [(65, 500, 50, False), (65, 2391, 67, False), (65, 3611, 68, True), (65, 4770, 201, False),
+                                          (200, 5929, 101, False), (65, 3611, 36, False), (200, 5929, 72, False), (1400, 1280, 159, False),
+                                          (1400, 1280, 161, False), (980, 2300, 100, True), (65, 500, 48, True), (65, 500, 47, False)])
+def test_32_bit_products_that_cannot_be_copied_in_pieces_and_the_widest_tiles(M, N, K, odd):
+    """Element by element in every width of the narrow tiles (32 to 96 columns) and in the transposed tiles of 64 columns, either side of
+    the lines between them; in pieces the two widths that the sizes above do not reach."""
+    g = torch.Generator().manual_seed(M + N + K)
+    store = torch.zeros(N * K + 1, device=DEV)
+    w = store[1:].view(N, K) if odd else store[:-1].view(N, K)
+    w.copy_(torch.randn(N, K, generator=g))
+    x, base = torch.randn(M, K, generator=g).to(DEV), torch.randn(M, N, generator=g).to(DEV)
+    y, added = torch.full((M, N), float("nan"), device=DEV), base.clone()
+    ops.gemm_simt(x, w, y)
+    ops.gemm_simt(x, w, added, accumulate=True)
+    few = torch.empty(31, N, device=DEV)
+    for r in range(0, M, 31):
+        n = min(31, M - r)
+        ops.gemm_simt(x[r:r + n].contiguous(), w, few[:n])
+        assert torch.equal(y[r:r + n], few[:n])
+    assert torch.equal(added, base + y)
+
+
 _SHARED_MEMORY_LIMITS = """
 import sys
 sys.path.insert(0, {root!r})

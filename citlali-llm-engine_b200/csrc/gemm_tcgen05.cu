@@ -18,8 +18,8 @@
 // several blocks so that every SM streams weights.  The splits of a tile are one thread-block
 // cluster: each block sends its float32 partial sums through distributed shared memory to the
 // block that owns that part of the tile, which adds them in split order and writes the result.
-// The split depends on the shape alone, never on the batch, so a row's result does not depend
-// on what else is in the step.
+// The split depends on the shape and the kind of epilogue alone, never on the batch, so a row's
+// result does not depend on what else is in the step.
 //
 // Every wait on an mbarrier gives up after a time limit, raises the error word and makes the
 // block leave through the normal exit (TMEM freed, copies in flight awaited).
@@ -89,6 +89,16 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
     return v;
 }
 
+// The wait for tensor-memory loads as what `a` and `b` come from, for arithmetic that follows.
+__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&a)[16], uint32_t (&b)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]), "+r"(a[8]), "+r"(a[9]),
+                   "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]), "+r"(b[0]), "+r"(b[1]), "+r"(b[2]),
+                   "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]), "+r"(b[8]), "+r"(b[9]), "+r"(b[10]), "+r"(b[11]),
+                   "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15])
+                 :: "memory");
+}
+
 // kAct: as in the pair kernel, the form whose epilogue adds a bias, squares or gates by GELU (tc_common.cuh).
 template <bool kFirst>
 __device__ __forceinline__ const float (&pick(const float (&)[kFirst ? 16 : 1], const float (&b)[16]))[16];
@@ -97,13 +107,19 @@ __device__ __forceinline__ const float (&pick<true>(const float (&a)[16], const 
 template <>
 __device__ __forceinline__ const float (&pick<false>(const float (&)[1], const float (&b)[16]))[16] { return b; }
 
-template <int BN, bool kSwapped, bool kAct>
+//
+// kChains: a sum over K in tensor memory loses up to an ulp an addition, all in one direction (the tensor core cuts off), so it is off
+// by as much as it is long (relative to the result, K 2,048 in one sum 2.1e-6, in eight 2.4e-7).  A form that takes the place of one whose K
+// was split over more blocks cuts its own range into kChains accumulators and adds these in float32: a block then has one unit.
+template <int BN, bool kSwapped, bool kAct, int kChains>
 __global__ void __launch_bounds__(threads_for(kSwapped, BN), (kSwapped && BN <= 128) ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmParams p) {
     constexpr int kStages = stages_for<BN>(kSwapped);
     constexpr uint32_t kBytesA = kBM * kBK * 2, kBytesB = BN * kBK * 2;
-    constexpr uint32_t kTmemCols = (kAccStages * BN) <= 32 ? 32 : (kAccStages * BN) <= 64 ? 64 : (kAccStages * BN) <= 128 ? 128
-                                   : (kAccStages * BN) <= 256 ? 256 : 512;        // a power of two
+    constexpr int kAccumulators = kChains > kAccStages ? kChains : kAccStages;
+    constexpr uint32_t kTmemCols = (kAccumulators * BN) <= 32 ? 32 : (kAccumulators * BN) <= 64 ? 64 : (kAccumulators * BN) <= 128 ? 128
+                                   : (kAccumulators * BN) <= 256 ? 256 : 512;        // a power of two
+    static_assert(kAccumulators * BN <= 512, "tensor memory has 512 columns");
     constexpr uint32_t kIdesc = instr_desc_bf16(kBM, BN);
 
     extern __shared__ uint8_t smem_raw[];
@@ -237,8 +253,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int as = acc_it % kAccStages;
                 if (!mbar_wait(smem_u32(&acc_empty_bar[as]), ((acc_it / kAccStages) & 1u) ^ 1u, abort_flag, p.error_flag, 102)) break;
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + as * BN;
+                uint32_t tmem_d = tmem_base + as * BN;
                 uint32_t accumulate = 0;
+                const int kb_per_chain = (kb1 - kb0 + kChains - 1) / kChains;
+                int next_chain = kb0 + kb_per_chain;
                 // whether the stage of the K block about to be multiplied has landed is looked up before the MMAs of
                 // the block ahead of it are issued, so that between two blocks' MMAs there is only the commit
                 bool landed = kb0 < kb1 && mbar_try_wait(full0 + stage * 8u, phase);
@@ -249,6 +267,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const uint32_t this_empty = empty0 + stage * 8u;
                     if (++stage == (uint32_t)kStages) { stage = 0; phase ^= 1u; }
                     landed = kb + 1 < kb1 && mbar_try_wait(full0 + stage * 8u, phase);
+                    if (kChains > 1 && kb == next_chain) {
+                        tmem_d += BN;
+                        accumulate = 0;
+                        next_chain += kb_per_chain;
+                    }
                     mma_bf16(tmem_d, da, db, kIdesc, accumulate);
                     mma_bf16(tmem_d, da + 2, db + 2, kIdesc, 1u);
                     mma_bf16(tmem_d, da + 4, db + 4, kIdesc, 1u);
@@ -368,6 +391,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         };
 
+        // 16 columns of the finished tile from `column` on: the accumulators of the chains that have a K block, added in order
+        auto load_columns = [&](uint32_t (&r)[16], uint32_t column, int range) {
+            tmem_ld16(column, r);
+            if constexpr (kChains > 1) {
+                const int kb_per_chain = (range + kChains - 1) / kChains;
+#pragma unroll
+                for (int chain = 1; chain < kChains; ++chain) {
+                    if (chain * kb_per_chain >= range) break;
+                    uint32_t more[16];
+                    tmem_ld16(column + (uint32_t)(chain * BN), more);
+                    tmem_ld_wait_for(r, more);
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) + __uint_as_float(more[c]));
+                }
+            }
+        };
+
         uint32_t acc_it = 0;
         for (int u = blockIdx.x; u < units; u += gridDim.x, ++acc_it) {
             int ta, tb, sp;
@@ -401,8 +441,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 for (int c0 = half * 32; c0 < BN; c0 += 64) {
                     const bool two = c0 + 16 < BN;
                     uint32_t r0[16], r1[16];
-                    tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN + c0, r0);
-                    if (two) tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN + c0 + 16, r1);
+                    load_columns(r0, tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN + c0, kb1 - kb0);
+                    if (two) load_columns(r1, tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN + c0 + 16, kb1 - kb0);
                     tmem_ld_wait();
                     float v[16];
 #pragma unroll
@@ -419,7 +459,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll 1
             for (int c0 = kSwapped ? ((warp - 2) >> 2) * 16 : BN; c0 < BN; c0 += 16 * kWarpsPerQuarter) {
                 uint32_t r[16];
-                tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN + c0, r);
+                load_columns(r, tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN + c0, kb1 - kb0);
                 tmem_ld_wait();
                 float v[16];
 #pragma unroll
@@ -543,23 +583,24 @@ struct Plan {
     bool swapped;
     int bn;
     int splits;
+    int chains;     // accumulators a block cuts its range of K into
     long cost;      // normal form: waves x the tile's time in the model's units; 0 for the swapped form
 };
 
-// The plan is a function of the shape alone.
+// The plan is a function of the shape, of whether the epilogue gates (tiles of whole runs) and of whether it does a norm's work (only the
+// swapped form's can).
 // Normal form: the grid runs in waves of one block per SM; the narrow tile's width is chosen so that the last
 // wave is as full as possible (measured at 2,048 rows, a tile's time hardly depends on its width: about
 // 20 + 0.03 x width microseconds at K = 4096).
 // Swapped form: up to 128 rows of x always; up to kMaxSwappedRows rows (one tile of 256 rows of x) when the
 // normal form would leave SMs without a tile, i.e. against a narrow weight matrix: a tile's K loop of 26 us
-// would then bound the product, while here every weight tile is streamed once and K is split over the SMs; unless K is short.
+// would then bound the product, while here every weight tile is streamed once and K is split over the SMs.
 // The split aims at a block (two for narrow tiles) on every SM and keeps at least four K blocks per block.
-// `normed`: the epilogue does a norm's work, which the normal form's does not.
 static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, bool gate_runs = false, bool normed = false) {
     Plan pl;
     pl.swapped = false;
     pl.bn = 128;
-    pl.splits = 1;
+    pl.splits = pl.chains = 1;
     pl.cost = 0;
     long normal_tiles = (long)((M + kBM - 1) / kBM) * ((N + 127) / 128);
     if (N >= 192) {
@@ -587,21 +628,26 @@ static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, b
         int pow2 = 1;
         while (pow2 * 2 <= s) pow2 *= 2;
         s = pow2;
-        // tiles of 256 rows of x fill an SM: of clusters of eight such blocks the device does not hold sixteen at once (130 to 256 rows,
-        // N 2,048, K 6,144 / 8,192: 27 / 30 -> 19 / 22 us)
-        if (pl.bn == 256 && s == 8 && tiles > 8) s = 4;
-        // more than 128 rows: the normal form instead, where a tile's whole K costs less than this form's share of it, its sums and their
-        // exchange (both in us; 130 / 256 rows, this form -> the normal one: K 1,024, N 5,632 17 / 19 -> 9; K 2,048, N 2,048 21 -> 14,
-        // N 8,192 19 / 20 -> 15, N 12,288 25 / 28 -> 15; K 4,096, N 6,144 24 / 25 -> 23, N 12,288 35 / 37 -> 26 / 27; this form stays at
-        // K 4,096, N 4,096, 18 us, where the normal one takes 28)
-        if (M > 128 && N >= 192 && force_splits <= 0 && !normed) {
-            const double here = 8.0 + 0.55 * ((kblocks + s - 1) / s) + (s > 1 ? 6.0 : 0.0);
-            const double there = 4.0 + (0.07 + 0.0017 * normal_bn) * (double)((normal_tiles + sm_count - 1) / sm_count) * kblocks;
-            if (there < here) {
+        // More than 128 rows: the normal form, one block a tile with the whole of K in as many accumulators as K would be split over blocks
+        // here (so the same sums), as far as that costs less than this form's sums and their exchange.  Four accumulators leave room for
+        // 128 columns, eight for none.  256 rows, this form -> the normal one: K whole, K 2,048 / 6,144, N 12,288 24 / 50 -> 15 / 38 us;
+        // in two, N 5,632, K 1,024 / 4,096 / 6,144 16 / 25 / 31 -> 9 / 23 / 33; in four, N 3,072, K 1,024 / 2,560 / 3,072 13 / 15.3 / 16.0 ->
+        // 9 / 15.1 / 17.1.
+        if (M > 128 && N >= 192 && force_splits <= 0 && !normed && (s == 1 || (s == 2 && kblocks <= 83) || (s == 4 && kblocks <= 41))) {
+            const int bn = s == 4 ? 128 : s == 2 ? 192 : normal_bn;
+            if ((long)((M + kBM - 1) / kBM) * ((N + bn - 1) / bn) <= sm_count) {
                 pl.swapped = false;
-                pl.bn = normal_bn;
+                pl.bn = bn;
+                pl.chains = s;
                 return pl;
             }
+        }
+        // Tiles of 256 rows of x fill an SM, and of clusters of eight such blocks the device holds fifteen at once, not sixteen: from
+        // sixteen tiles on, four blocks with two accumulators each (N 2,048, K 2,048 / 6,144 21 / 27 -> 14 / 20 us; N 1,920, 15 tiles by eight,
+        // 12 / 15).
+        if (pl.bn == 256 && s == 8 && tiles > 15 && force_splits <= 0) {
+            s = 4;
+            pl.chains = 2;
         }
         if (force_splits > 0) s = force_splits > kMaxSplits ? kMaxSplits : force_splits;
         if (s > kblocks) s = kblocks;
@@ -611,11 +657,11 @@ static Plan make_plan(int M, int N, int K, int sm_count, int force_splits = 0, b
     return pl;
 }
 
-template <int BN, bool kSwapped, bool kAct>
+template <int BN, bool kSwapped, bool kAct, int kChains>
 static int launch_form(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
     constexpr int stages = stages_for<BN>(kSwapped);
     const size_t smem = (size_t)stages * (kBM * kBK * 2 + BN * kBK * 2) + (kSwapped ? (BN < 128 ? BN * 512 + 4096 : 0) : 8 * kEpilogueStageBytes) + 1024;      // ring, split-K receive area behind it, alignment
-    auto kernel = gemm_tc_kernel<BN, kSwapped, kAct>;
+    auto kernel = gemm_tc_kernel<BN, kSwapped, kAct, kChains>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -625,16 +671,18 @@ static int launch_form(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
     const int tiles_a = (p.rows_a + kBM - 1) / kBM, tiles_b = (p.rows_b + BN - 1) / BN;
     const int units = tiles_a * tiles_b * p.splits;
     const int per_sm = (kSwapped && BN <= 128) ? 2 : 1;
-    // split K: one block per (tile, split), the splits of a tile being one cluster; else a persistent grid
-    const int grid = p.splits > 1 ? units : (units < sm_count * per_sm ? units : sm_count * per_sm);
+    // split K: one block per (tile, split), the splits of a tile being one cluster; several accumulators: one block a tile; else a
+    // persistent grid
+    const int grid = p.splits > 1 || kChains > 1 ? units : (units < sm_count * per_sm ? units : sm_count * per_sm);
     launch_kernel_clustered(kernel, grid, threads_for(kSwapped, BN), smem, p.splits > 1 ? p.splits : 1, stream, ma, mb, p);
     return CITLALI_LAUNCH_CHECK();
 }
 
-template <int BN, bool kSwapped>
+template <int BN, bool kSwapped, int kChains = 1>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
     const bool act = p.bias != nullptr || p.out_kind == kSquaredBF16 || p.out_kind == kGeluBF16;
-    return act ? launch_form<BN, kSwapped, true>(ma, mb, p, sm_count, stream) : launch_form<BN, kSwapped, false>(ma, mb, p, sm_count, stream);
+    return act ? launch_form<BN, kSwapped, true, kChains>(ma, mb, p, sm_count, stream)
+               : launch_form<BN, kSwapped, false, kChains>(ma, mb, p, sm_count, stream);
 }
 
 }  // namespace tc
@@ -796,7 +844,7 @@ static int gemm_tc_any(const void* x, const void* w, void* y, int y_dtype, int M
             case 32: rc = launch<32, true>(ma, mb, p, sm_count, stream); break;
             case 64: rc = launch<64, true>(ma, mb, p, sm_count, stream); break;
             case 128: rc = launch<128, true>(ma, mb, p, sm_count, stream); break;
-            default: rc = launch<256, true>(ma, mb, p, sm_count, stream); break;
+            default: rc = pl.chains == 2 ? launch<256, true, 2>(ma, mb, p, sm_count, stream) : launch<256, true>(ma, mb, p, sm_count, stream); break;
         }
     } else {
         if ((rc = make_map(&ma, x, M, K, kBM))) return rc;
@@ -806,8 +854,8 @@ static int gemm_tc_any(const void* x, const void* w, void* y, int y_dtype, int M
             case 240: rc = launch<240, false>(ma, mb, p, sm_count, stream); break;
             case 224: rc = launch<224, false>(ma, mb, p, sm_count, stream); break;
             case 208: rc = launch<208, false>(ma, mb, p, sm_count, stream); break;
-            case 192: rc = launch<192, false>(ma, mb, p, sm_count, stream); break;
-            default: rc = launch<128, false>(ma, mb, p, sm_count, stream); break;
+            case 192: rc = pl.chains == 2 ? launch<192, false, 2>(ma, mb, p, sm_count, stream) : launch<192, false>(ma, mb, p, sm_count, stream); break;
+            default: rc = pl.chains == 4 ? launch<128, false, 4>(ma, mb, p, sm_count, stream) : launch<128, false>(ma, mb, p, sm_count, stream); break;
         }
     }
     return rc;

@@ -494,6 +494,53 @@ def test_gemm_tc(M, N, K, one_block_or_pairs):
     assert plan["swapped"] or M > 128          # few rows: the weights are the 128-row operand
 
 
+@pytest.mark.parametrize("M, N, K, sums", [(129, 1152, 2048, 8), (256, 1152, 6144, 8), (200, 1920, 6144, 8), (256, 1921, 2048, 8),
+                                           (129, 2048, 6144, 8), (130, 2176, 2120, 8), (256, 1024, 1024, 4), (200, 2080, 1544, 4),
+                                           (250, 4096, 2624, 4), (250, 4096, 2632, 4), (256, 9472, 520, 2), (129, 5632, 5312, 2),
+                                           (200, 5632, 5320, 2), (130, 12288, 2048, 1), (256, 416, 264, 1)])
+def test_gemm_tc_of_129_to_256_rows(M, N, K, sums):
+    """The products either side of the lines that decide between the weights on the wide side split by eight, by four, and the form for
+    many rows, against float64: stored, added, gated, with a bias and an activation, and with a norm's work in the epilogue.  However a
+    product runs, its K is added up in ``sums`` parts (one sum of K products is off by an ulp for every 16 of them, always to one side):
+    the bits of that split, or for eight of them an error no larger than its."""
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g) / K ** 0.5).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    top = float(want.abs().max())
+    tol = 2 ** -23 * (K / 16 / sums + sums) * top           # an ulp of a running sum for 16 products and for each sum of sums
+    flag = torch.zeros(4, dtype=torch.int32, device=DEV)
+    xd, wd = x.to(DEV), w.to(DEV)
+    y, split = torch.full((M, N), 7.0, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_tc(xd, wd, y, error_flag=flag)
+    ops.gemm_tc(xd, wd, split, error_flag=flag, force_splits=sums)
+    assert float((y.double().cpu() - want).abs().max()) <= tol
+    if sums < 8:
+        assert torch.equal(y, split)
+    else:
+        assert float((y.double().cpu() - want).norm()) <= 1.1 * float((split.double().cpu() - want).norm())
+    base = torch.randn(M, N, generator=g)
+    acc = base.to(DEV)
+    ops.gemm_tc(xd, wd, acc, accumulate=True, error_flag=flag)
+    assert float((acc.double().cpu() - (base.double() + want)).abs().max()) <= tol + 2 ** -23 * float(base.abs().max())
+    sumsq = torch.rand(M, 3, generator=g)
+    ops.gemm_tc(xd, wd, y, error_flag=flag, row_scale=(sumsq.to(DEV), 6, 1e-6))
+    scale = torch.rsqrt(sumsq.double().sum(1, keepdim=True) / 6 + 1e-6)
+    assert float(((y.double().cpu() - want * scale) / scale).abs().max()) <= tol + 4 * 2 ** -23 * top
+    bias = torch.randn(N, generator=g)
+    half = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_tc_act(xd, wd, half, bias=bias.to(DEV), act="relu_squared", error_flag=flag)
+    squared = (want + bias.double()).clamp(min=0) ** 2
+    assert float((half.double().cpu() - squared).abs().max()) <= 2 ** -8 * float(squared.max())
+    if N % 32 == 0:
+        act = torch.empty(M, N // 2, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_tc(xd, wd, act, error_flag=flag, swiglu=True)
+        runs = want.view(M, N // 32, 2, 16)
+        gated = (runs[:, :, 0] * torch.sigmoid(runs[:, :, 0]) * runs[:, :, 1]).reshape(M, N // 2)
+        assert float((act.double().cpu() - gated).abs().max()) <= 2 ** -8 * float(gated.abs().max())
+    assert flag.tolist() == [0, 0, 0, 0]
+
+
 def test_gemm_tc_rows_do_not_depend_on_the_batch():
     """Within one width of the narrow tile (up to 16, 32, 64, 128 rows) a row's result is the same
     bit for bit whatever else is in the batch; between widths the K split may differ, and with it

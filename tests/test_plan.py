@@ -28,13 +28,21 @@ def test_few_rows_put_the_weights_on_the_wide_side(M, bn):
     assert splits in (1, 2, 4, 8)
 
 
-@pytest.mark.parametrize("N, K, form", [(12288, 2048, (False, 192, 1)), (2048, 2048, (False, 192, 1)), (5632, 1024, (False, 192, 1)),
+@pytest.mark.parametrize("N, K, form", [(12288, 2048, (False, 192, 1)), (2048, 2048, (True, 256, 4)), (5632, 1024, (False, 192, 1)),
                                         (2048, 6144, (True, 256, 4)), (4096, 4096, (True, 256, 4)), (1024, 4096, (True, 256, 8)),
                                         (4096, 12288, (True, 256, 4))])
 def test_more_than_128_rows_take_the_weights_wide_side_only_where_k_is_long(N, K, form):
     assert plan(129, N, K) == plan(256, N, K) == form
     assert plan(128, N, K)[:2] == (True, 128) and not plan(257, N, K)[0]
     assert plan(200, N, K, force=2)[0]                   # a forced split is one of the few-row form
+
+
+@pytest.mark.parametrize("K", [2048, 3072, 4096, 12288])
+def test_more_than_128_rows_split_k_by_eight_up_to_fifteen_tiles(K):
+    """N of 8, 9, 12 and 15 tiles of 128 weight rows; with 16 of them clusters of eight blocks do not fit the device at once."""
+    for M in (129, 256):
+        assert [plan(M, N, K) for N in (1024, 1025, 1152, 1536, 1920)] == [(True, 256, 8)] * 5
+        assert plan(M, 1921, K) == plan(M, 2048, K) == (True, 256, 4)
 
 
 def test_k_is_split_by_shape_alone():

@@ -182,9 +182,13 @@ int citlali_argmax_rows_wide(const float* logits, int32_t* tokens, float* scratc
 int citlali_sample_rows(const float* logits, const float* temperature, const float* uniform,
                         int32_t* tokens, int rows, int vocab, cudaStream_t stream);
 
-// The tensor-core product (bfloat16 operands, float accumulation).  citlali_gemm_tc_plan tells
-// how a shape runs: whether the weights are the 128-row operand (*swapped), the narrow tile
-// (*bn) and the K split (*splits).  force_splits > 0 replaces the plan's split (at most 8).
+// The tensor-core product (bfloat16 operands, float accumulation).  citlali_gemm_tc_plan_for tells how a shape runs: whether the
+// weights are the 128-row operand (*swapped), the narrow tile (*bn), the K split (*splits) and in how many float sums K is added
+// up before these are added (*sums: a block may keep several).  gated: a gate epilogue (SiLU or GELU); normed: a norm's
+// work in the epilogue (citlali_gemm_tc_normed), which only the swapped form does.  force_splits > 0 replaces the plan's split
+// (at most 8).  citlali_gemm_tc_plan: the same of a product with neither.
+int citlali_gemm_tc_plan_for(int M, int N, int K, int gated, int normed, int sm_count, int force_splits, int* swapped, int* bn,
+                             int* splits, int* sums);
 int citlali_gemm_tc_plan(int M, int N, int K, int sm_count, int force_splits, int* swapped, int* bn, int* splits);
 // y = x[M, K] . w[N, K]^T.  mode bits: 1 = y (float32) += product; 2 = SiLU-gate epilogue (w's rows
 // alternate in runs of 16 between gate and up; y is bfloat16 [M, N/2]).  K must be a multiple of 8

@@ -751,14 +751,20 @@ extern "C" int citlali_wait_selftest(int32_t* error_flag, int* result, long long
     return CITLALI_LAUNCH_CHECK();
 }
 
-// How the product of this shape would run: *swapped, *bn and the K split (*splits).
-extern "C" int citlali_gemm_tc_plan(int M, int N, int K, int sm_count, int force_splits, int* swapped, int* bn, int* splits) {
+// How the product of this shape would run: *swapped, *bn, the K split (*splits) and in how many sums K is added up (*sums).
+extern "C" int citlali_gemm_tc_plan_for(int M, int N, int K, int gated, int normed, int sm_count, int force_splits, int* swapped, int* bn,
+                                        int* splits, int* sums) {
     if (sm_count <= 0) sm_count = device_sm_count();
-    Plan pl = make_plan(M, N, K, sm_count, force_splits);
+    const Plan pl = make_plan(M, N, K, sm_count, force_splits, gated != 0, normed != 0);
     if (swapped) *swapped = pl.swapped;
     if (bn) *bn = pl.bn;
     if (splits) *splits = pl.splits;
+    if (sums) *sums = pl.splits * pl.chains;
     return 0;
+}
+
+extern "C" int citlali_gemm_tc_plan(int M, int N, int K, int sm_count, int force_splits, int* swapped, int* bn, int* splits) {
+    return citlali_gemm_tc_plan_for(M, N, K, 0, 0, sm_count, force_splits, swapped, bn, splits, nullptr);
 }
 
 // y = x . w^T with x [M, K] and w [N, K] bfloat16, contiguous, 16-byte aligned, K a multiple of 8.
@@ -774,7 +780,7 @@ extern "C" int citlali_gemm_tc(const void* x, const void* w, void* y, int y_dtyp
                                   nullptr, 0, 0, 0.0f, stream);
 }
 
-// citlali_gemm_tc_normed: citlali_gemm_tc for few rows of x (the form with the weights as the 128-row operand: see citlali_gemm_tc_plan) with a
+// citlali_gemm_tc_normed: citlali_gemm_tc for few rows of x (the form with the weights as the 128-row operand: see citlali_gemm_tc_plan_for) with a
 // layer norm's work in its epilogue.  `emit_rows` / `emit_sumsq` (both or neither; mode bit 0, N a multiple of 32): the
 // product is added to the float32 rows y as always, and the updated rows also go out as bfloat16 [M, N] with the sums of
 // their squares over each 32 consecutive features, float32 [M, N / 32].  `scale_sumsq` (float32 [M, scale_groups], the

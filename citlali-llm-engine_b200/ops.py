@@ -432,12 +432,12 @@ def sm_count(device) -> int:
     return n
 
 
-def gemm_tc_plan(M: int, N: int, K: int, device, force_splits: int = 0) -> dict:
-    """How the tensor-core product of this shape runs."""
-    swapped, bn, splits = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
-    lib().citlali_gemm_tc_plan(_i(M), _i(N), _i(K), _i(sm_count(device)), _i(force_splits), ctypes.byref(swapped),
-                               ctypes.byref(bn), ctypes.byref(splits))
-    return {"swapped": bool(swapped.value), "bn": bn.value, "splits": splits.value}
+def gemm_tc_plan(M: int, N: int, K: int, device, force_splits: int = 0, gated: bool = False, normed: bool = False) -> dict:
+    """How the tensor-core product of this shape runs; ``gated``: with the gate epilogue, ``normed``: with a norm's work in the epilogue."""
+    swapped, bn, splits, sums = ctypes.c_int(), ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+    lib().citlali_gemm_tc_plan_for(_i(M), _i(N), _i(K), _i(1 if gated else 0), _i(1 if normed else 0), _i(sm_count(device)), _i(force_splits),
+                                   ctypes.byref(swapped), ctypes.byref(bn), ctypes.byref(splits), ctypes.byref(sums))
+    return {"swapped": bool(swapped.value), "bn": bn.value, "splits": splits.value, "sums": sums.value}
 
 
 def wait_selftest(error_flag: torch.Tensor, limit_ms: float = 2.0):
@@ -535,7 +535,7 @@ def norm_inputs(x: torch.Tensor, rows_out: torch.Tensor, sumsq: torch.Tensor):
 
 def gemm_tc_is_small_form(M: int, N: int, K: int, device) -> bool:
     """Whether the product of this shape runs the form for few rows of x, whose epilogue can do a norm's work."""
-    return gemm_tc_plan(M, N, K, device)["swapped"]
+    return gemm_tc_plan(M, N, K, device, normed=True)["swapped"]
 
 
 def gemm_tc(x, w, y, accumulate=False, error_flag=None, swiglu=False, force_splits=0, emit=None, row_scale=None):

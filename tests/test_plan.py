@@ -45,6 +45,22 @@ def test_more_than_128_rows_split_k_by_eight_up_to_fifteen_tiles(K):
         assert plan(M, 1921, K) == plan(M, 2048, K) == (True, 256, 4)
 
 
+@pytest.mark.parametrize("N, K, sums", [(2048, 2048, 8), (1152, 12288, 8), (4096, 2624, 4), (4096, 2688, 4), (5632, 5312, 2), (5632, 5376, 2),
+                                        (12288, 2048, 1), (256, 256, 1)])
+def test_more_than_128_rows_add_k_up_in_as_many_sums_whatever_the_form(monkeypatch, N, K, sums):
+    """One sum over all of K is off by as much as K is long: the form for many rows, and a split by four where one by eight does not fit,
+    keep as many sums as K would be split over blocks.  A norm's work in the epilogue takes the form that can do it."""
+    library()
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    for M in (129, 256):
+        plain, normed = ops.gemm_tc_plan(M, N, K, None), ops.gemm_tc_plan(M, N, K, None, normed=True)
+        assert plain["sums"] == ops.gemm_tc_plan(M, N, K, None, gated=True)["sums"] == normed["sums"] == sums
+        assert normed["swapped"] and ops.gemm_tc_is_small_form(M, N, K, None)
+        many = K in (2624, 5312) or sums == 1
+        assert plain["swapped"] != many and plain["bn"] == (256 if not many else 128 if sums == 4 else 192)
+    assert ops.gemm_tc_plan(257, N, K, None)["sums"] == 1 and not ops.gemm_tc_is_small_form(257, N, K, None)
+
+
 def test_k_is_split_by_shape_alone():
     # 148 SMs, two blocks each: 296 places for (tile, split) pairs; a split keeps four K blocks of 64 at least
     assert plan(8, 6144, 4096) == (True, 16, 4)          # 48 tiles: 6 would fit, powers of two only

@@ -130,6 +130,8 @@ int citlali_attention_prefill(const void* q, int q_stride, const void* k_pool, c
                               int nq, int nkv, int head_dim, int value_dim, int page_size, int window, int keep_first,
                               float scale, float softcap, const float* gate, size_t gate_stride, const float* sink,
                               const float* turns, int turn_pairs, float* out32, cudaStream_t stream);
+// Which kernel a run of max_new tokens takes: 2 citlali_attention_prefill_tc, 1 citlali_attention_prefill, 0 neither.
+int citlali_attention_run_form(int q_stride, int out_stride, int head_dim, int page_size, int max_new);
 // sink [nq] (may be null): the softmax's denominator also counts exp(sink[head]), neither scaled nor capped.  turns
 // [rows, value_dim / 2] (cos, sin) (may be null; 16-byte aligned): the result's pairs (m, m + value_dim / 2), or with
 // turn_pairs (2m, 2m + 1), are turned back by the row's angles, ahead of the gate.  out32 (may be null; not with turns): the

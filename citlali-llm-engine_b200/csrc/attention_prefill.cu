@@ -330,6 +330,15 @@ extern "C" int citlali_attention_prefill_supports(int head_dim, int page_size) {
     }
 }
 
+// Which kernel takes runs of at most max_new new tokens, bfloat16 rows so many elements apart: 2 citlali_attention_prefill_tc, 1
+// citlali_attention_prefill, 0 neither.  A query tile of the tcgen05 kernel has 128 rows (two at a time), one here 64:
+// below 48 tokens most of what it multiplies would be empty rows.
+extern "C" int citlali_attention_run_form(int q_stride, int out_stride, int head_dim, int page_size, int max_new) {
+    if (q_stride % 8 != 0) return 0;
+    if (max_new >= 48 && out_stride % 8 == 0 && head_dim == kRunTcHead && page_size == kRunTcPage) return 2;
+    return citlali_attention_prefill_supports(head_dim, page_size);
+}
+
 // 1 if citlali_attention_prefill has a kernel for keys of d and values of vd elements.
 extern "C" int citlali_attention_prefill_supports_sizes(int d, int vd, int page_size) {
     if (d == vd && citlali_attention_prefill_supports(d, page_size)) return 1;

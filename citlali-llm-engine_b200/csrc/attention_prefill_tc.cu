@@ -63,7 +63,7 @@ namespace fatc {
 
 using namespace tc;
 
-constexpr int kD = 128, kTileQ = 128, kTileK = 128, kPage = 64;
+constexpr int kD = kRunTcHead, kTileQ = 128, kTileK = 128, kPage = kRunTcPage;
 constexpr int kWarpLoadK = 16, kWarpLoadV = 17, kWarpMma = 18;
 constexpr int kThreads = 608;
 constexpr int kHalfKeys = kTileK / 2;                  // keys of a tile that one softmax thread works on

@@ -63,6 +63,9 @@ inline int raise_shared_limit(Kernel kernel, size_t bytes, size_t most) {
     return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
+// The head and page size that attention_prefill_tc.cu takes, for the rule in attention_prefill.cu that decides between the two.
+constexpr int kRunTcHead = 128, kRunTcPage = 64;
+
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg = {};

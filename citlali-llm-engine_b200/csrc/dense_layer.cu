@@ -8,16 +8,13 @@
 
 using namespace citlali;
 
-// From here on the tcgen05 kernel takes a run of new tokens, below it the one with tiles of fewer rows.
-constexpr int kTensorCoreRows = 48;
-
-static bool on_tcgen05(int head_dim, int page_size, int max_new) {
-    return max_new >= kTensorCoreRows && citlali_attention_prefill_tc_supports(head_dim, page_size);
+static int attention_form(int nq, int nkv, int head_dim, int page_size, int max_new) {
+    return citlali_attention_run_form((nq + 2 * nkv) * head_dim, nq * head_dim, head_dim, page_size, max_new);
 }
 
 extern "C" int citlali_dense_layer_supports(int nq, int nkv, int head_dim, int page_size, int max_new) {
-    if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || ((nq + 2 * nkv) * head_dim) % 8 != 0 || (nq * head_dim) % 8 != 0) return 0;
-    return on_tcgen05(head_dim, page_size, max_new) || citlali_attention_prefill_supports(head_dim, page_size) ? 1 : 0;
+    if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || (nq * head_dim) % 8 != 0) return 0;
+    return attention_form(nq, nkv, head_dim, page_size, max_new) != 0 ? 1 : 0;
 }
 
 extern "C" int citlali_dense_layer(const CitlaliDenseLayer* l, float* x, void* qkv, void* heads, void* act, const void* in_rows,
@@ -43,7 +40,7 @@ extern "C" int citlali_dense_layer(const CitlaliDenseLayer* l, float* x, void* q
                                       l->page_table, l->page_table_stride, l->k_pool, l->v_pool, kBF16, l->page_size, rows, l->nq,
                                       l->nkv, l->head_dim, l->head_eps, 1, stream);
     if (code) return code;
-    code = on_tcgen05(l->head_dim, l->page_size, max_new)
+    code = attention_form(l->nq, l->nkv, l->head_dim, l->page_size, max_new) == 2
                ? citlali_attention_prefill_tc(qkv, width, rows, l->k_pool, l->v_pool, l->pool_pages, l->page_table, l->page_table_stride,
                                               seq_start, seq_slot, seq_past, heads, out, sequences, max_new, l->nq, l->nkv,
                                               l->head_dim, l->page_size, l->window, l->scale, nullptr, stream)

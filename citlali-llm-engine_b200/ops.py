@@ -8,7 +8,6 @@ CUDA device, they raise.
 from __future__ import annotations
 
 import ctypes
-import math
 import operator
 import struct
 from typing import Optional
@@ -301,14 +300,15 @@ def attention(q, q_stride, cache_view, batch, out, nq, nkv, head_dim, window, sc
     require(not torch.cuda.is_current_stream_capturing(),
             "attention: this dtype and head size run a kernel whose launch is sized from the host's lists of lengths, "
             "which a captured step would freeze; such a model steps without CUDA graphs")
-    if (q.dtype == torch.bfloat16 and q_stride % 8 == 0 and out.shape[1] % 8 == 0 and batch.max_new >= 48
-            and lib().citlali_attention_prefill_tc_supports(_i(head_dim), _i(cache_view.page_size))):
+    form = 0
+    if q.dtype == torch.bfloat16:
+        form = lib().citlali_attention_run_form(_i(q_stride), _i(out.shape[1]), _i(head_dim), _i(cache_view.page_size), _i(batch.max_new))
+    if form == 2:
         attention_prefill_tc(q, q_stride, cache_view.keys, cache_view.values, cache_view.page_table, batch.seq_start,
                              batch.seq_slot, batch.seq_past, out, batch.sequences, batch.max_new, nq, nkv, head_dim,
                              cache_view.page_size, window, scale)
         return
-    if (q.dtype == torch.bfloat16 and q_stride % 8 == 0
-            and lib().citlali_attention_prefill_supports(_i(head_dim), _i(cache_view.page_size))):
+    if form == 1:
         attention_prefill(q, q_stride, cache_view.keys, cache_view.values, cache_view.page_table, batch.seq_start,
                           batch.seq_slot, batch.seq_past, out, batch.sequences, batch.max_new, nq, nkv, head_dim,
                           cache_view.page_size, window, scale)
@@ -586,10 +586,10 @@ def dense_layer_supports(nq, nkv, head_dim, page_size, max_new) -> bool:
 
 
 def dense_layer(weights, gains, inv_freq, rotary_dim, cache_view, sizes, eps, x, scratch, normed_in, normed_mid, normed_out, batch,
-                error_flag):
+                error_flag, scale):
     """A whole layer over at most 128 rows (csrc/dense_layer.cu): ``weights`` (qkv, o, gate_up, down), ``gains`` of the head norms,
     ``sizes`` (hidden, inter, query heads, key heads, head size, window), ``eps`` (head norms, mixer's norm, feed-forward's norm),
-    ``scratch`` (qkv rows, heads, activations), three pairs (rows, sums of squares).  Every tensor the kernels read or write is checked
+    ``scratch`` (qkv rows, heads, activations), three pairs (rows, sums of squares), the scores' ``scale``.  Every tensor the kernels read or write is checked
     here, as the six calls this one stands for check theirs."""
     qkv, o, gate_up, down = weights
     hidden, inter, nq, nkv, d, window = sizes
@@ -613,7 +613,7 @@ def dense_layer(weights, gains, inv_freq, rotary_dim, cache_view, sizes, eps, x,
     layer = _DENSE_LAYER.pack(
         qkv.data_ptr(), o.data_ptr(), gate_up.data_ptr(), down.data_ptr(), _ptr(q_gain) or 0, _ptr(k_gain) or 0, inv_freq.data_ptr(),
         keys.data_ptr(), values.data_ptr(), table.data_ptr(), _F32 if q_gain is None else _dtype_code(q_gain), rotary_dim, table.shape[1],
-        keys.shape[0], cache_view.page_size, hidden, inter, nq, nkv, d, window, eps[0], 1.0 / math.sqrt(d), eps[1], eps[2])
+        keys.shape[0], cache_view.page_size, hidden, inter, nq, nkv, d, window, eps[0], scale, eps[1], eps[2])
     _check(lib().citlali_dense_layer(
         layer, x.data_ptr(), scratch[0].data_ptr(), scratch[1].data_ptr(), scratch[2].data_ptr(), normed_in[0].data_ptr(),
         normed_in[1].data_ptr(), normed_mid[0].data_ptr(), normed_mid[1].data_ptr(), normed_out[0].data_ptr(), normed_out[1].data_ptr(),

@@ -41,6 +41,7 @@ class GQAttention:
         require(self.window is None or int(self.window) > 0, f"{prefix}: window must be positive or None")
         pos = dict(params.get("position") or {"kind": "none"})
         self.position = part_class("position", pos.pop("kind"))(pos, self.d)
+        self.scale = 1.0 / math.sqrt(self.d)
         self.prefix = prefix
         names = [f"{prefix}.q_proj.weight"]
         outs = [self.nq * self.d]
@@ -137,7 +138,7 @@ class GQAttention:
                 ops.qk_norm_rope_cache(qkv, None, None, self.inv_freq, self.rotary_dim, *common, write_cache=True)
         out = torch.empty((batch.rows, self.nq * self.d), dtype=self.dtype, device=qkv.device)
         ops.attention(qkv, qkv.shape[1], cache_view, batch, out, self.nq, self.nkv, self.d,
-                      int(self.window or 0), 1.0 / math.sqrt(self.d))
+                      int(self.window or 0), self.scale)
         self.o.forward(out, accumulate_into=residual, emit=emit)
         return residual
 

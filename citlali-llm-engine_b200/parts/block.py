@@ -116,7 +116,7 @@ class PreNormResidualBlock:
                             mixer.inv_freq, mixer.rotary_dim, cache_view,
                             (hidden, ff.inter, mixer.nq, mixer.nkv, mixer.d, int(mixer.window or 0)),
                             (float(mixer.eps or 0.0), self.mixer_norm.eps, self.feed_forward_norm.eps), x, batch.layer_scratch[1],
-                            (carried.rows, carried.sumsq), after_mixer, after_ff, batch, self.error_flag)
+                            (carried.rows, carried.sumsq), after_mixer, after_ff, batch, self.error_flag, mixer.scale)
             batch.norm_carry = NormedRows(after_ff[0], after_ff[1], hidden)
             return x
         self.mixer.forward(carried.with_eps(self.mixer_norm.eps), batch, cache_view, x, write_cache, emit=after_mixer)

@@ -39,7 +39,7 @@ def _call(a):
     cache = types.SimpleNamespace(keys=a["keys"], values=a["values"], page_table=a["page_table"], page_size=64)
     ops.dense_layer((a["qkv"], a["o"], a["gate_up"], a["down"]), (a["q_gain"], a["k_gain"]), a["inv_freq"], D, cache,
                     (HIDDEN, INTER, NQ, NKV, D, 0), (1e-6, 1e-6, 1e-6), a["x"], (a["s_qkv"], a["s_heads"], a["s_act"]),
-                    (a["in_rows"], a["in_sums"]), (a["mid_rows"], a["mid_sums"]), (a["out_rows"], a["out_sums"]), batch, a["error_flag"])
+                    (a["in_rows"], a["in_sums"]), (a["mid_rows"], a["mid_sums"]), (a["out_rows"], a["out_sums"]), batch, a["error_flag"], 0.25)
 
 
 @pytest.fixture

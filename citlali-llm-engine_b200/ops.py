@@ -576,13 +576,21 @@ def gemm_tc(x, w, y, accumulate=False, error_flag=None, swiglu=False, force_spli
            "gemm_tc")
 
 
-_ONLY_I32, _ONLY_F32, _ONLY_BF16 = {torch.int32}, {torch.float32}, {torch.bfloat16}
+def _all_are(dtype, tensors) -> bool:
+    """Whether all of them are contiguous tensors of ``dtype`` on a CUDA device, in one pass: a call with thirty of them is one of many in
+    a step that waits for the host."""
+    for t in tensors:
+        if t.dtype is not dtype or not t.is_cuda or not t.is_contiguous():
+            return False
+    return True
+
+
 # ``CitlaliDenseLayer`` of csrc/api.h: ten addresses, eleven whole numbers, four floats, filled up to the structure's alignment
 _DENSE_LAYER = struct.Struct("@10P11i4f0P")
 
 
 def dense_layer_supports(nq, nkv, head_dim, page_size, max_new) -> bool:
-    return bool(lib().citlali_dense_layer_supports(_i(nq), _i(nkv), _i(head_dim), _i(page_size), _i(max_new)))
+    return lib().citlali_dense_layer_supports(nq, nkv, head_dim, page_size, max_new) != 0
 
 
 def dense_layer(weights, gains, inv_freq, rotary_dim, cache_view, sizes, eps, x, scratch, normed_in, normed_mid, normed_out, batch,
@@ -598,10 +606,10 @@ def dense_layer(weights, gains, inv_freq, rotary_dim, cache_view, sizes, eps, x,
     indices = (batch.row_slot, batch.row_pos, batch.seq_start, batch.seq_slot, batch.seq_past, table)
     in_bf16 = (*weights, *scratch, keys, values, normed_in[0], normed_mid[0], normed_out[0])
     in_f32 = (x, inv_freq, normed_in[1], normed_mid[1], normed_out[1])
-    _need_cuda(*in_bf16, *in_f32, *indices, q_gain, k_gain, error_flag)
-    require({t.dtype for t in indices} == _ONLY_I32, "dense_layer: index tensors are int32")
-    require({t.dtype for t in in_bf16} == _ONLY_BF16, "dense_layer: weights, cache and rows are bfloat16")
-    require({t.dtype for t in in_f32} == _ONLY_F32, "dense_layer: residual rows, frequencies and sums of squares are float32")
+    _need_cuda(q_gain, k_gain, error_flag)
+    if not (_all_are(torch.bfloat16, in_bf16) and _all_are(torch.float32, in_f32) and _all_are(torch.int32, indices)):
+        _need_cuda(*in_bf16, *in_f32, *indices)
+        require(False, "dense_layer: weights, cache and rows are bfloat16, residual rows, frequencies and sums of squares float32, indices int32")
     require(q_gain is None or k_gain is None or q_gain.dtype == k_gain.dtype, "dense_layer: q and k gains differ in dtype")
     stream, sums, out = x.shape, (rows, hidden // 32), (nq + 2 * nkv) * d
     require(qkv.shape == (out, hidden) and o.shape == (hidden, nq * d) and gate_up.shape == (2 * inter, hidden)

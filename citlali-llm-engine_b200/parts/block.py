@@ -45,8 +45,17 @@ class PreNormResidualBlock:
             self.feed_forward = build_part("feed_forward", layer_spec.part("feed_forward"))
 
     def kernel_sources(self, dtype):
-        whole = type(self.mixer) is GQAttention and type(self.feed_forward) is GatedSiluFeedForward
-        return ("dense_layer",) if whole and dtype == torch.bfloat16 else ()
+        """The layer from one call, where its parts and sizes can come to it (``_from_one_call`` behind ``norms_in_products``)."""
+        mixer, ff = self.mixer, self.feed_forward
+        whole = (dtype == torch.bfloat16 and type(mixer) is GQAttention and type(ff) is GatedSiluFeedForward and self._norms_can_move()
+                 and mixer.kv_projection and mixer.position.inv_freq is not None and (mixer.nq * mixer.d) % 8 == 0
+                 and ff.plain and ff.inter % 16 == 0)
+        return ("dense_layer",) if whole else ()
+
+    def _norms_can_move(self) -> bool:
+        """Whether the two norms are of a kind and size that the products around them can do."""
+        return (type(self.mixer_norm) is RMSNorm and type(self.feed_forward_norm) is RMSNorm
+                and self.mixer_norm.size % 32 == 0 and self.mixer_norm.size == self.feed_forward_norm.size)
 
     def parts(self):
         return [p for p in (self.mixer_norm, self.mixer, self.feed_forward_norm, self.feed_forward) if p is not None]
@@ -62,9 +71,7 @@ class PreNormResidualBlock:
             p.bind(weights, ctx)
         self.norms_in_products = (
             self.mixer is not None and self.feed_forward is not None and ctx.dtype == torch.bfloat16
-            and type(self.mixer_norm) is RMSNorm and type(self.feed_forward_norm) is RMSNorm
-            and not self.mixer_norm.gain_downstream and not self.feed_forward_norm.gain_downstream
-            and self.mixer_norm.size % 32 == 0 and self.mixer_norm.size == self.feed_forward_norm.size
+            and self._norms_can_move() and not self.mixer_norm.gain_downstream and not self.feed_forward_norm.gain_downstream
             and callable(getattr(self.mixer, "can_absorb_norm", None)) and self.mixer.can_absorb_norm()
             and callable(getattr(self.feed_forward, "can_absorb_norm", None)) and self.feed_forward.can_absorb_norm())
         if self.norms_in_products:

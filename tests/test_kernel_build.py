@@ -44,6 +44,18 @@ def test_models_name_existing_sources():
     assert named == ["attention_generic", "elementwise", "gemm_simt"]
 
 
+@pytest.mark.parametrize("change, named", [({}, True), (dict(hidden_size=80), False), (dict(intermediate_size=72), False),
+                                           (dict(head_dim=18, num_attention_heads=2), False)])
+def test_a_model_names_the_layer_from_one_call_only_where_it_can_run_it(change, named):
+    """Widths that keep the norms out of the products, and inner and head sizes their forms do not take, leave the source out; so does the
+    32-bit path."""
+    q = cb.config_from_dict(dict(dict(architectures=["Qwen3ForCausalLM"], num_hidden_layers=1, hidden_size=64, num_attention_heads=4,
+                                      num_key_value_heads=2, head_dim=32, intermediate_size=64, vocab_size=50, rope_theta=1e4,
+                                      rms_norm_eps=1e-6, tie_word_embeddings=True, max_position_embeddings=64), **change))
+    sources = lambda dtype: DecoderModel(q.to_model_spec(), BuildContext(torch.device("cpu"), dtype)).kernel_sources()
+    assert ("dense_layer" in sources(torch.bfloat16)) == named and "dense_layer" not in sources(torch.float32)
+
+
 def test_an_entry_point_compiles_its_own_source_only(tmp_path, monkeypatch):
     if shutil.which("nvcc") is None and not os.path.isfile("/usr/local/cuda/bin/nvcc"):
         pytest.skip("no nvcc here")

@@ -162,7 +162,8 @@ def qwen3_config(width: int, layers: int, vocab: int):
 
 
 class KernelTimer:
-    """While active, every kernel function of :mod:`ops` runs between two CUDA events."""
+    """While active, every kernel function of :mod:`ops` runs between two CUDA events; layers that could come from one call make their
+    launches one by one, so that each is timed."""
 
     SKIP = {"lib", "prepare_kernels", "launch_count", "sm_count", "zero_counters", "attention", "gemm_tc_plan", "gemm_tc_accepts",
             "gemm_tc_pair_plan", "gemm_tc_runs_on_pairs", "gemm_tc_is_small_form", "gemm_tc_set_pair_rows",
@@ -188,6 +189,8 @@ class KernelTimer:
                 self.records.append((_name, _shape_note(_name, a), start, end))
                 return out
             setattr(ops, name, timed)
+        self._saved["dense_layer_supports"] = ops.dense_layer_supports
+        ops.dense_layer_supports = lambda *sizes: False
         return self
 
     def __exit__(self, *exc):

@@ -15,8 +15,8 @@
 //   delta_chunk_scan           one block a (sequence, head, VS columns of the values): the chunks in order, S in registers and in shared
 //                              memory.  [K; Q] S is the bulk: 256 threads, 8 x 4 outputs each over a slice of the 128 k, the slices'
 //                              sums added through shared memory; the next chunk's rows arrive meanwhile.  VS is 32, or 16 where that
-//                              leaves SMs idle.  Two warps a scheduler and five barriers a chunk: latency, beside some 4,100 wavefronts of
-//                              shared memory and 3,600 FMA issues a scheduler in a chunk's 8,800 clocks.
+//                              leaves SMs idle.  Two warps a scheduler and four barriers a chunk: latency, beside 5,000 wavefronts of
+//                              shared memory and 3,600 FMA issues a scheduler in a chunk's 9,000 clocks.
 // One sequence of 2,048 tokens, 32 heads over 16 key heads, 128 x 128: 316 us for both kernels (31 of them the coefficients); the walk of
 // two tokens a step 948.
 #include "api.h"
@@ -254,8 +254,8 @@ delta_chunk_scan_kernel(const float* __restrict__ prep, int prep_stride, const f
     fetch(0);
     // Where a warp's lanes stand in a product.  Of a 16-byte read of shared memory two neighbours (or two lanes two apart) that read the
     // same place are served together, lanes further apart are not: columns in the lane's low bits and rows above them cost the columns'
-    // operand four wavefronts a read, columns in every other bit and rows in those between cost either operand two.  (By count the scan's reads
-    // 4,100 wavefronts a chunk instead of 5,900; with the coefficients, columns in the low bits -> every other bit: one sequence of
+    // operand four wavefronts a read, columns in every other bit and rows in those between cost either operand two.  (By the counters
+    // 5,000 wavefronts a chunk instead of 6,000, 800 of them bank conflicts instead of 200; with the coefficients, columns in the low bits -> every other bit: one sequence of
     // 2,048 tokens, 32 heads 323 -> 316 us, 8 heads (16 columns a block) 232 -> 214, five of 155 to 540 tokens, 16 heads 149 -> 145.)
     const int lane = tid & 31, warp = tid >> 5;
     const int even = (lane & 1) | ((lane >> 1) & 2) | ((lane >> 2) & 4), odd = ((lane >> 1) & 1) | ((lane >> 2) & 2);    // bits 0 2 4; 1 3

@@ -2,7 +2,8 @@
 //   qkv = rms(x) W_qkv^T | head norms, rotation, cache | attention | x += . W_o^T | act = silu(gate) up | x += act W_down^T
 // of citlali_gemm_tc_normed, citlali_qk_norm_rope_cache and citlali_attention_prefill(_tc), with the two norms in the products.
 // What bounds a step of few rows is the host: 15 us a launch from Python, where the call itself is 3 to 4, against 6 to 10 us of a kernel
-// of 23 rows.  (14 layers of width 2,048, a prompt of 23: 1,338 -> 846 us a step; three sequences that go on by up to 3 tokens: 1,277 -> 715.)
+// of 23 rows.  (14 layers of width 2,048, a prompt of 23: 1,360 -> 850 us a step; three sequences behind some 700 tokens that go on by 1
+// or 2: 1,310 -> 1,000; 100 rows as before, 1,350: there, as in the second case by now, the kernels are as long.)
 #include "api.h"
 #include "common.cuh"
 

@@ -196,7 +196,8 @@ def test_32_bit_products_give_a_row_the_same_bits_in_steps_of_any_size(N, K, odd
 @pytest.mark.parametrize("M, N, K, odd", [(64, 1024, 96, False), (65, 1531, 100, False), (682, 1024, 68, False), (500, 1100, 33, False),
                                           (130, 2300, 64, True), (273, 2400, 40, False), (1200, 1024, 36, False)])
 def test_narrow_32_bit_products_give_the_bits_of_few_rows(M, N, K, odd):
-    """Every width of the narrow tiles (32 to 96 columns), ragged rows, columns and last tiles of k, in pieces and element by element."""
+    """Narrow tiles of 32, 48 and 80 columns, ragged rows, columns and last tiles of k, in pieces and element by element (the other widths and
+    forms are in the next test)."""
     g = torch.Generator().manual_seed(M + N + K)
     store = torch.zeros(N * K + 1, device=DEV)
     w = store[1:].view(N, K) if odd else store[:-1].view(N, K)

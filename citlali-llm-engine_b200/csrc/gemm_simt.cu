@@ -182,7 +182,8 @@ gemm_simt_wide_kernel(const float* __restrict__ x, const float* __restrict__ w, 
 // What bounds it: a block or two an SM, a warp or two a scheduler, so the chain of reads and multiply-adds of a thread.  Rows of both
 // operands lie in shared memory as they do in memory, 32 k of each, copied in 16-byte pieces (kPieces; else element by element) three
 // tiles deep; a thread's 16-byte reads are four k of a row, so a copy costs a quarter of the instructions, and 8 RN multiply-adds a k
-// need no moves.  Element by element a warp copies 32 k of one row (eight lanes a row, four k apart: 49 -> 45 us at 682 rows, N 1,024, K 1,022).  Lanes are placed as in the delta rule's scan: two that read the same place are neighbours or two apart, and a read
+// need no moves.  Element by element a warp copies 32 k of one row (eight lanes a row, four k apart: 49 -> 45 us at 682 rows, N 1,024, K 1,022).
+// Lanes are placed as in the delta rule's scan: two that read the same place are neighbours or two apart, and a read
 // costs two wavefronts.
 // 682 rows one product after another, 64 x 64 tiles of the kernel above -> here: N 1,024, K 1,024 / 2,816 (143 tiles of 64 x 80 instead of
 // 176) 94 / 223 -> 43 / 112 us; N 1,536, K 1,024 97 -> 62; 200 rows, N 1,024 / 1,536 47 / 71 -> 22 / 29; 33 rows, N 1,024 41 -> 21.
